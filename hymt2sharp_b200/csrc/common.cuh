@@ -160,3 +160,11 @@ template <typename T, int V> __device__ __forceinline__ void store_pack(T* p, co
         for (int i = 0; i < V; i++) p[i] = r.v[i];
     }
 }
+
+// 16 bytes from global to shared memory without a register in between; with `ok` false the 16 bytes are zeros and `src` is not read.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }

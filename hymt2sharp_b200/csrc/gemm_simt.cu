@@ -117,9 +117,147 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
     }
 }
 
+// Few rows of float32 (a decode step of the 32-bit engine): a block streams ROWS_N weight rows (and, for the swiglu epilogue, their
+// up rows) through a ring of ROWS_BK columns in shared memory, with the rows of A beside them; a thread owns one weight row (pair)
+// and every 8th row of A.  Every output is one chain of FMAs over ascending k, exactly as in the tile kernel, so a row's result is
+// the same bit for bit whichever kernel it meets.  What bounds it: the chain and its operands' way through shared memory (a warp's
+// 8 weight rows by 4 rows of A are one wavefront a read), for wide products also the weights' way from memory.  1.8B sizes, 8 rows:
+// gate and up (100 MB) 46 us, against 216 in tiles of 64 rows; down (50 MB) 36 against 490, whose 32 blocks of tiles walked all
+// of K with two barriers every 16 columns; q/k/v 23 against 170, O 15 against 205.  Computing with one or two warps of 2 x 2 entries
+// a thread took 39 and 71 (a warp issues one such read in six cycles).
+constexpr int ROWS_N = 16, ROWS_THREADS = 128, ROWS_BK = 128, ROWS_LD = ROWS_BK + 4, ROWS_MAX_M = 64;
+
+__host__ __device__ constexpr int rows_stage_floats(int mp, int nb) { return (nb * ROWS_N + mp) * ROWS_LD; }
+__host__ __device__ constexpr int rows_stages(int mp, int nb) {
+    const int fit = 75 * 1024 / (4 * rows_stage_floats(mp, nb));      // three blocks an SM
+    return fit < 3 ? 3 : (fit > 8 ? 8 : fit);
+}
+
+template <int MP, int EPI>
+__global__ void __launch_bounds__(ROWS_THREADS)
+gemm_rows_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, long lda, long ldw,
+                 long ldc, GluRule glu) {
+    constexpr int NB = EPI == EPI_SWIGLU ? 2 : 1, PM = MP / 8, STAGES = rows_stages(MP, NB), WR = NB * ROWS_N;
+    constexpr int CHUNK = PM == 1 ? 4 : (PM == 2 ? 2 : 1);    // pieces of four columns that are read ahead
+    extern __shared__ __align__(16) float ring[];       // STAGES x (weight rows, then rows of A) of ROWS_LD floats
+    const int tid = threadIdx.x, n0 = blockIdx.x * ROWS_N;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int col = (warp & 1) * 8 + (lane & 7), mg = (warp >> 1) * 4 + (lane >> 3);
+    const int steps = (K + ROWS_BK - 1) / ROWS_BK;
+    // The weights' first columns are asked into L2 while the kernel in front still runs (a hint: it cannot read anything too early).
+    for (int i = tid; i < WR * STAGES * (ROWS_BK / 32); i += ROWS_THREADS) {
+        const int r = i % WR, k = (i / WR) * 32, n = n0 + r % ROWS_N;
+        if (n < N && k < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + ((size_t)(r / ROWS_N) * N + n) * ldw + k));
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int PIECES = ROWS_BK / 4;
+    const int lr = tid / PIECES, lx = (tid % PIECES) * 4;                 // loader: a warp a row of 128 columns
+    auto fetch = [&](int step) {
+        float* dst = ring + (size_t)(step % STAGES) * rows_stage_floats(MP, NB) + lx;
+        const int k = step * ROWS_BK + lx;
+        const bool in = k < K;
+#pragma unroll
+        for (int r = 0; r < WR; r += ROWS_THREADS / PIECES) {
+            const int n = n0 + (lr + r) % ROWS_N;
+            const bool ok = in && n < N;
+            cp_async16(dst + (lr + r) * ROWS_LD, ok ? W + ((size_t)((lr + r) / ROWS_N) * N + n) * ldw + k : W, ok);
+        }
+        for (int r = lr; r < M; r += ROWS_THREADS / PIECES) cp_async16(dst + (WR + r) * ROWS_LD, in ? A + (size_t)r * lda + k : A, in);
+    };
+    float acc[NB][PM];
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+        for (int i = 0; i < PM; i++) acc[b][i] = 0.f;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++) {
+        if (s < steps) fetch(s);
+        cp_async_commit();
+    }
+    for (int step = 0; step < steps; step++) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();      // this step's columns have landed for every thread, and the step before is no longer read
+        if (step + STAGES - 1 < steps) fetch(step + STAGES - 1);
+        cp_async_commit();
+        const float* base = ring + (size_t)(step % STAGES) * rows_stage_floats(MP, NB);
+        const float* wp = base + col * ROWS_LD;
+        const float* ap = base + (WR + mg) * ROWS_LD;
+        if (mg >= M) continue;
+        // (rows of A from M on: whatever the ring holds there, for sums that nobody reads)
+        float4 w[2][CHUNK][NB], a[2][CHUNK][PM];
+        auto read = [&](int to, int k) {
+#pragma unroll
+            for (int c = 0; c < CHUNK; c++) {
+#pragma unroll
+                for (int b = 0; b < NB; b++) w[to][c][b] = *reinterpret_cast<const float4*>(wp + b * ROWS_N * ROWS_LD + k + 4 * c);
+#pragma unroll
+                for (int i = 0; i < PM; i++) a[to][c][i] = *reinterpret_cast<const float4*>(ap + i * 8 * ROWS_LD + k + 4 * c);
+            }
+        };
+        read(0, 0);
+#pragma unroll
+        for (int k = 0; k < ROWS_BK; k += 4 * CHUNK) {
+            const int now = (k / (4 * CHUNK)) & 1;
+            if (k + 4 * CHUNK < ROWS_BK) read(now ^ 1, k + 4 * CHUNK);
+#pragma unroll
+            for (int c = 0; c < CHUNK; c++)
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+#pragma unroll
+                    for (int b = 0; b < NB; b++)
+#pragma unroll
+                        for (int i = 0; i < PM; i++)
+                            acc[b][i] = fmaf(reinterpret_cast<const float*>(&a[now][c][i])[x], reinterpret_cast<const float*>(&w[now][c][b])[x], acc[b][i]);
+        }
+    }
+    const int n = n0 + col;
+    if (n >= N) return;
+#pragma unroll
+    for (int i = 0; i < PM; i++) {
+        const int m = mg + 8 * i;
+        if (m >= M) continue;
+        float* c = C + (size_t)m * ldc + n;
+        if constexpr (EPI == EPI_STORE) *c = acc[0][i];
+        else if constexpr (EPI == EPI_ACCUMULATE) *c = *c + acc[0][i];
+        else *c = glu_at(glu, acc[0][i], acc[NB - 1][i], n, N);
+    }
+}
+
+template <int MP, int EPI>
+int launch_rows(float* C, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldc, GluRule glu, cudaStream_t stream) {
+    constexpr int NB = EPI == EPI_SWIGLU ? 2 : 1;
+    constexpr int smem = rows_stages(MP, NB) * rows_stage_floats(MP, NB) * 4;
+    static_assert(smem <= 227 * 1024, "the ring fits a block's shared memory");
+    cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<MP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) { hymt2_set_error("gemm_rows: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
+    launch_pdl(gemm_rows_kernel<MP, EPI>, dim3((N + ROWS_N - 1) / ROWS_N), dim3(ROWS_THREADS), smem, stream, C, A, W, M, N, K, lda, ldw, ldc, glu);
+    return hymt2_check_launch("gemm_rows");
+}
+
+template <int EPI>
+int launch_rows_for(float* C, const float* A, const float* W, int M, int N, int K, long lda, long ldw, long ldc, GluRule glu, cudaStream_t stream) {
+    if (M <= 8) return launch_rows<8, EPI>(C, A, W, M, N, K, lda, ldw, ldc, glu, stream);
+    if (M <= 16) return launch_rows<16, EPI>(C, A, W, M, N, K, lda, ldw, ldc, glu, stream);
+    if (M <= 32) return launch_rows<32, EPI>(C, A, W, M, N, K, lda, ldw, ldc, glu, stream);
+    return launch_rows<64, EPI>(C, A, W, M, N, K, lda, ldw, ldc, glu, stream);
+}
+
 template <typename TA, typename TW, typename TC>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda, long ldw, long ldc, int epi,
            cudaStream_t stream, int batch = 1, long a_bs = 0, long w_bs = 0, long c_bs = 0, GluRule glu = GluRule{}) {
+    if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TC) == 4) {
+        // few rows whose pieces of 16 bytes lie on their boundaries (33 to 64 of them only while the weight rows' blocks are all resident
+        // at twice an SM: 64 rows against 2,048 x 2,048 take 37 us there and 92 in tiles, against 12,288 x 2,048 195 and 126)
+        if ((M <= 32 || (M <= ROWS_MAX_M && N <= 296 * ROWS_N)) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+            (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
+            float* c = (float*)C;
+            const float *a = (const float*)A, *w = (const float*)W;
+            if (epi == EPI_STORE) return launch_rows_for<EPI_STORE>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
+            if (epi == EPI_ACCUMULATE) return launch_rows_for<EPI_ACCUMULATE>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
+            return launch_rows_for<EPI_SWIGLU>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
+        }
+    }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
     const bool vec_a = (lda % 4 == 0) && ((uintptr_t)A % 16 == 0) && (a_bs * sizeof(TA)) % 16 == 0;
     const bool vec_w = (ldw % 4 == 0) && ((uintptr_t)W % 16 == 0) && (w_bs * sizeof(TW)) % 16 == 0;
