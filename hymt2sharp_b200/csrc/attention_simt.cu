@@ -213,6 +213,381 @@ attention_simt_kernel(AttnParams p) {
     }
 }
 
+// ---- float32, keys and values of one width, nothing but the mask: the 32-bit engine's prompts and decode steps ----------------
+// Two kernels for that form.  Both compute what the kernel above computes, in the same order bit for bit: a score is one chain of
+// FMAs over ascending entries, keys come in tiles of 32 from a multiple of 32, a tile's sum is that of the eight lanes' four
+// keys each, and an output entry is one chain over ascending keys.  So a row does not know which kernel it met, nor which rows it
+// shared a block with (a tile that is masked for a row leaves it as it was).  Keys and values arrive by cp.async, 16 bytes at a
+// time, while the tile before is worked on.
+constexpr int PLAIN_THREADS = 128, PLAIN_P_LD = KEY_TILE + 4;
+
+// The tile of keys and values from position k0 on into shared memory [KEY_TILE][d + 4] each; keys past the sequence are zeros.
+__device__ __forceinline__ void plain_fetch_tile(const AttnParams& p, const int* table, int kvh, int k0, int kv_len, float* ks, float* vs) {
+    const int block = table[k0 / p.block_tokens], valid = block >= 0 ? min(KEY_TILE, kv_len - k0) : 0;
+    const size_t base = block >= 0 ? (((size_t)block * p.nkv + kvh) * p.block_tokens + (k0 % p.block_tokens)) * p.d : 0;
+    const float *kp = (const float*)p.k_cache + base, *vp = (const float*)p.v_cache + base;
+    const int pieces = p.d / 4, ld = p.d + 4;
+    for (int i = threadIdx.x; i < KEY_TILE * pieces; i += PLAIN_THREADS) {
+        const int j = i / pieces, x = (i - j * pieces) * 4;
+        const bool ok = j < valid;
+        cp_async16(ks + j * ld + x, kp + (ok ? j * p.d + x : 0), ok);
+        cp_async16(vs + j * ld + x, vp + (ok ? j * p.d + x : 0), ok);
+    }
+}
+
+__device__ __forceinline__ float plain_dot4(const float4& a, const float4& b, float c) {
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
+}
+
+// One token a sequence: a block is a (sequence, kv head, chunk of keys), its rows the kv head's up to 4 * RR heads.  A thread has
+// one (head, key) pair of a tile, or RR of them, then four output entries of a head.  Few rows meet each key, so the step's time
+// is that of the keys' and values' way from memory plus a chain of tiles; the ring keeps RING - 1 tiles on the way.
+// 8 sequences of up to 1,000 keys, 16 heads on 4: 20 us, against 351 in the kernel above.
+template <int RR, int DI, int RING>
+__global__ void __launch_bounds__(PLAIN_THREADS)
+attention_plain_decode_kernel(AttnParams p) {
+    extern __shared__ __align__(16) float smem[];
+    const int d = p.d, ld = d + 4, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* ring = smem;                                       // RING x (keys, values)
+    float* Qs = ring + RING * 2 * KEY_TILE * ld;              // [4 * RR][ld]
+    float* Ps = Qs + 4 * RR * ld;                             // [4 * RR][PLAIN_P_LD]: scores, then what they become
+    float* Cs = Ps + 4 * RR * PLAIN_P_LD;                     // [4 * RR]: a tile's correction of a row
+    pdl_wait();
+    pdl_launch_dependents();
+    const int b = blockIdx.z / p.max_splits, split = blockIdx.z % p.max_splits;
+    const int slot = p.slot_ids[b];
+    if (slot < 0) return;
+    const int tok0 = p.cu_seqlens[b];
+    if (p.cu_seqlens[b + 1] <= tok0) return;
+    const int kv_len = p.kv_lens[b], pos = kv_len - 1;
+    const int g = p.nh / p.nkv, kvh = blockIdx.y / p.head_chunks, head0 = kvh * g + (blockIdx.y % p.head_chunks) * p.heads_per_tile;
+    const int rows = min(p.heads_per_tile, (kvh + 1) * g - head0);
+    const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+    int key_begin = lo, key_end = kv_len;
+    if (p.split_keys > 0) {
+        key_begin = max(key_begin, split * p.split_keys);
+        key_end = min(key_end, (split + 1) * p.split_keys);
+    }
+    const int first = (key_begin / KEY_TILE) * KEY_TILE;
+    const int tiles = key_end > first ? (key_end - first + KEY_TILE - 1) / KEY_TILE : 0;
+    const int* table = p.block_table + (size_t)slot * p.table_stride;
+    const int tile_floats = KEY_TILE * ld;
+#pragma unroll
+    for (int t = 0; t < RING - 1; t++) {
+        if (t < tiles) plain_fetch_tile(p, table, kvh, first + t * KEY_TILE, kv_len, ring + t * 2 * tile_floats, ring + (t * 2 + 1) * tile_floats);
+        cp_async_commit();
+    }
+    const float* q = (const float*)p.q + ((size_t)tok0 * p.nh + head0) * d;
+    for (int i = tid; i < 4 * RR * d; i += PLAIN_THREADS) {
+        const int r = i / d, x = i - r * d;
+        Qs[r * ld + x] = r < rows ? q[(size_t)r * d + x] : 0.f;
+    }
+    const int r4 = lane >> 3, part = warp * 8 + (lane & 7);   // rows r4 + 4 * rr; key `part` of a tile, then entries 4 * (part + 32 * i)
+    float4 acc[RR][DI];
+#pragma unroll
+    for (int rr = 0; rr < RR; rr++)
+#pragma unroll
+        for (int i = 0; i < DI; i++) acc[rr][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float m[RR], l[RR];                                       // of row warp + 4 * rr
+#pragma unroll
+    for (int rr = 0; rr < RR; rr++) { m[rr] = -INFINITY; l[rr] = 0.f; }
+    for (int t = 0; t < tiles; t++) {
+        cp_async_wait<RING - 2>();
+        __syncthreads();
+        if (t + RING - 1 < tiles) {
+            float* dst = ring + ((t + RING - 1) % RING) * 2 * tile_floats;
+            plain_fetch_tile(p, table, kvh, first + (t + RING - 1) * KEY_TILE, kv_len, dst, dst + tile_floats);
+        }
+        cp_async_commit();
+        const float* ks = ring + (t % RING) * 2 * tile_floats;
+        const float* vs = ks + tile_floats;
+        const int key = first + t * KEY_TILE + part;
+        const bool visible = key >= key_begin && key < key_end;
+        float dot[RR];
+#pragma unroll
+        for (int rr = 0; rr < RR; rr++) dot[rr] = 0.f;
+#pragma unroll 8
+        for (int x = 0; x < d; x += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(ks + part * ld + x);
+#pragma unroll
+            for (int rr = 0; rr < RR; rr++) dot[rr] = plain_dot4(*reinterpret_cast<const float4*>(Qs + (r4 + 4 * rr) * ld + x), k4, dot[rr]);
+        }
+#pragma unroll
+        for (int rr = 0; rr < RR; rr++) Ps[(r4 + 4 * rr) * PLAIN_P_LD + part] = visible ? dot[rr] * p.scale : -INFINITY;
+        __syncthreads();
+#pragma unroll
+        for (int rr = 0; rr < RR; rr++) {
+            float* row = Ps + (warp + 4 * rr) * PLAIN_P_LD;
+            const float s = row[lane];
+            const float m_new = fmaxf(m[rr], warp_max(s));
+            float corr = 1.f, pj = 0.f;
+            if (m_new > -INFINITY) {
+                corr = expf(m[rr] - m_new);
+                pj = expf(s - m_new);
+            }
+            const int c = lane & 7;
+            float psum = __shfl_sync(0xffffffffu, pj, c);
+#pragma unroll
+            for (int kk = 1; kk < 4; kk++) psum += __shfl_sync(0xffffffffu, pj, c + 8 * kk);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+            l[rr] = l[rr] * corr + psum;
+            m[rr] = m_new;
+            row[lane] = pj;
+            if (lane == 0) Cs[warp + 4 * rr] = corr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < DI; i++) {
+            const int x = 4 * (part + 32 * i);
+            if (x < d) {
+#pragma unroll
+                for (int rr = 0; rr < RR; rr++) {
+                    const float corr = Cs[r4 + 4 * rr];
+                    acc[rr][i].x *= corr; acc[rr][i].y *= corr; acc[rr][i].z *= corr; acc[rr][i].w *= corr;
+                }
+#pragma unroll 8
+                for (int j = 0; j < KEY_TILE; j++) {
+                    const float4 v = *reinterpret_cast<const float4*>(vs + j * ld + x);
+#pragma unroll
+                    for (int rr = 0; rr < RR; rr++) {
+                        const float pj = Ps[(r4 + 4 * rr) * PLAIN_P_LD + j];
+                        acc[rr][i].x = fmaf(pj, v.x, acc[rr][i].x); acc[rr][i].y = fmaf(pj, v.y, acc[rr][i].y);
+                        acc[rr][i].z = fmaf(pj, v.z, acc[rr][i].z); acc[rr][i].w = fmaf(pj, v.w, acc[rr][i].w);
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();                                          // (the last tile's Cs have been read)
+#pragma unroll
+    for (int rr = 0; rr < RR; rr++) {
+        const int r = warp + 4 * rr;
+        if (lane == 0) Cs[r] = l[rr] > 0.f ? 1.f / l[rr] : 0.f;
+        if (p.split_keys > 0 && lane == 0 && r < rows) {
+            float* ml = p.part_ml + (((size_t)tok0 * p.nh + head0 + r) * p.max_splits + split) * 2;
+            ml[0] = m[rr];
+            ml[1] = l[rr];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int rr = 0; rr < RR; rr++) {
+        const int r = r4 + 4 * rr;
+        if (r >= rows) continue;
+        const size_t row_index = (size_t)tok0 * p.nh + head0 + r;
+        const float inv = p.split_keys > 0 ? 1.f : Cs[r];
+        float* dst = p.split_keys > 0 ? p.part_acc + (row_index * p.max_splits + split) * d : (float*)p.out + row_index * d;
+#pragma unroll
+        for (int i = 0; i < DI; i++) {
+            const int x = 4 * (part + 32 * i);
+            if (x < d) *reinterpret_cast<float4*>(dst + x) = make_float4(acc[rr][i].x * inv, acc[rr][i].y * inv, acc[rr][i].z * inv, acc[rr][i].w * inv);
+        }
+    }
+}
+
+// Prompts: a block owns 16 * RT (token, head) rows of a kv head, eight lanes share RT of them: a lane has four keys of a tile for
+// the scores (c, c + 8, c + 16, c + 24) and pieces of four output entries (4 c, 4 c + 32, ...).  Longest tiles come first.  What
+// bounds it is the issue of FMAs and of the shared-memory reads beside them.  531 tokens, 16 heads on 4: 155 us, against 603.
+template <int RT, int DI>
+__global__ void __launch_bounds__(PLAIN_THREADS)
+attention_plain_prompt_kernel(AttnParams p) {
+    constexpr int ROWS_B = 16 * RT;
+    extern __shared__ __align__(16) float smem[];
+    const int d = p.d, ld = d + 4, tid = threadIdx.x;
+    const int tile_floats = KEY_TILE * ld;
+    float* ring = smem;                                       // 2 x (keys, values)
+    float* Qs = ring + 4 * tile_floats;                       // [ROWS_B][ld]
+    float* Ps = Qs + ROWS_B * ld;                             // [ROWS_B][PLAIN_P_LD]
+    pdl_wait();
+    pdl_launch_dependents();
+    const int b = blockIdx.z;
+    const int slot = p.slot_ids[b];
+    if (slot < 0) return;
+    const int tok0 = p.cu_seqlens[b], T_b = p.cu_seqlens[b + 1] - tok0, kv_len = p.kv_lens[b];
+    const int tile_tok0 = (gridDim.x - 1 - blockIdx.x) * p.tokens_per_tile;
+    if (tile_tok0 >= T_b) return;
+    const int g = p.nh / p.nkv, kvh = blockIdx.y / p.head_chunks, chunk = blockIdx.y % p.head_chunks;
+    const int last_tok = min(T_b, tile_tok0 + p.tokens_per_tile) - 1;
+    const int first_pos = kv_len - T_b + tile_tok0;
+    const int key_begin = p.window > 0 ? max(0, first_pos - p.window + 1) : 0, key_end = kv_len - T_b + last_tok + 1;
+    const int first = (key_begin / KEY_TILE) * KEY_TILE, tiles = (key_end - first + KEY_TILE - 1) / KEY_TILE;
+    const int* table = p.block_table + (size_t)slot * p.table_stride;
+    plain_fetch_tile(p, table, kvh, first, kv_len, ring, ring + tile_floats);
+    cp_async_commit();
+    for (int i = tid; i < ROWS_B * (d / 4); i += PLAIN_THREADS) {
+        const int r = i / (d / 4), x = (i - r * (d / 4)) * 4;
+        const int tk = tile_tok0 + r / p.heads_per_tile, hg = chunk * p.heads_per_tile + r % p.heads_per_tile;
+        const bool ok = r < p.tokens_per_tile * p.heads_per_tile && tk < T_b && hg < g;
+        *reinterpret_cast<float4*>(Qs + r * ld + x) =
+            ok ? *reinterpret_cast<const float4*>((const float*)p.q + ((size_t)(tok0 + tk) * p.nh + kvh * g + hg) * d + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int rg = tid >> 3, c = tid & 7;
+    int row_pos[RT], row_lo[RT];                              // (a row that does not exist sees nothing)
+    size_t row_index[RT];
+    float m[RT], l[RT];
+    float4 acc[RT][DI];
+#pragma unroll
+    for (int i = 0; i < RT; i++) {
+        const int r = rg + 16 * i;
+        const int tk = tile_tok0 + r / p.heads_per_tile, hg = chunk * p.heads_per_tile + r % p.heads_per_tile;
+        const bool ok = r < p.tokens_per_tile * p.heads_per_tile && tk < T_b && hg < g;
+        row_pos[i] = ok ? kv_len - T_b + tk : -1;
+        row_lo[i] = p.window > 0 ? max(0, row_pos[i] - p.window + 1) : 0;
+        row_index[i] = (size_t)(tok0 + tk) * p.nh + kvh * g + hg;
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < DI; j++) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int t = 0; t < tiles; t++) {
+        cp_async_wait<0>();
+        __syncthreads();
+        if (t + 1 < tiles) {
+            float* dst = ring + ((t + 1) & 1) * 2 * tile_floats;
+            plain_fetch_tile(p, table, kvh, first + (t + 1) * KEY_TILE, kv_len, dst, dst + tile_floats);
+        }
+        cp_async_commit();
+        const float* ks = ring + (t & 1) * 2 * tile_floats;
+        const float* vs = ks + tile_floats;
+        const int k0 = first + t * KEY_TILE;
+        float s[RT][4];
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) s[i][kk] = 0.f;
+#pragma unroll 4
+        for (int x = 0; x < d; x += 4) {
+            float4 k4[4];
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) k4[kk] = *reinterpret_cast<const float4*>(ks + (c + 8 * kk) * ld + x);
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                const float4 q4 = *reinterpret_cast<const float4*>(Qs + (rg + 16 * i) * ld + x);
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) s[i][kk] = plain_dot4(q4, k4[kk], s[i][kk]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            float tile_max = -INFINITY;
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) {
+                const int key = k0 + c + 8 * kk;
+                s[i][kk] = key >= row_lo[i] && key <= row_pos[i] ? s[i][kk] * p.scale : -INFINITY;
+                tile_max = fmaxf(tile_max, s[i][kk]);
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, o));
+            const float m_new = fmaxf(m[i], tile_max);
+            float corr = 1.f, psum = 0.f;
+            float* pr = Ps + (rg + 16 * i) * PLAIN_P_LD + c;
+            if (m_new > -INFINITY) {
+                corr = expf(m[i] - m_new);
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) {
+                    const float pj = expf(s[i][kk] - m_new);
+                    pr[8 * kk] = pj;
+                    psum += pj;
+                }
+            } else {
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) pr[8 * kk] = 0.f;
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+            l[i] = l[i] * corr + psum;
+            m[i] = m_new;
+#pragma unroll
+            for (int j = 0; j < DI; j++) { acc[i][j].x *= corr; acc[i][j].y *= corr; acc[i][j].z *= corr; acc[i][j].w *= corr; }
+        }
+        __syncwarp();                                         // (a row's eight lanes are in one warp)
+#pragma unroll 2
+        for (int j4 = 0; j4 < KEY_TILE; j4 += 4) {
+            float4 p4[RT];
+#pragma unroll
+            for (int i = 0; i < RT; i++) p4[i] = *reinterpret_cast<const float4*>(Ps + (rg + 16 * i) * PLAIN_P_LD + j4);
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+#pragma unroll
+                for (int i = 0; i < DI; i++) {
+                    const int x = 4 * c + 32 * i;
+                    if (x < d) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + (j4 + jj) * ld + x);
+#pragma unroll
+                        for (int r = 0; r < RT; r++) {
+                            const float pj = jj == 0 ? p4[r].x : jj == 1 ? p4[r].y : jj == 2 ? p4[r].z : p4[r].w;
+                            acc[r][i].x = fmaf(pj, v.x, acc[r][i].x); acc[r][i].y = fmaf(pj, v.y, acc[r][i].y);
+                            acc[r][i].z = fmaf(pj, v.z, acc[r][i].z); acc[r][i].w = fmaf(pj, v.w, acc[r][i].w);
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < RT; i++) {
+        if (row_pos[i] < 0) continue;
+        const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+#pragma unroll
+        for (int j = 0; j < DI; j++) {
+            const int x = 4 * c + 32 * j;
+            if (x < d) *reinterpret_cast<float4*>((float*)p.out + row_index[i] * d + x) =
+                make_float4(acc[i][j].x * inv, acc[i][j].y * inv, acc[i][j].z * inv, acc[i][j].w * inv);
+        }
+    }
+}
+
+template <typename K>
+int plain_launch(K kernel, dim3 grid, size_t smem, cudaStream_t stream, const AttnParams& p) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) { hymt2_set_error("attention: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
+    launch_pdl(kernel, grid, dim3(PLAIN_THREADS), smem, stream, p);
+    return hymt2_check_launch("attention_plain");
+}
+
+// Steps of one token a sequence (with or without chunks of keys).
+int plain_decode(AttnParams p, int batch, cudaStream_t stream) {
+    const int g = p.nh / p.nkv;
+    p.heads_per_tile = g < 16 ? g : 16;
+    p.head_chunks = (g + p.heads_per_tile - 1) / p.heads_per_tile;
+    const dim3 grid(1, p.nkv * p.head_chunks, batch * p.max_splits);
+    HYMT2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "attention: grid too large (batch %d x splits %d)", batch, p.max_splits);
+    const int rr = (p.heads_per_tile + 3) / 4, ring = p.d <= 128 ? 4 : 2;
+    const size_t smem = sizeof(float) * ((size_t)(ring * 2 * KEY_TILE + 4 * rr) * (p.d + 4) + 4 * rr * (PLAIN_P_LD + 1));
+#define PLAIN_DECODE(RR) (p.d <= 128 ? plain_launch(attention_plain_decode_kernel<RR, 1, 4>, grid, smem, stream, p) \
+                                     : plain_launch(attention_plain_decode_kernel<RR, 2, 2>, grid, smem, stream, p))
+    if (rr == 1) return PLAIN_DECODE(1);
+    if (rr == 2) return PLAIN_DECODE(2);
+    if (rr == 3) return PLAIN_DECODE(3);
+    return PLAIN_DECODE(4);
+#undef PLAIN_DECODE
+}
+
+template <int RT>
+int plain_prompt_rows(AttnParams p, int batch, int max_new_tokens, cudaStream_t stream) {
+    const dim3 grid((max_new_tokens + p.tokens_per_tile - 1) / p.tokens_per_tile, p.nkv * p.head_chunks, batch);
+    HYMT2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "attention: grid too large (batch %d)", batch);
+    const size_t smem = sizeof(float) * ((size_t)(4 * KEY_TILE + 16 * RT) * (p.d + 4) + 16 * RT * PLAIN_P_LD);
+    if (p.d <= 32) return plain_launch(attention_plain_prompt_kernel<RT, 1>, grid, smem, stream, p);
+    if (p.d <= 64) return plain_launch(attention_plain_prompt_kernel<RT, 2>, grid, smem, stream, p);
+    if constexpr (RT == 4) return plain_launch(attention_plain_prompt_kernel<RT, 4>, grid, smem, stream, p);
+    else if (p.d <= 128) return plain_launch(attention_plain_prompt_kernel<RT, 4>, grid, smem, stream, p);
+    else return plain_launch(attention_plain_prompt_kernel<RT, 8>, grid, smem, stream, p);
+}
+
+// Prompts: the more rows a block has, the fewer reads an FMA costs; 32 rows instead of 64 while the blocks would not fill the SMs twice
+// (two blocks fit an SM), and for heads whose outputs would not fit the registers.
+int plain_prompt(AttnParams p, int batch, int tokens, int max_new_tokens, cudaStream_t stream) {
+    const int g = p.nh / p.nkv;
+    const int rt = p.d <= 128 && (long)tokens * p.nh >= 64L * 2 * 148 ? 4 : 2;
+    p.heads_per_tile = g < 16 * rt ? g : 16 * rt;
+    p.tokens_per_tile = 16 * rt / p.heads_per_tile;
+    p.head_chunks = (g + p.heads_per_tile - 1) / p.heads_per_tile;
+    return rt == 4 ? plain_prompt_rows<4>(p, batch, max_new_tokens, stream) : plain_prompt_rows<2>(p, batch, max_new_tokens, stream);
+}
+
 constexpr int MERGE_WEIGHTS = 128, MERGE_COLS = 4;
 
 inline int merge_threads(int dv) { return dv > 256 ? 256 : (dv > 128 ? 128 : 64); }
@@ -373,6 +748,18 @@ static int attention_simt_general(void* out, const void* q, const void* k_cache,
     HYMT2_REQUIRE(maps >= 1 && (maps == 1 || v_cache) && softcap >= 0.f && temp_every > 0, "attention: %d maps, a cap of %g, a temperature every %d positions",
                   maps, (double)softcap, temp_every);
     p.maps = maps; p.softcap = softcap; p.temp_coef = temp_coef; p.temp_every = temp_every;
+    // the form of the 32-bit engine's own attention, its rows on 16-byte boundaries (a chunked step of several tokens a sequence stays
+    // with the general kernel)
+    if (dtype == HYMT2_F32 && d == dv && d % 4 == 0 && d <= MAX_D && v_cache && maps == 1 && !p.sink && softcap == 0.f && temp_coef == 0.f &&
+        (split_keys == 0 || max_new_tokens == 1) && (uintptr_t)q % 16 == 0 && (uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0 &&
+        (uintptr_t)out % 16 == 0 && (uintptr_t)part_acc % 16 == 0) {
+        int prc = max_new_tokens == 1 ? plain_decode(p, batch, stream) : plain_prompt(p, batch, tokens, max_new_tokens, stream);
+        if (prc == HYMT2_OK && split_keys > 0) {
+            launch_pdl(attention_merge_kernel<float>, dim3(tokens * nh), dim3(merge_threads(dv)), 0, stream, p, tokens);
+            prc = hymt2_check_launch("attention_merge");
+        }
+        return prc;
+    }
     const size_t smem = sizeof(float) * ((size_t)ROWS * d + (size_t)KEY_TILE * (d + 1) + (v_cache ? (size_t)KEY_TILE * dv : 0) + ROWS * KEY_TILE);
     dim3 grid((max_new_tokens + p.tokens_per_tile - 1) / p.tokens_per_tile, nkv * p.head_chunks * maps, batch * p.max_splits);
     HYMT2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "attention: grid too large (batch %d x splits %d)", batch, p.max_splits);

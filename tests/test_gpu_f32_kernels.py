@@ -1,12 +1,14 @@
-"""The kernels of the 32-bit path at the sizes where their tiles end: the products for few rows and in tiles.  Every sum keeps one
+"""The kernels of the 32-bit path at the sizes where their tiles end: the products for few rows and in tiles, and the attention of
+its plain form.  Every sum keeps one
 order whichever kernel runs, so the kernels are compared with each other bit for bit, and with 64-bit sums within the bound of a
 chain of K float32 FMAs, K * 2^-24 * sum |a| |w| (twice that, for the add into the output)."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
-from test_gpu_kernels import DEV, _ops
+from test_gpu_kernels import DEV, _ops, _paged
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +42,30 @@ def test_products_of_few_rows_and_in_tiles_agree_bit_for_bit(M, N, K):
             assert ((outs[0].double() - ref[:, :N]).abs() <= bound[:, :N]).all()
         elif epilogue == ops.EPILOGUE_ACCUMULATE:
             assert ((outs[0].double() - base.double() - ref[:, :N]).abs() <= bound[:, :N] + 2.0 ** -23 * (base.double().abs() + ref[:, :N].abs())).all()
+
+
+@pytest.mark.parametrize("nh, nkv, d, window", [(4, 4, 128, 0), (16, 2, 128, 0), (6, 2, 40, 0), (20, 1, 64, 50), (5, 1, 256, 100), (8, 2, 8, 0), (64, 1, 128, 0)])
+@pytest.mark.parametrize("news", [[1, 1, 1, 1], [70, 1, 45, 300]])
+def test_attention_of_the_plain_form_is_the_general_kernels_bit_for_bit(nh, nkv, d, window, news):
+    ops = _ops()
+    torch.manual_seed(nh * 100 + d)
+    lens = [700, 1, 257, 320]
+    keys = [torch.randn(L, nkv, d, device=DEV) for L in lens]
+    vals = [torch.randn(L, nkv, d, device=DEV) for L in lens]
+    kp, vp, table = _paged(keys, vals, 64, torch.float32)
+    T = sum(news)
+    q = torch.randn(T, nh * d, device=DEV)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(news)]), dtype=torch.int32, device=DEV)
+    slots, kv = torch.tensor([0, 1, -1, 3], dtype=torch.int32, device=DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    for split in ((0, 256) if max(news) == 1 else (0,)):
+        splits = -(-max(lens) // 256) if split else 0
+        scratch = (None, None)
+        if split:
+            scratch = tuple(torch.full((n,), float("nan"), device=DEV) for n in ops.attention_simt_scratch(T, nh, d, splits))
+        outs = []
+        for x in (q, _shifted(q)):       # (the second takes the general kernel)
+            out = torch.full((T, nh * d), 5.0, device=DEV)
+            ops.attention_simt(out, x, kp, vp, table, cu, slots, kv, 4, max(news), nh, nkv, d, 1 / math.sqrt(d), window, split, splits, *scratch)
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1])
+        assert (outs[0][sum(news[:2]):sum(news[:3])] == 5.0).all()      # a padding row is left alone
