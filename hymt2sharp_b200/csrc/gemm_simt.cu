@@ -14,6 +14,7 @@
 
 namespace {
 
+// the grouped product's tiles (64 x 64, four by four a thread); BK is the tile kernels' step
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, THREADS = 256;
 
 enum { EPI_STORE = 0, EPI_ACCUMULATE = 1, EPI_SWIGLU = 2 };
@@ -36,83 +37,120 @@ __device__ __forceinline__ void load4(const T* row, int k, int K, bool row_ok, b
     }
 }
 
-template <typename TA, typename TW, typename TC, int EPI>
-__global__ void __launch_bounds__(THREADS)
+template <typename TC, int EPI>
+__device__ __forceinline__ void finish(TC* c, float acc, float up, const GluRule& glu, int n, int N) {
+    if constexpr (EPI == EPI_STORE) *c = from_float<TC>(acc);
+    else if constexpr (EPI == EPI_ACCUMULATE) *c = from_float<TC>(to_float(*c) + acc);
+    else *c = from_float<TC>(glu_at(glu, acc, up, n, N));
+}
+
+// Tiles of TILE_M rows of A by TILE_N weight rows (for the swiglu epilogue half of them gate rows, half their up rows).  A warp
+// owns 4 * PM x 8 * PN entries, a thread PM x PN of them, two rows of A to an FMA instruction: its PM entries of A and PN of W a k
+// are shared-memory reads that most of the warp's lanes have in common.  The next step's 16 columns are on their way to registers
+// while this step's are worked on; shared memory has two buffers, so a step has one barrier.  What bounds it: the FMA pipe (74
+// TFLOP/s) and the issue of what feeds it.  531 rows against 12,288 x 2,048 (gate and up of the 1.8B sizes): 606 us; 4 x 4 entries a
+// thread, one buffer and single-word reads, which this replaced, took 769.  Also measured there: plain FMAs 684, 8 x 8 entries
+// with 128 threads 650 to 700, 8 x 16 668, W stored twice for the pairs 838.
+template <typename TA, typename TW, typename TC, int EPI, int TILE_M, int TILE_N, int PM, int PN>
+__global__ void __launch_bounds__(TILE_M* TILE_N / (PM * PN))
 gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restrict__ W, int M, int N, int K,
                  long lda, long ldw, long ldc, bool vec_a, bool vec_w, long a_bs, long w_bs, long c_bs, GluRule glu) {
-    constexpr int NB = EPI == EPI_SWIGLU ? 2 : 1;
+    constexpr int NB = EPI == EPI_SWIGLU ? 2 : 1, NT = TILE_M * TILE_N / (PM * PN), COLS = TILE_N / NB, PC = PN / NB;
+    constexpr int WARPS_N = TILE_N / (8 * PN);
+    constexpr int LDA = TILE_M + 4, LDW = TILE_N + 4;
+    constexpr int PIECES_A = TILE_M * BK / 4 / NT, PIECES_W = TILE_N * BK / 4 / NT;
+    static_assert(PIECES_A * NT * 4 == TILE_M * BK && PIECES_W * NT * 4 == TILE_N * BK, "whole pieces a thread");
     // a batch of products with the same sizes: blockIdx.z picks the operands (strides in elements)
     A += (size_t)blockIdx.z * a_bs;
     W += (size_t)blockIdx.z * w_bs;
     C += (size_t)blockIdx.z * c_bs;
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[NB][BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int lrow = tid >> 2, lk = (tid & 3) * 4;  // loader: 64 rows x 4 groups of 4 k
-    const int tm = (tid >> 4) * TM, tn = (tid & 15) * TN;
+    __shared__ __align__(16) float As[2][BK][LDA];
+    __shared__ __align__(16) float Ws[2][BK][LDW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * COLS;
+    const int tm = (warp / WARPS_N) * 4 * PM + (lane >> 3) * PM;
+    const int tx = (warp % WARPS_N) * 8 + (lane & 7);      // this thread's columns: tx * PC + [0, PC) of every half
+    const int lk = (tid & 3) * 4;                          // loader: a row's 4 groups of 4 k side by side
 
-    float acc[NB][TM][TN];
+    uint64_t acc[NB][PM / 2][PC];                          // rows tm + 2 i and tm + 2 i + 1
 #pragma unroll
     for (int b = 0; b < NB; b++)
 #pragma unroll
-        for (int i = 0; i < TM; i++)
+        for (int i = 0; i < PM / 2; i++)
 #pragma unroll
-            for (int j = 0; j < TN; j++) acc[b][i][j] = 0.f;
+            for (int j = 0; j < PC; j++) acc[b][i][j] = 0;
 
-    const bool a_ok = m0 + lrow < M, w_ok = n0 + lrow < N;
-    const TA* a_row = A + (size_t)(a_ok ? m0 + lrow : 0) * lda;
-    const TW* w_row[NB];
+    const TA* a_row[PIECES_A];
+    const TW* w_row[PIECES_W];
+    bool a_ok[PIECES_A], w_ok[PIECES_W];
 #pragma unroll
-    for (int b = 0; b < NB; b++) w_row[b] = W + ((size_t)b * N + (w_ok ? n0 + lrow : 0)) * ldw;
-
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        float va[4], vw[NB][4];
-        load4(a_row, k0 + lk, K, a_ok, vec_a, va);
+    for (int i = 0; i < PIECES_A; i++) {
+        const int m = m0 + (tid >> 2) + i * (NT / 4);
+        a_ok[i] = m < M;
+        a_row[i] = A + (size_t)(a_ok[i] ? m : 0) * lda;
+    }
 #pragma unroll
-        for (int b = 0; b < NB; b++) load4(w_row[b], k0 + lk, K, w_ok, vec_w, vw[b]);
+    for (int i = 0; i < PIECES_W; i++) {
+        const int r = (tid >> 2) + i * (NT / 4), n = n0 + r % COLS;
+        w_ok[i] = n < N;
+        w_row[i] = W + ((size_t)(r / COLS) * N + (w_ok[i] ? n : 0)) * ldw;
+    }
+    float va[PIECES_A][4], vw[PIECES_W][4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < PIECES_A; i++) load4(a_row[i], k0 + lk, K, a_ok[i], vec_a, va[i]);
+#pragma unroll
+        for (int i = 0; i < PIECES_W; i++) load4(w_row[i], k0 + lk, K, w_ok[i], vec_w, vw[i]);
+    };
+    fetch(0);
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += BK, buf ^= 1) {
+        // (the buffer written here was last read two steps ago, in front of the barrier of the step between)
+#pragma unroll
+        for (int i = 0; i < PIECES_A; i++)
+#pragma unroll
+            for (int x = 0; x < 4; x++) As[buf][lk + x][(tid >> 2) + i * (NT / 4)] = va[i][x];
+#pragma unroll
+        for (int i = 0; i < PIECES_W; i++)
+#pragma unroll
+            for (int x = 0; x < 4; x++) Ws[buf][lk + x][(tid >> 2) + i * (NT / 4)] = vw[i][x];
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            As[lk + i][lrow] = va[i];
-#pragma unroll
-            for (int b = 0; b < NB; b++) Ws[b][lk + i][lrow] = vw[b][i];
-        }
-        __syncthreads();
+        if (k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            float a[TM], w[NB][TN];
+            uint64_t a[PM / 2];
+            float w[NB][PC];
 #pragma unroll
-            for (int i = 0; i < TM; i++) a[i] = As[kk][tm + i];
+            for (int i = 0; i < PM / 2; i += 2) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][tm + 2 * i]);
+                a[i] = v.x; a[i + 1] = v.y;
+            }
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const float* src = &Ws[buf][kk][b * COLS + tx * PC];
+                if constexpr (PC == 4) *reinterpret_cast<float4*>(w[b]) = *reinterpret_cast<const float4*>(src);
+                else *reinterpret_cast<float2*>(w[b]) = *reinterpret_cast<const float2*>(src);
+            }
 #pragma unroll
             for (int b = 0; b < NB; b++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) w[b][j] = Ws[b][kk][tn + j];
+                for (int j = 0; j < PC; j++) {
+                    const uint64_t ww = pack2(w[b][j], w[b][j]);
 #pragma unroll
-            for (int b = 0; b < NB; b++)
-#pragma unroll
-                for (int i = 0; i < TM; i++)
-#pragma unroll
-                    for (int j = 0; j < TN; j++) acc[b][i][j] = fmaf(a[i], w[b][j], acc[b][i][j]);
+                    for (int i = 0; i < PM / 2; i++) acc[b][i][j] = fma2(a[i], ww, acc[b][i][j]);
+                }
         }
     }
 
 #pragma unroll
-    for (int i = 0; i < TM; i++) {
+    for (int i = 0; i < PM; i++) {
         const int m = m0 + tm + i;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < TN; j++) {
-            const int n = n0 + tn + j;
-            if (n >= N) continue;
-            TC* c = C + (size_t)m * ldc + n;
-            if constexpr (EPI == EPI_STORE) {
-                *c = from_float<TC>(acc[0][i][j]);
-            } else if constexpr (EPI == EPI_ACCUMULATE) {
-                *c = from_float<TC>(to_float(*c) + acc[0][i][j]);
-            } else {
-                *c = from_float<TC>(glu_at(glu, acc[0][i][j], acc[NB - 1][i][j], n, N));
-            }
+        for (int j = 0; j < PC; j++) {
+            const int n = n0 + tx * PC + j;
+            const float2 v = unpack2(acc[0][i / 2][j]), u = unpack2(acc[NB - 1][i / 2][j]);
+            if (n < N) finish<TC, EPI>(C + (size_t)m * ldc + n, i & 1 ? v.y : v.x, i & 1 ? u.y : u.x, glu, n, N);
         }
     }
 }
@@ -243,6 +281,39 @@ int launch_rows_for(float* C, const float* A, const float* W, int M, int N, int 
     return launch_rows<64, EPI>(C, A, W, M, N, K, lda, ldw, ldc, glu, stream);
 }
 
+// Which tiles: the ones whose busiest SM has the least to do.  A wave of blocks costs an SM its tiles' entries; smaller tiles read
+// shared memory more often per FMA (531 rows: an entry of 64 x 64 costs 1.05 and of 32 x 64 1.35 of one of 64 x 128).
+inline int pick_tile(int M, int N, int NB, int batch) {
+    const int tm[3] = {64, 64, 32}, tn[3] = {128, 64, 64};
+    const double cost[3] = {1.0, 1.05, 1.35};
+    int best = 0;
+    double least = 0.0;
+    for (int i = 0; i < 3; i++) {
+        const long blocks = (long)((M + tm[i] - 1) / tm[i]) * ((N + tn[i] / NB - 1) / (tn[i] / NB)) * batch;
+        const double c = (double)((blocks + 147) / 148) * tm[i] * tn[i] * cost[i];
+        if (i == 0 || c < least) { best = i; least = c; }
+    }
+    return best;
+}
+
+template <typename TA, typename TW, typename TC, int EPI>
+int launch_tiles(TC* C, const TA* A, const TW* W, int M, int N, int K, long lda, long ldw, long ldc, cudaStream_t stream, int batch,
+                 long a_bs, long w_bs, long c_bs, GluRule glu) {
+    constexpr int NB = EPI == EPI_SWIGLU ? 2 : 1;
+    const bool vec_a = (lda % 4 == 0) && ((uintptr_t)A % 16 == 0) && (a_bs * sizeof(TA)) % 16 == 0;
+    const bool vec_w = (ldw % 4 == 0) && ((uintptr_t)W % 16 == 0) && (w_bs * sizeof(TW)) % 16 == 0;
+#define HYMT2_GEMM_TILE(BM_, BN_, PM_, PN_)                                                                                            \
+    gemm_simt_kernel<TA, TW, TC, EPI, BM_, BN_, PM_, PN_><<<dim3((N + BN_ / NB - 1) / (BN_ / NB), (M + BM_ - 1) / BM_, batch),         \
+                                                            BM_ * BN_ / (PM_ * PN_), 0, stream>>>(                                     \
+        C, A, W, M, N, K, lda, ldw, ldc, vec_a, vec_w, a_bs, w_bs, c_bs, glu)
+    const int tile = pick_tile(M, N, NB, batch);
+    if (tile == 0) HYMT2_GEMM_TILE(64, 128, 8, 4);
+    else if (tile == 1) HYMT2_GEMM_TILE(64, 64, 8, 4);
+    else HYMT2_GEMM_TILE(32, 64, 4, 4);
+#undef HYMT2_GEMM_TILE
+    return hymt2_check_launch("gemm_simt");
+}
+
 template <typename TA, typename TW, typename TC>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda, long ldw, long ldc, int epi,
            cudaStream_t stream, int batch = 1, long a_bs = 0, long w_bs = 0, long c_bs = 0, GluRule glu = GluRule{}) {
@@ -258,17 +329,11 @@ int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda,
             return launch_rows_for<EPI_SWIGLU>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
         }
     }
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-    const bool vec_a = (lda % 4 == 0) && ((uintptr_t)A % 16 == 0) && (a_bs * sizeof(TA)) % 16 == 0;
-    const bool vec_w = (ldw % 4 == 0) && ((uintptr_t)W % 16 == 0) && (w_bs * sizeof(TW)) % 16 == 0;
-#define HYMT2_GEMM_CASE(E)                                                                                  \
-    gemm_simt_kernel<TA, TW, TC, E><<<grid, THREADS, 0, stream>>>((TC*)C, (const TA*)A, (const TW*)W, M, N, K, \
-                                                                  lda, ldw, ldc, vec_a, vec_w, a_bs, w_bs, c_bs, glu)
-    if (epi == EPI_STORE) HYMT2_GEMM_CASE(EPI_STORE);
-    else if (epi == EPI_ACCUMULATE) HYMT2_GEMM_CASE(EPI_ACCUMULATE);
-    else HYMT2_GEMM_CASE(EPI_SWIGLU);
+#define HYMT2_GEMM_CASE(E) launch_tiles<TA, TW, TC, E>((TC*)C, (const TA*)A, (const TW*)W, M, N, K, lda, ldw, ldc, stream, batch, a_bs, w_bs, c_bs, glu)
+    if (epi == EPI_STORE) return HYMT2_GEMM_CASE(EPI_STORE);
+    if (epi == EPI_ACCUMULATE) return HYMT2_GEMM_CASE(EPI_ACCUMULATE);
+    return HYMT2_GEMM_CASE(EPI_SWIGLU);
 #undef HYMT2_GEMM_CASE
-    return hymt2_check_launch("gemm_simt");
 }
 
 
