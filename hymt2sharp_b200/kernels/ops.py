@@ -31,16 +31,37 @@ def dtype_code(t: torch.dtype) -> int:
 _library = None
 
 
+# The functions that a prompt's step calls layer after layer, with the types of their arguments: such a call takes Python's own
+# numbers (an address, a stream's handle) as they are, where an undeclared one wants a ctypes object built around each of its
+# thirty.  A short prompt's step is as long as the host takes to launch it.  p: address, i: int, l: long, f: float.
+_DECLARED = {"hymt2_gemm_tc_norm": "pippiiilllipl" "pippp" "iifppip" "iffp",
+             "hymt2_gemm_tc_rope_kv": "ppiillpppp" "iipppppipp" "ifiiipppiif",
+             "hymt2_attention_prefill_tc": "pppplpiipppiiiiiifipp"}
+
+
 def _lib():
     global _library
     if _library is None:
-        _library = load_library()
+        library = load_library()
+        kinds = {"p": c_void_p, "i": c_int, "l": c_long, "f": c_float}
+        for name, types in _DECLARED.items():
+            getattr(library, name).argtypes = [kinds[t] for t in types]
+        _library = library
     return _library
 
 
-def _stream() -> c_void_p:
+def _raw_stream() -> int:
     # (the raw handle: torch.cuda.current_stream() builds a Stream object for it, ten times the cost, once per launch)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _stream() -> c_void_p:
+    return c_void_p(_raw_stream())
+
+
+def _address(t: torch.Tensor | None) -> int:
+    """An argument of a declared function."""
+    return 0 if t is None else t.data_ptr()
 
 
 def _ptr(t: torch.Tensor | None) -> c_void_p:
@@ -312,9 +333,12 @@ class GluRule:
 
 GLU_KINDS = {"silu": 0, "clamped": 1}
 GLU_SILU = GluRule()
+_GLU_PLAIN = (c_int(0), c_float(0.0), c_float(1.0), c_void_p(0))   # what _glu_arguments gives for the plain rule without a bias
 
 
 def _glu_arguments(glu: GluRule | None, bias: torch.Tensor | None, n: int, epilogue: int, with_bias: bool = True) -> tuple:
+    if glu is None and bias is None:
+        return _GLU_PLAIN if with_bias else _GLU_PLAIN[:3]
     glu = glu or GLU_SILU
     if bias is not None:
         _f32(bias, "glu bias", 2 * n)
@@ -464,12 +488,10 @@ def gemm_tc(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int, 
         _need(normed, "normed", torch.bfloat16, 2); _need(gain, "gain", None, 1); _need(ss_out, "ss_out", torch.float32, 2)
         if tiles == 0 or normed.shape != (T, N) or gain.shape[0] != N or ss_out.shape != (T, tiles) or out.dtype != torch.float32:
             raise KernelError(f"gemm_tc: norm_after does not fit T={T} N={N} K={K} epilogue {epilogue} (tiles {tiles})")
-    _check(_lib().hymt2_gemm_tc_norm(_ptr(out), c_int(dtype_code(out.dtype)), _ptr(a), _ptr(w), c_int(T), c_int(N), c_int(K),
-                                     c_long(a.stride(0)), c_long(w.stride(0)), c_long(out.stride(0)), c_int(epilogue),
-                                     _ptr(ws), c_long(ws.numel() if ws is not None else 0), _ptr(cnt),
-                                     c_int(cnt.numel() if cnt is not None else 0), _ptr(status), _stream(),
-                                     _ptr(ss_in), c_int(tiles_in), c_int(width), c_float(eps), _ptr(normed), _ptr(gain),
-                                     c_int(dtype_code(gain.dtype) if gain is not None else F32), _ptr(ss_out),
+    _check(_lib().hymt2_gemm_tc_norm(out.data_ptr(), dtype_code(out.dtype), a.data_ptr(), w.data_ptr(), T, N, K, a.stride(0), w.stride(0),
+                                     out.stride(0), epilogue, _address(ws), ws.numel() if ws is not None else 0, _address(cnt),
+                                     cnt.numel() if cnt is not None else 0, status.data_ptr(), _raw_stream(), _address(ss_in), tiles_in, width, eps,
+                                     _address(normed), _address(gain), dtype_code(gain.dtype) if gain is not None else F32, _address(ss_out),
                                      *_glu_arguments(glu, glu_bias, N, epilogue)), "gemm_tc")
 
 
@@ -551,14 +573,12 @@ def gemm_tc_rope_kv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pla
         if q_gain.shape[0] != d or k_gain.shape[0] != d:
             raise KernelError("gemm_tc_rope_kv: the gains must hold head_dim values")
         gain_dtype = dtype_code(q_gain.dtype)
-    _check(_lib().hymt2_gemm_tc_rope_kv(_ptr(x), _ptr(w), c_int(T), c_int(x.shape[1]), c_long(x.stride(0)), c_long(w.stride(0)),
-                                        _ptr(q_out), _ptr(k_plane), _ptr(v_plane), _ptr(block_table),
-                                        c_int(block_table.stride(0)), c_int(block_tokens), _ptr(token_seq), _ptr(token_pos),
-                                        _ptr(slot_ids), _ptr(inv_freq), _ptr(angles), c_int(rope_dim), _ptr(q_gain), _ptr(k_gain),
-                                        c_int(gain_dtype), c_float(eps), c_int(nh), c_int(nkv), c_int(1 if write else 0),
-                                        _ptr(status), _stream(), _ptr(row_scale[0] if row_scale else None),
-                                        c_int(row_scale[0].shape[1] if row_scale else 0), c_int(row_scale[1] if row_scale else 0),
-                                        c_float(row_scale[2] if row_scale else 0.0)), "gemm_tc_rope_kv")
+    ss_in, width, ss_eps = row_scale if row_scale else (None, 0, 0.0)
+    _check(_lib().hymt2_gemm_tc_rope_kv(x.data_ptr(), w.data_ptr(), T, x.shape[1], x.stride(0), w.stride(0), q_out.data_ptr(), _address(k_plane),
+                                        _address(v_plane), block_table.data_ptr(), block_table.stride(0), block_tokens, token_seq.data_ptr(),
+                                        token_pos.data_ptr(), slot_ids.data_ptr(), _address(inv_freq), _address(angles), rope_dim,
+                                        _address(q_gain), _address(k_gain), gain_dtype, eps, nh, nkv, 1 if write else 0, status.data_ptr(),
+                                        _raw_stream(), _address(ss_in), ss_in.shape[1] if row_scale else 0, width, ss_eps), "gemm_tc_rope_kv")
 
 
 def gemm_tc_describe(tokens: int, out_features: int, inner: int, epilogue: int, sm_count: int = 0) -> dict:
@@ -729,11 +749,10 @@ def attention_prefill_tc(out: torch.Tensor, q: torch.Tensor, k_plane: torch.Tens
     _need(block_table, "block_table", torch.int32, 2)
     for t, n in ((cu_seqlens, "cu_seqlens"), (slot_ids, "slot_ids"), (kv_lens, "kv_lens")):
         _need(t, n, torch.int32, 1)
-    _check(_lib().hymt2_attention_prefill_tc(_ptr(out), _ptr(q), _ptr(k_plane), _ptr(v_plane), c_long(k_plane.shape[0]),
-                                             _ptr(block_table), c_int(block_table.stride(0)), c_int(k_plane.shape[2]),
-                                             _ptr(cu_seqlens), _ptr(slot_ids), _ptr(kv_lens), c_int(batch), c_int(T),
-                                             c_int(max_new_tokens), c_int(nh), c_int(nkv), c_int(d), c_float(scale),
-                                             c_int(window), _ptr(status), _stream()), "attention_prefill_tc")
+    _check(_lib().hymt2_attention_prefill_tc(out.data_ptr(), q.data_ptr(), k_plane.data_ptr(), v_plane.data_ptr(), k_plane.shape[0],
+                                             block_table.data_ptr(), block_table.stride(0), k_plane.shape[2], cu_seqlens.data_ptr(),
+                                             slot_ids.data_ptr(), kv_lens.data_ptr(), batch, T, max_new_tokens, nh, nkv, d, scale, window,
+                                             status.data_ptr(), _raw_stream()), "attention_prefill_tc")
 
 
 _counters: dict = {}
