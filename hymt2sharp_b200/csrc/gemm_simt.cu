@@ -319,7 +319,7 @@ int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda,
            cudaStream_t stream, int batch = 1, long a_bs = 0, long w_bs = 0, long c_bs = 0, GluRule glu = GluRule{}) {
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TC) == 4) {
         // few rows whose pieces of 16 bytes lie on their boundaries (33 to 64 of them only while the weight rows' blocks are all resident
-        // at twice an SM: 64 rows against 2,048 x 2,048 take 37 us there and 92 in tiles, against 12,288 x 2,048 195 and 126)
+        // at twice an SM: 64 rows against 2,048 x 2,048 take 43 us there and 92 in tiles, against 12,288 x 2,048 195 and 125)
         if ((M <= 32 || (M <= ROWS_MAX_M && N <= 296 * ROWS_N)) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
             (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
             float* c = (float*)C;
