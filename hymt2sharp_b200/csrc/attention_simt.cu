@@ -541,7 +541,8 @@ attention_plain_prompt_kernel(AttnParams p) {
 
 template <typename K>
 int plain_launch(K kernel, dim3 grid, size_t smem, cudaStream_t stream, const AttnParams& p) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit is the kernel's, not the call's: the same for every head size, so that threads do not lower it for one another)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) { hymt2_set_error("attention: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
     launch_pdl(kernel, grid, dim3(PLAIN_THREADS), smem, stream, p);
     return hymt2_check_launch("attention_plain");

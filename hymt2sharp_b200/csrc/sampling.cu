@@ -695,8 +695,10 @@ HYMT2_API int hymt2_sample(int* out, const float* logits, long row_stride, int r
     if (rows == 0) return HYMT2_OK;
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "sample: bad sizes rows=%d vocab=%d", rows, vocab);
     const size_t smem = sizeof(float) * CLUSTER_PIECES * (size_t)(((vocab + THREADS - 1) / THREADS) | 1);
-    if (smem <= 200 * 1024 && rows <= (1 << 27)) {
-        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr int most = 200 * 1024;
+    if (smem <= most && rows <= (1 << 27)) {
+        // (the limit is the kernel's, not the call's: the same for every vocabulary, so that threads do not lower it for one another)
+        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) { hymt2_set_error("sample: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
         launch_clusters(sample_cluster_kernel, rows, smem, stream, out, logits, row_stride, vocab, inv_temperature, rng_states, row_map);
         return hymt2_check_launch("sample");
