@@ -24,6 +24,8 @@
 // `diff_combine_kernel`: o = a1 - lambda * a2, then o / sqrt(mean(o^2) + eps) * factor over the head's dv entries.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int ROWS = 16, LANES_PER_ROW = 8, KEY_TILE = 32, MAX_D = 256, MAX_D_WIDE = 640, MAX_DV_WIDE = 512;
@@ -502,28 +504,41 @@ attention_plain_prompt_kernel(AttnParams p) {
             for (int j = 0; j < DI; j++) { acc[i][j].x *= corr; acc[i][j].y *= corr; acc[i][j].z *= corr; acc[i][j].w *= corr; }
         }
         __syncwarp();                                         // (a row's eight lanes are in one warp)
+        // Values of a tile that a row does not see are not even multiplied by its weights of zero: they may be infinite, and the row
+        // must not know of them.
+        bool sees[RT], all = true;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            sees[i] = row_pos[i] < 0 || (k0 <= row_pos[i] && k0 + KEY_TILE > row_lo[i]);
+            all = all && sees[i];
+        }
+        auto add_values = [&](auto edge) {
 #pragma unroll 2
-        for (int j4 = 0; j4 < KEY_TILE; j4 += 4) {
-            float4 p4[RT];
+            for (int j4 = 0; j4 < KEY_TILE; j4 += 4) {
+                float4 p4[RT];
 #pragma unroll
-            for (int i = 0; i < RT; i++) p4[i] = *reinterpret_cast<const float4*>(Ps + (rg + 16 * i) * PLAIN_P_LD + j4);
+                for (int i = 0; i < RT; i++) p4[i] = *reinterpret_cast<const float4*>(Ps + (rg + 16 * i) * PLAIN_P_LD + j4);
 #pragma unroll
-            for (int jj = 0; jj < 4; jj++) {
+                for (int jj = 0; jj < 4; jj++) {
 #pragma unroll
-                for (int i = 0; i < DI; i++) {
-                    const int x = 4 * c + 32 * i;
-                    if (x < d) {
-                        const float4 v = *reinterpret_cast<const float4*>(vs + (j4 + jj) * ld + x);
+                    for (int i = 0; i < DI; i++) {
+                        const int x = 4 * c + 32 * i;
+                        if (x < d) {
+                            const float4 v = *reinterpret_cast<const float4*>(vs + (j4 + jj) * ld + x);
 #pragma unroll
-                        for (int r = 0; r < RT; r++) {
-                            const float pj = jj == 0 ? p4[r].x : jj == 1 ? p4[r].y : jj == 2 ? p4[r].z : p4[r].w;
-                            acc[r][i].x = fmaf(pj, v.x, acc[r][i].x); acc[r][i].y = fmaf(pj, v.y, acc[r][i].y);
-                            acc[r][i].z = fmaf(pj, v.z, acc[r][i].z); acc[r][i].w = fmaf(pj, v.w, acc[r][i].w);
+                            for (int r = 0; r < RT; r++) {
+                                if (decltype(edge)::value && !sees[r]) continue;
+                                const float pj = jj == 0 ? p4[r].x : jj == 1 ? p4[r].y : jj == 2 ? p4[r].z : p4[r].w;
+                                acc[r][i].x = fmaf(pj, v.x, acc[r][i].x); acc[r][i].y = fmaf(pj, v.y, acc[r][i].y);
+                                acc[r][i].z = fmaf(pj, v.z, acc[r][i].z); acc[r][i].w = fmaf(pj, v.w, acc[r][i].w);
+                            }
                         }
                     }
                 }
             }
-        }
+        };
+        if (__all_sync(0xffffffffu, all)) add_values(std::false_type{});
+        else add_values(std::true_type{});
         __syncwarp();
     }
 #pragma unroll

@@ -69,3 +69,30 @@ def test_attention_of_the_plain_form_is_the_general_kernels_bit_for_bit(nh, nkv,
             outs.append(out)
         assert torch.equal(outs[0], outs[1])
         assert (outs[0][sum(news[:2]):sum(news[:3])] == 5.0).all()      # a padding row is left alone
+
+
+@pytest.mark.parametrize("nh, nkv, d", [(4, 4, 128), (6, 2, 40), (16, 2, 64), (3, 1, 256)])
+@pytest.mark.parametrize("window", [0, 20])
+def test_a_row_does_not_know_values_of_tiles_it_cannot_see(nh, nkv, d, window):
+    """Keys and values that are not finite reach no row but those that see their tile of 32 keys."""
+    ops = _ops()
+    torch.manual_seed(nh + d)
+    T = 200
+    keys, vals, q = torch.randn(T, nkv, d, device=DEV), torch.randn(T, nkv, d, device=DEV), torch.randn(T, nh * d, device=DEV)
+    bad_k, bad_v = keys.clone(), vals.clone()
+    for at, value in ((40, math.nan), (150, math.inf), (199, -math.inf)):
+        bad_v[at], bad_k[at] = value, value
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    outs = []
+    for k, v in ((keys, vals), (bad_k, bad_v)):
+        kp, vp, table = _paged([k], [v], 64, torch.float32)
+        out = torch.empty(T, nh * d, device=DEV)
+        ops.attention_simt(out, q, kp, vp, table, i32(0, T), i32(0), i32(T), 1, T, nh, nkv, d, 1 / math.sqrt(d), window)
+        outs.append(out)
+    tile = lambda p: p // 32
+    for p in range(T):
+        low = max(0, p - window + 1) if window else 0
+        if not any(tile(low) <= tile(at) <= tile(p) for at in (40, 150, 199)):
+            assert torch.equal(outs[0][p], outs[1][p]), p
+        if any(low <= at <= p for at in (40, 150, 199)):
+            assert not outs[1][p].isfinite().any(), p
