@@ -1,4 +1,4 @@
-// Token sampling on the GPU, a cluster of blocks per row of logits (one block where a vocabulary is too wide for that).
+// Token sampling on the GPU, one block or a cluster of eight blocks per row of logits.
 //
 //  * argmax: the first index that holds the maximum (src/HyMT2Sharp/Sampling.cs:298-334).
 //  * filters: repetition penalty over a window of recent tokens
@@ -195,12 +195,12 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_
     const int begin = min(vocab, (int)threadIdx.x * piece), end = min(vocab, begin + piece);
 
     float mx = -INFINITY;
-    for (int i = begin; i < end; i++) mx = fmaxf(mx, x[i] * inv_t);
+    for (int i = begin; i < end; i++) mx = fmaxf(mx, __fmul_rn(x[i], inv_t));
     mx = block_max(mx, scratch);
 
     float part = 0.f;
     for (int i = begin; i < end; i++) {
-        const float v = x[i] * inv_t;
+        const float v = __fmul_rn(x[i], inv_t);
         part += v == -INFINITY ? 0.f : expf(v - mx);
     }
     const float before = block_exclusive_scan<float>(part, warp_totals, &total_s);
@@ -224,7 +224,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_
         float acc = before;
         int pick = -1, last = -1;
         for (int i = begin; i < end; i++) {
-            const float v = x[i] * inv_t;
+            const float v = __fmul_rn(x[i], inv_t);
             const float pr = v == -INFINITY ? 0.f : expf(v - mx);
             if (pr <= 0.f) continue;
             last = i;
@@ -238,7 +238,7 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_
         // r lies past the last survivor through rounding: take the last entry with p > 0
         int last = -1;
         for (int i = begin; i < end; i++) {
-            const float v = x[i] * inv_t;
+            const float v = __fmul_rn(x[i], inv_t);
             if (v != -INFINITY && expf(v - mx) > 0.f) last = i;
         }
         if (last >= 0) atomicMax(&pick_s, last);
@@ -247,11 +247,12 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_
     if (threadIdx.x == 0) out[row] = pick_s >= 0 ? pick_s : 0;
 }
 
-// The same row by a cluster: block r of CLUSTER has the contiguous pieces of threads 128 r to 128 r + 127 of the kernel above, reads
+// The same row by a cluster of blocks.  Block r of CLUSTER has the contiguous pieces of threads 128 r to 128 r + 127 of the kernel above, reads
 // them once, side by side, into shared memory, and makes the exponentials there in parallel; a piece's sum, the scan over the
-// pieces and the walk inside the chosen piece add in the order of the kernel above, so the token is the same bit for bit.  The row's
-// blocks swap their maxima and their pieces' sums through distributed shared memory.  120,818 logits, 8 rows:
-// filters, argmax and draw together 59 us, against 552; the draw alone was 54, one block a row that read the logits three times, neighbouring threads 118 logits apart.
+// pieces and the walk inside the chosen piece add in the order of the kernel above, and both round a logit times 1 / temperature by
+// itself, so the token is the same bit for bit.  The row's blocks swap their maxima and their pieces' sums through distributed
+// shared memory.  120,818 logits, 8 rows: 17 us, against 61 for one block a row, which reads the logits three times, neighbouring
+// threads 118 logits apart.
 constexpr int CLUSTER = 8, CLUSTER_PIECES = THREADS / CLUSTER;
 
 __global__ void __launch_bounds__(THREADS)
@@ -361,12 +362,12 @@ struct FilterParams {
     const int* row_map;            // logits row -> sequence row, < 0 = skip
 };
 
-// A row is filtered by a cluster of blocks, each with a contiguous slice of the vocabulary, which it reads again in every pass (from
-// its own cache).  Thresholds are found by three radix passes over the keys (11, 11 and 10 bits): every block counts its slice's keys
-// per bin, a block adds up an eighth of the bins for all, and all walk the totals from the top.  After a top-k of up to FEW
-// entries the survivors go to the first block, which ranks them and settles min-p and top-p there.  120,818 logits, 8 rows, top-k 20,
-// top-p, penalty: with argmax and draw 59 us, against 552, of which the filters were 477: one block a row counted with 32 lanes on a few of 256 bins, four passes for top-k and four for
-// top-p, and read neighbouring logits from neighbouring threads in only half of its passes.
+// A row is filtered by one block or a cluster of them, each with a contiguous slice of the vocabulary, which it reads again in every
+// pass (from its own cache).  Thresholds are found by three radix passes over the keys (11, 11 and 10 bits): every block counts its
+// slice's keys per bin, a block adds up its share of the bins for all, and all walk the totals from the top.  After a top-k of up to
+// FEW entries the survivors go to the first block, which ranks them and settles min-p and top-p there.  What bounds it: the chain of
+// passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows, with top-k 20, top-p and penalty 31 us (one block a
+// row: 75), with top-p alone 58 (317), with min-p alone 13 (32).
 constexpr int FEW = 1024, BINS = 2048;
 
 struct FilterShared {
@@ -386,39 +387,50 @@ struct FilterShared {
 template <typename V> __device__ __forceinline__ V* bins_of(FilterShared& s) { return reinterpret_cast<V*>(s.hist); }
 template <typename V> __device__ __forceinline__ V* totals_of(FilterShared& s) { return reinterpret_cast<V*>(s.total); }
 
+// The blocks that share a row: a cluster of BLOCKS, or one block, which needs no cluster for it.
+template <int BLOCKS>
+struct RowBlocks {
+    __device__ void sync() const {
+        if constexpr (BLOCKS > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    }
+    template <typename V> __device__ V* of(V* mine, int rank) const {       // block `rank`'s copy of a shared variable
+        if constexpr (BLOCKS > 1) return cg::this_cluster().map_shared_rank(mine, rank);
+        else return mine;
+    }
+};
+
 // Adds up the blocks' bins: afterwards every block has the row's in `total`.  (In the order of the blocks: the same sum everywhere.)
-template <typename V>
-__device__ void gather_bins(cg::cluster_group& cluster, FilterShared& s, int bins) {
-    const int share = bins / CLUSTER, rank = cluster.block_rank();
-    cluster.sync();
+template <typename V, int BLOCKS>
+__device__ void gather_bins(RowBlocks<BLOCKS> blocks, FilterShared& s, int bins, int rank) {
+    const int share = bins / BLOCKS;
+    blocks.sync();
     for (int i = threadIdx.x; i < share; i += THREADS) {
         V sum = 0;
-        for (int r = 0; r < CLUSTER; r++) sum += *cluster.map_shared_rank(&bins_of<V>(s)[rank * share + i], r);
-        for (int r = 0; r < CLUSTER; r++) *cluster.map_shared_rank(&totals_of<V>(s)[rank * share + i], r) = sum;
+        for (int r = 0; r < BLOCKS; r++) sum += *blocks.of(&bins_of<V>(s)[rank * share + i], r);
+        for (int r = 0; r < BLOCKS; r++) *blocks.of(&totals_of<V>(s)[rank * share + i], r) = sum;
     }
-    cluster.sync();
+    blocks.sync();
 }
 
-// Every block's `value` into counts[] / floats[] of every block.
-__device__ __forceinline__ void swap_values(cg::cluster_group& cluster, int* mine, int value) {
-    if (threadIdx.x < CLUSTER) *cluster.map_shared_rank(&mine[cluster.block_rank()], threadIdx.x) = value;
-    cluster.sync();
-}
-__device__ __forceinline__ void swap_values(cg::cluster_group& cluster, float* mine, float value) {
-    if (threadIdx.x < CLUSTER) *cluster.map_shared_rank(&mine[cluster.block_rank()], threadIdx.x) = value;
-    cluster.sync();
+// Every block's `value` into mine[] of every block, at [place].
+template <typename V, int BLOCKS>
+__device__ __forceinline__ void swap_values(RowBlocks<BLOCKS> blocks, V* mine, int place, V value) {
+    if (threadIdx.x < BLOCKS) *blocks.of(&mine[place], threadIdx.x) = value;
+    blocks.sync();
 }
 
+template <int BLOCKS>
 __global__ void __launch_bounds__(THREADS)
 filter_kernel(FilterParams p) {
     __shared__ FilterShared s;
-    cg::cluster_group cluster = cg::this_cluster();
+    const RowBlocks<BLOCKS> blocks;
     pdl_wait();
-    const int row = blockIdx.x / CLUSTER, rank = blockIdx.x % CLUSTER, tid = threadIdx.x;
+    const int row = blockIdx.x / BLOCKS, rank = blockIdx.x % BLOCKS, tid = threadIdx.x;
     const int srow = p.row_map ? p.row_map[row] : row;
     if (srow < 0) return;
     float* x = p.logits + (size_t)row * p.row_stride;
-    const int vocab = p.vocab, slice = (vocab + CLUSTER - 1) / CLUSTER;
+    const int vocab = p.vocab, slice = (vocab + BLOCKS - 1) / BLOCKS;
     const int begin = min(vocab, rank * slice), end = min(vocab, begin + slice);
     const int piece = (slice + THREADS - 1) / THREADS;                          // a thread's contiguous piece of the slice
     const int pb = min(end, begin + tid * piece), pe = min(end, pb + piece);
@@ -449,7 +461,7 @@ filter_kernel(FilterParams p) {
     const int k = p.top_k ? p.top_k[srow] : 0;
     const float top_p = p.top_p ? p.top_p[srow] : 1.f, min_p = p.min_p ? p.min_p[srow] : 0.f;
     if (tid == 0) s.n_few = 0;
-    cluster.sync();     // every block of the row runs: its shared memory may be written to (the returns above are the whole row's)
+    blocks.sync();     // every block of the row runs: its shared memory may be written to (the returns above are the whole row's)
     const bool by_mass = top_p < 1.f || min_p > 0.f;
     const bool by_rank = k > 0 && k < vocab, few = by_rank && k <= FEW && by_mass;
 
@@ -465,7 +477,7 @@ filter_kernel(FilterParams p) {
                 const uint32_t key = float_key(x[i] * inv_t);
                 if ((key & mask) == prefix) atomicAdd(&s.hist[(key >> shift) & (bins - 1)], 1);
             }
-            gather_bins<int>(cluster, s, bins);
+            gather_bins<int>(blocks, s, bins, rank);
             // from the top: the bin in which the remaining-th key lies
             const int per = bins / THREADS, top = bins - 1 - tid * per;
             int mine = 0;
@@ -486,7 +498,7 @@ filter_kernel(FilterParams p) {
         const uint32_t kth = prefix;
         const int here = s.hist[s.bin];
         const bool all_ties = s.total[s.bin] == remaining;
-        swap_values(cluster, s.counts, here);
+        swap_values(blocks, s.counts, rank, here);
         if (!all_ties) {
             int ties = 0;
             for (int i = pb; i < pe; i++) ties += float_key(x[i] * inv_t) == kth;
@@ -497,8 +509,8 @@ filter_kernel(FilterParams p) {
             }
             __syncthreads();
         }
-        int* n_few = cluster.map_shared_rank(&s.n_few, 0);
-        unsigned long long* list = cluster.map_shared_rank(s.few, 0);
+        int* n_few = blocks.of(&s.n_few, 0);
+        unsigned long long* list = blocks.of(s.few, 0);
         const uint32_t lowest = float_key(-INFINITY);
         for (int i = begin + tid; i < end; i += THREADS) {
             const uint32_t key = float_key(x[i] * inv_t);
@@ -508,7 +520,7 @@ filter_kernel(FilterParams p) {
     }
 
     if (few) {
-        cluster.sync();
+        blocks.sync();
         if (rank != 0) return;
         // ranks by key, ties by index; the mass before an entry is then a scan
         const int n = s.n_few;
@@ -536,20 +548,27 @@ filter_kernel(FilterParams p) {
         float mx = -INFINITY;
         for (int i = begin + tid; i < end; i += THREADS) mx = fmaxf(mx, x[i] * inv_t);
         mx = block_max(mx, s.scratch);
-        swap_values(cluster, s.floats, mx);
-        for (int r = 0; r < CLUSTER; r++) mx = fmaxf(mx, s.floats[r]);
+        swap_values(blocks, s.floats, rank, mx);
+        for (int r = 0; r < BLOCKS; r++) mx = fmaxf(mx, s.floats[r]);
         // the mass of everything that is left after top-k: top-p's limit is a share of it,
         // also when min-p drops entries first (Sampling.cs:272-274 uses the sum from before)
         float sum = 0.f;
-        for (int i = begin + tid; i < end; i += THREADS) {
-            const float v = x[i] * inv_t;
-            sum += v == -INFINITY ? 0.f : expf(v - mx);
+        if (top_p < 1.f) {
+            // (of a whole row's eighths one after the other, however many blocks share them: the same limit)
+            const int eighth = (vocab + CLUSTER - 1) / CLUSTER;
+            for (int e = rank * (CLUSTER / BLOCKS); e < (rank + 1) * (CLUSTER / BLOCKS); e++) {
+                const int last = min(vocab, (e + 1) * eighth);
+                float part = 0.f;
+                for (int i = min(vocab, e * eighth) + tid; i < last; i += THREADS) {
+                    const float v = x[i] * inv_t;
+                    part += v == -INFINITY ? 0.f : expf(v - mx);
+                }
+                part = block_sum(part, s.scratch);
+                if (e == rank * (CLUSTER / BLOCKS)) blocks.sync();      // (the maxima have been read)
+                swap_values(blocks, s.floats, e, part);
+            }
+            for (int e = 0; e < CLUSTER; e++) sum += s.floats[e];
         }
-        sum = block_sum(sum, s.scratch);
-        cluster.sync();
-        swap_values(cluster, s.floats, sum);
-        sum = 0.f;
-        for (int r = 0; r < CLUSTER; r++) sum += s.floats[r];
         if (min_p > 0.f) {
             // p >= min_p * p_max with p_max = exp(0) = 1
             for (int i = begin + tid; i < end; i += THREADS) {
@@ -576,7 +595,7 @@ filter_kernel(FilterParams p) {
                     const uint32_t key = float_key(v);
                     if ((key & mask) == prefix) atomicAdd(&bins_of<float>(s)[(key >> shift) & (bins - 1)], expf(v - mx));
                 }
-                gather_bins<float>(cluster, s, bins);
+                gather_bins<float>(blocks, s, bins, rank);
                 const float* mass = totals_of<float>(s);
                 const int per = bins / THREADS, top = bins - 1 - tid * per;
                 float mine = 0.f;
@@ -606,8 +625,8 @@ filter_kernel(FilterParams p) {
                 ties += v != -INFINITY && float_key(v) == prefix;
             }
             int at = block_exclusive_scan<int>(ties, s.warp_i, &s.total_i);
-            cluster.sync();
-            swap_values(cluster, s.counts, s.total_i);
+            blocks.sync();
+            swap_values(blocks, s.counts, rank, s.total_i);
             for (int r = 0; r < rank; r++) at += s.counts[r];
             for (int i = pb; i < pe; i++) {
                 const float v = x[i] * inv_t;
@@ -622,7 +641,7 @@ filter_kernel(FilterParams p) {
             }
         }
     }
-    cluster.sync();     // (nobody leaves while another block may still write to its shared memory)
+    blocks.sync();     // (nobody leaves while another block may still write to its shared memory)
 }
 
 // history[sequence, count % stride] = token; count += 1 (the ring of Sampling.cs:158-169)
@@ -636,6 +655,9 @@ __global__ void record_history_kernel(int* history, int* counts, int stride, con
     history[(size_t)srow * stride + c % stride] = tokens[row];
     counts[srow] = c + 1;
 }
+
+constexpr size_t SAMPLE_SHARED = 200 * 1024;
+inline size_t sample_shared(int vocab) { return sizeof(float) * CLUSTER_PIECES * (size_t)(((vocab + THREADS - 1) / THREADS) | 1); }
 
 // CLUSTER blocks a row, behind the kernel in front (programmatic dependent launch).
 template <typename... KArgs, typename... Args>
@@ -689,21 +711,41 @@ HYMT2_API int hymt2_seed_rng(uint64_t* states, const int* rows, const uint64_t* 
     return hymt2_check_launch("seed_rng");
 }
 
+// How many blocks draw a row's token, one or CLUSTER; the token does not hang on it.  A cluster pays where the row is wide and the
+// clusters of a step run side by side: 12,000 logits 8 us with one block and 7 with eight for 8 rows, 8 and 14 for 64; 24,000 logits
+// 13 and 10 for 24 rows, 13 and 14 for 37; 120,818 logits 61 and 17 for 8 rows, 62 and 58 for 100, 62 and 81 for 148.  One block's
+// reads lie a piece apart: pieces of a multiple of 32 logits (128 bytes) crowd its cache, and a cluster is the faster one for any
+// number of rows (65,536 logits, 256 rows: 145 and 85).  More than 408,576 logits do not fit the cluster's shared memory.
+HYMT2_API int hymt2_sample_blocks(int rows, int vocab) {
+    const int piece = (vocab + THREADS - 1) / THREADS;
+    if (vocab < 16384 || sample_shared(vocab) > SAMPLE_SHARED || rows > (1 << 27)) return 1;
+    return rows <= (vocab < 32768 ? 32 : 100) || piece % 32 == 0 ? CLUSTER : 1;
+}
+
+// The same for the filters.  What is counted and ranked does not hang on it; the mass per bin of a top-p without a top-k before it
+// is added up in the order of the atomics either way.  A cluster has seven blocks more a row to launch and to wait for, so it needs
+// logits to read and few enough rows to run side by side.  us with one block and with eight, for top-k 20 + top-p + penalty / top-p
+// alone / min-p alone: 3,000 logits, 8 rows 13 19 / 21 20 / 6 7; 12,000 logits, 8 rows 15 20 / 40 24 / 7 8, 64 rows 16 45 / 41 57 /
+// 8 15; 32,768 logits, 64 rows 22 48 / 110 77 / 11 15, 100 rows 24 75 / 111 130 / 12 25; 120,818 logits, 64 rows 89 86 / 331 187 /
+// 46 40, 100 rows 106 144 / 349 314 / 63 69; 300,000 logits, 100 rows 325 292 / 1036 715 / 185 162, 148 rows 379 405 / 1103 1020 /
+// 237 230.
+HYMT2_API int hymt2_filter_blocks(int rows, int vocab) {
+    return vocab >= 8192 && rows <= vocab / 400 && (rows <= 64 || rows <= vocab / 2000) ? CLUSTER : 1;
+}
+
 HYMT2_API int hymt2_sample(int* out, const float* logits, long row_stride, int rows, int vocab,
                            const float* inv_temperature, uint64_t* rng_states, const int* row_map,
                            cudaStream_t stream) {
     if (rows == 0) return HYMT2_OK;
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "sample: bad sizes rows=%d vocab=%d", rows, vocab);
-    const size_t smem = sizeof(float) * CLUSTER_PIECES * (size_t)(((vocab + THREADS - 1) / THREADS) | 1);
-    constexpr int most = 200 * 1024;
-    if (smem <= most && rows <= (1 << 27)) {
+    if (hymt2_sample_blocks(rows, vocab) == CLUSTER) {
         // (the limit is the kernel's, not the call's: the same for every vocabulary, so that threads do not lower it for one another)
-        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SHARED);
         if (e != cudaSuccess) { hymt2_set_error("sample: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
-        launch_clusters(sample_cluster_kernel, rows, smem, stream, out, logits, row_stride, vocab, inv_temperature, rng_states, row_map);
+        launch_clusters(sample_cluster_kernel, rows, sample_shared(vocab), stream, out, logits, row_stride, vocab, inv_temperature, rng_states,
+                        row_map);
         return hymt2_check_launch("sample");
     }
-    // a vocabulary of more than 400,000: its pieces do not fit the cluster's shared memory
     sample_kernel<<<rows, THREADS, 0, stream>>>(out, logits, row_stride, vocab, inv_temperature, rng_states,
                                                 row_map);
     return hymt2_check_launch("sample");
@@ -717,7 +759,7 @@ HYMT2_API int hymt2_filter_logits(float* logits, long row_stride, int rows, int 
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "filter: bad sizes rows=%d vocab=%d", rows, vocab);
     FilterParams p{logits, row_stride, vocab, inv_temperature, top_k, top_p, min_p, penalty, history,
                    history_stride, row_map};
-    HYMT2_REQUIRE(rows <= (1 << 27), "filter: %d rows", rows);
-    launch_clusters(filter_kernel, rows, 0, stream, p);
+    if (hymt2_filter_blocks(rows, vocab) == CLUSTER) launch_clusters(filter_kernel<CLUSTER>, rows, 0, stream, p);
+    else launch_pdl(filter_kernel<1>, dim3(rows), dim3(THREADS), 0, stream, p);
     return hymt2_check_launch("filter_logits");
 }

@@ -858,6 +858,16 @@ def sample(out: torch.Tensor, logits: torch.Tensor, inv_temperature: torch.Tenso
                                _ptr(inv_temperature), _ptr(rng_states), _ptr(row_map), _stream()), "sample")
 
 
+def sample_blocks(rows: int, vocab: int) -> int:
+    """Blocks that draw one row's token in `sample` (1 or 8); the token is the same either way.  Works without a GPU."""
+    return int(_lib().hymt2_sample_blocks(c_int(rows), c_int(vocab)))
+
+
+def filter_blocks(rows: int, vocab: int) -> int:
+    """Blocks that share a row in `filter_logits` (1 or 8).  Works without a GPU."""
+    return int(_lib().hymt2_filter_blocks(c_int(rows), c_int(vocab)))
+
+
 def filter_logits(logits: torch.Tensor, inv_temperature: torch.Tensor, top_k: torch.Tensor | None,
                   top_p: torch.Tensor | None, min_p: torch.Tensor | None, penalty: torch.Tensor | None,
                   history: torch.Tensor | None, row_map: torch.Tensor | None = None) -> None:

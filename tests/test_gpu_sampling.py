@@ -95,3 +95,75 @@ def test_draws_from_wide_rows_fall_into_their_interval(vocab):
             u = float(refs[r].next_single())
             assert np.isfinite(logits[r, tok].item())
             assert (cdf[r][tok - 1] if tok else 0.0) - 1e-5 <= u <= cdf[r][tok] + 1e-5
+
+
+@pytest.mark.parametrize("vocab, many", [(20000, 40), (120818, 104), (16999, 300)])
+def test_draws_are_the_same_with_one_block_a_row_and_with_eight(vocab, many):
+    ops = _ops()
+    assert ops.sample_blocks(many, vocab) == 1 and ops.sample_blocks(8, vocab) == 8
+    torch.manual_seed(vocab)
+    logits = torch.randn(many, vocab, device=DEV) * 4
+    logits[1, torch.rand(vocab, device=DEV) < 0.9] = -math.inf
+    logits[2] = -math.inf
+    logits[3, 5:] = -math.inf
+    inv_t = torch.rand(many, device=DEV) + 0.5
+    inv_t[4] = 0.0                                      # a greedy row is left alone
+    rows = torch.arange(many, dtype=torch.int32, device=DEV)
+    states = torch.zeros(many, 4, dtype=torch.int64, device=DEV)
+    ops.seed_rng(states, rows, torch.arange(many, dtype=torch.int64, device=DEV) * 7 + 1)
+    other = states.clone()
+    for _ in range(40):
+        one, eight = torch.full((many,), -9, dtype=torch.int32, device=DEV), torch.full((many,), -9, dtype=torch.int32, device=DEV)
+        ops.sample(one, logits, inv_t, states)
+        for at in range(0, many, 8):
+            n = min(8, many - at)
+            ops.sample(eight[at:at + n], logits[at:at + n], inv_t, other, rows[at:at + n].contiguous())
+        assert torch.equal(one, eight) and torch.equal(states, other)
+        assert one[4] == -9 and one[2] == 0
+
+
+def test_draws_from_rows_too_wide_for_a_cluster_fall_into_their_interval():
+    from plain.hunyuan_plain import Xoshiro256StarStar
+    ops = _ops()
+    vocab = 410000
+    assert ops.sample_blocks(1, vocab) == 1
+    torch.manual_seed(1)
+    logits = torch.randn(1, vocab, device=DEV) * 3
+    cdf = torch.softmax(logits.double() / 0.7, dim=1).cumsum(1).cpu().numpy()[0]
+    states = torch.zeros(1, 4, dtype=torch.int64, device=DEV)
+    ops.seed_rng(states, torch.zeros(1, dtype=torch.int32, device=DEV), torch.tensor([5], dtype=torch.int64, device=DEV))
+    ref, out, inv_t = Xoshiro256StarStar(5), torch.empty(1, dtype=torch.int32, device=DEV), torch.full((1,), 1 / 0.7, device=DEV)
+    for _ in range(50):
+        ops.sample(out, logits, inv_t, states)
+        tok, u = int(out[0]), float(ref.next_single())
+        assert (cdf[tok - 1] if tok else 0.0) - 1e-5 <= u <= cdf[tok] + 1e-5
+
+
+@pytest.mark.parametrize("vocab, many", [(9001, 24), (20000, 72)])
+@pytest.mark.parametrize("k, top_p, min_p", [(1, 1.0, 0.0), (20, 0.6, 0.0), (50, 0.9, 0.05), (1500, 1.0, 0.02), (1500, 0.9, 0.0), (0, 0.8, 0.0), (0, 1.0, 0.02), (0, 1.0, 0.0)])
+def test_filters_are_the_same_with_one_block_a_row_and_with_eight(vocab, many, k, top_p, min_p):
+    ops = _ops()
+    assert ops.filter_blocks(many, vocab) == 1 and ops.filter_blocks(4, vocab) == 8
+    rng = np.random.default_rng(vocab + k)
+    x = (rng.standard_normal((many, vocab)) * 2.5).astype(np.float32)
+    x[1::4] = np.round(x[1::4] * 2) / 2                                  # ties, at the threshold too
+    x[2, rng.random(vocab) < 0.4] = -np.inf
+    history = rng.integers(0, vocab, (many, 16)).astype(np.int32)
+    history[:, 3:6] = history[:, :1]
+    f32 = lambda v: torch.full((many,), v, dtype=torch.float32, device=DEV)
+    arguments = (f32(1 / 0.7), torch.full((many,), k, dtype=torch.int32, device=DEV), f32(top_p), f32(min_p), f32(1.1), torch.from_numpy(history).to(DEV))
+    one, eight = torch.from_numpy(x).to(DEV), torch.from_numpy(x).to(DEV)
+    ops.filter_logits(one, *arguments)
+    rows = torch.arange(many, dtype=torch.int32, device=DEV)
+    for at in range(0, many, 4):
+        ops.filter_logits(eight[at:at + 4], *arguments, rows[at:at + 4].contiguous())
+    if top_p == 1.0 or 0 < k <= 1024:        # nothing but counts, ranks and sums in one order
+        assert torch.equal(one, eight)
+        return
+    one, eight = one.cpu().numpy(), eight.cpu().numpy()
+    for r in range(many):                    # the mass per bin is added up in the order of the atomics
+        want, keep, near = _filtered(x[r], float(np.float32(1 / 0.7)), k, top_p, min_p, float(np.float32(1.1)), history[r])
+        differ = np.isfinite(one[r]) != np.isfinite(eight[r])
+        assert (~differ | near).all()
+        both = ~differ & np.isfinite(one[r])
+        assert (one[r][both] == eight[r][both]).all()

@@ -1,0 +1,12 @@
+"""Which kernel a call takes, where a rule on its sizes decides (no GPU)."""
+import pytest
+
+from hymt2sharp_b200.kernels import ops
+
+
+@pytest.mark.parametrize("rows, vocab, filters, draw", [
+    (8, 120818, 8, 8), (64, 120818, 8, 8), (65, 120818, 1, 8), (100, 120818, 1, 8), (101, 120818, 1, 1), (148, 300000, 8, 1), (64, 32768, 8, 8),
+    (256, 32768, 1, 8), (256, 65536, 1, 8), (256, 300, 1, 1), (1, 300, 1, 1), (8, 5000, 1, 1), (8, 12000, 8, 1), (40, 16384, 8, 1), (41, 16384, 1, 1),
+    (33, 20000, 8, 1), (32, 20000, 8, 8), (1, 408576, 8, 8), (1, 408577, 8, 1), (2 ** 31 - 1, 120818, 1, 1)])
+def test_rows_are_filtered_and_drawn_by_one_block_where_a_cluster_would_be_slower(rows, vocab, filters, draw):
+    assert (ops.filter_blocks(rows, vocab), ops.sample_blocks(rows, vocab)) == (filters, draw)
