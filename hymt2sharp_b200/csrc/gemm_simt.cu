@@ -282,14 +282,20 @@ int launch_rows_for(float* C, const float* A, const float* W, int M, int N, int 
 }
 
 // Which tiles: the ones whose busiest SM has the least to do.  A wave of blocks costs an SM its tiles' entries; smaller tiles read
-// shared memory more often per FMA (531 rows: an entry of 64 x 64 costs 1.05 and of 32 x 64 1.35 of one of 64 x 128).
-inline int pick_tile(int M, int N, int NB, int batch) {
+// shared memory more often per FMA (531 rows: an entry of 64 x 64 costs 1.05 and of 32 x 64 1.35 of one of 64 x 128).  Operands of 16
+// bits are converted on their way into shared memory; while 64 x 64 tiles fill no more than an SM each, a product takes as long as one
+// of its tiles, and twice the threads with half the entries shorten that: 129 rows against 2,048 x 2,048 in bfloat16 take 120 us with
+// 4 x 4 entries a thread and 167 with 8 x 4.
+enum { TILES_64x128 = 0, TILES_64x64 = 1, TILES_32x64 = 2, TILES_64x64_SHORT = 3, ROWS_STREAMED = 4 };
+
+inline int pick_tile(int M, int N, int NB, int batch, bool narrow) {
     const int tm[3] = {64, 64, 32}, tn[3] = {128, 64, 64};
     const double cost[3] = {1.0, 1.05, 1.35};
     int best = 0;
     double least = 0.0;
     for (int i = 0; i < 3; i++) {
         const long blocks = (long)((M + tm[i] - 1) / tm[i]) * ((N + tn[i] / NB - 1) / (tn[i] / NB)) * batch;
+        if (i == TILES_64x64 && narrow && blocks <= 148) return TILES_64x64_SHORT;
         const double c = (double)((blocks + 147) / 148) * tm[i] * tn[i] * cost[i];
         if (i == 0 || c < least) { best = i; least = c; }
     }
@@ -306,22 +312,26 @@ int launch_tiles(TC* C, const TA* A, const TW* W, int M, int N, int K, long lda,
     gemm_simt_kernel<TA, TW, TC, EPI, BM_, BN_, PM_, PN_><<<dim3((N + BN_ / NB - 1) / (BN_ / NB), (M + BM_ - 1) / BM_, batch),         \
                                                             BM_ * BN_ / (PM_ * PN_), 0, stream>>>(                                     \
         C, A, W, M, N, K, lda, ldw, ldc, vec_a, vec_w, a_bs, w_bs, c_bs, glu)
-    const int tile = pick_tile(M, N, NB, batch);
-    if (tile == 0) HYMT2_GEMM_TILE(64, 128, 8, 4);
-    else if (tile == 1) HYMT2_GEMM_TILE(64, 64, 8, 4);
-    else HYMT2_GEMM_TILE(32, 64, 4, 4);
+    constexpr bool narrow = sizeof(TA) == 2 || sizeof(TW) == 2;
+    const int tile = pick_tile(M, N, NB, batch, narrow);
+    if (tile == TILES_64x128) HYMT2_GEMM_TILE(64, 128, 8, 4);
+    else if (tile == TILES_64x64) HYMT2_GEMM_TILE(64, 64, 8, 4);
+    else if (tile == TILES_32x64) HYMT2_GEMM_TILE(32, 64, 4, 4);
+    else if constexpr (narrow) HYMT2_GEMM_TILE(64, 64, 4, 4);
 #undef HYMT2_GEMM_TILE
     return hymt2_check_launch("gemm_simt");
 }
+
+// Few rows whose weights are streamed: 33 to 64 of them only while the weight rows' blocks are all resident
+// at twice an SM: 64 rows against 2,048 x 2,048 take 43 us there and 92 in tiles, against 12,288 x 2,048 195 and 125.
+inline bool rows_streamed(int M, int N) { return M <= 32 || (M <= ROWS_MAX_M && N <= 296 * ROWS_N); }
 
 template <typename TA, typename TW, typename TC>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda, long ldw, long ldc, int epi,
            cudaStream_t stream, int batch = 1, long a_bs = 0, long w_bs = 0, long c_bs = 0, GluRule glu = GluRule{}) {
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TC) == 4) {
-        // few rows whose pieces of 16 bytes lie on their boundaries (33 to 64 of them only while the weight rows' blocks are all resident
-        // at twice an SM: 64 rows against 2,048 x 2,048 take 43 us there and 92 in tiles, against 12,288 x 2,048 195 and 125)
-        if ((M <= 32 || (M <= ROWS_MAX_M && N <= 296 * ROWS_N)) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
-            (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
+        // (pieces of 16 bytes that lie on their boundaries)
+        if (rows_streamed(M, N) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
             float* c = (float*)C;
             const float *a = (const float*)A, *w = (const float*)W;
             if (epi == EPI_STORE) return launch_rows_for<EPI_STORE>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
@@ -576,6 +586,13 @@ gemm_skinny_grouped_kernel(TC* __restrict__ C, const T* __restrict__ A, const T*
 }  // namespace
 
 // C[M,N] (ldc) = epilogue(A[M,K] (lda) · W[N,K]^T (ldw)); for the swiglu epilogue W has 2N rows.
+// Which kernel a product takes: the number of its tiles above, or ROWS_STREAMED.  narrow: operands of 16 bits (one or both); aligned:
+// K and the rows' strides multiples of 4, both operands on 16 bytes.
+HYMT2_API int hymt2_gemm_simt_route(int M, int N, int epi, int batch, int narrow, int aligned) {
+    if (!narrow && aligned && batch == 1 && rows_streamed(M, N)) return ROWS_STREAMED;
+    return pick_tile(M, N, epi == EPI_SWIGLU ? 2 : 1, batch, narrow != 0);
+}
+
 HYMT2_API int hymt2_gemm_simt(void* C, int c_dtype, const void* A, int a_dtype, const void* W, int w_dtype,
                               int M, int N, int K, long lda, long ldw, long ldc, int epilogue,
                               int glu_kind, float glu_limit, float glu_alpha, const float* glu_bias, cudaStream_t stream) {

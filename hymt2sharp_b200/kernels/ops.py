@@ -368,6 +368,13 @@ def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int
                                   c_int(epilogue), *_glu_arguments(glu, glu_bias, N, epilogue), _stream()), "gemm_simt")
 
 
+def gemm_simt_route(rows: int, columns: int, epilogue: int = EPILOGUE_STORE, batch: int = 1, narrow: bool = False, aligned: bool = True) -> str:
+    """The kernel that gemm_simt runs: the tiles' rows of `a` x weight rows, or "rows" (few rows, the weights streamed).  `narrow`: an
+    operand of 16 bits; `aligned`: inner sizes and row strides multiples of 4, operands on 16 bytes.  Works without a GPU."""
+    which = _lib().hymt2_gemm_simt_route(c_int(rows), c_int(columns), c_int(epilogue), c_int(batch), c_int(narrow), c_int(aligned))
+    return ("64x128", "64x64", "32x64", "64x64 short", "rows")[which]
+
+
 _status: dict = {}
 _status_of: dict = {}   # the same by what callers pass (a torch.device with an index)
 

@@ -44,6 +44,51 @@ def test_products_of_few_rows_and_in_tiles_agree_bit_for_bit(M, N, K):
             assert ((outs[0].double() - base.double() - ref[:, :N]).abs() <= bound[:, :N] + 2.0 ** -23 * (base.double().abs() + ref[:, :N].abs())).all()
 
 
+# sizes whose last tile is ragged in both directions, with the tiles that the rule picks for them
+_TILES = [(100, 5003, 0, False, "64x128"), (65, 4099, 2, False, "64x128"), (65, 4099, 0, False, "64x64"), (130, 1001, 2, False, "64x64"),
+          (65, 131, 1, False, "32x64"), (67, 130, 2, False, "32x64"), (100, 5003, 1, True, "64x128"), (65, 4099, 2, True, "64x128"),
+          (130, 8001, 1, True, "64x64"), (100, 5003, 2, True, "64x64"), (65, 5003, 0, True, "32x64"), (65, 3001, 2, True, "32x64"),
+          (65, 131, 0, True, "64x64 short"), (129, 1001, 1, True, "64x64 short"), (129, 70, 2, True, "64x64 short")]
+
+
+@pytest.mark.parametrize("M, N, epilogue, narrow, tile", _TILES)
+@pytest.mark.parametrize("K", [131, 132, 16, 3])
+def test_products_in_every_tile(M, N, epilogue, narrow, tile, K):
+    ops = _ops()
+    assert ops.gemm_simt_route(M, N, epilogue, narrow=narrow, aligned=False) == tile
+    torch.manual_seed(M + N + K)
+    bf = torch.bfloat16
+    for ta, tw, to in ([(bf, bf, bf), (torch.float32, bf, torch.float32), (bf, torch.float32, torch.float32)] if narrow else [(torch.float32,) * 3]):
+        a = torch.randn(M, K, device=DEV).to(ta)
+        w = (torch.randn(2 * N if epilogue == ops.EPILOGUE_SWIGLU else N, K, device=DEV) / math.sqrt(K)).to(tw)
+        base = torch.randn(M, N, device=DEV).to(to)
+        outs = []
+        wide = torch.zeros(M, K + 4, device=DEV, dtype=ta)                       # rows a piece of 16 bytes further apart
+        wide[:, :K] = a
+        for x in (a, _shifted(a), wide[:, :K]):
+            out = base.clone()
+            ops.gemm_simt(out, x, w, epilogue)
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+        for m in (0, 63, M - 1):                                                 # one row alone
+            one = base[m:m + 1].clone()
+            ops.gemm_simt(one, a[m:m + 1].contiguous(), w, epilogue)
+            assert torch.equal(one, outs[0][m:m + 1])
+        ref, sums = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+        error = K * 2.0 ** -24 * sums                                            # a chain of K float32 FMAs
+        store = 2.0 ** -8 if to == bf else 2.0 ** -23                            # and the rounding of what is stored
+        if epilogue == ops.EPILOGUE_SWIGLU:
+            g, u = ref[:, :N], ref[:, N:]
+            silu = g / (1 + torch.exp(-g))
+            want = silu * u
+            # |silu'| <= 1.1; the exponential and the division are within a few units of 2^-24
+            bound = 1.1 * error[:, :N] * (u.abs() + error[:, N:]) + silu.abs() * error[:, N:] + (store + 2.0 ** -20) * want.abs() + 1e-12
+        else:
+            want = ref + base.double() if epilogue == ops.EPILOGUE_ACCUMULATE else ref
+            bound = error + store * (want.abs() + ref.abs()) + 1e-12
+        assert ((outs[0].double() - want).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("nh, nkv, d, window", [(4, 4, 128, 0), (16, 2, 128, 0), (6, 2, 40, 0), (20, 1, 64, 50), (5, 1, 256, 100), (8, 2, 8, 0), (64, 1, 128, 0)])
 @pytest.mark.parametrize("news", [[1, 1, 1, 1], [70, 1, 45, 300]])
 def test_attention_of_the_plain_form_is_the_general_kernels_bit_for_bit(nh, nkv, d, window, news):

@@ -10,3 +10,11 @@ from hymt2sharp_b200.kernels import ops
     (33, 20000, 8, 1), (32, 20000, 8, 8), (1, 408576, 8, 8), (1, 408577, 8, 1), (2 ** 31 - 1, 120818, 1, 1)])
 def test_rows_are_filtered_and_drawn_by_one_block_where_a_cluster_would_be_slower(rows, vocab, filters, draw):
     assert (ops.filter_blocks(rows, vocab), ops.sample_blocks(rows, vocab)) == (filters, draw)
+
+
+@pytest.mark.parametrize("rows, columns, epilogue, narrow, kernel", [
+    (129, 2048, 0, True, "64x64 short"), (300, 1000, 0, True, "64x64 short"), (600, 500, 0, True, "64x64 short"), (1, 8192, 0, True, "64x64 short"),
+    (129, 4096, 2, True, "64x64"), (64, 9472, 0, True, "64x64 short"), (64, 9473, 0, True, "64x128"), (531, 6144, 2, True, "64x128"),
+    (531, 3072, 0, False, "64x64"), (531, 6144, 2, False, "64x128"), (129, 2048, 0, False, "64x64"), (65, 130, 0, False, "32x64")])
+def test_tiles_of_products_on_cuda_cores(rows, columns, epilogue, narrow, kernel):
+    assert ops.gemm_simt_route(rows, columns, epilogue, narrow=narrow) == kernel
