@@ -48,7 +48,7 @@ __device__ __forceinline__ void finish(TC* c, float acc, float up, const GluRule
 // owns 4 * PM x 8 * PN entries, a thread PM x PN of them, two rows of A to an FMA instruction: its PM entries of A and PN of W a k
 // are shared-memory reads that most of the warp's lanes have in common.  The next step's 16 columns are on their way to registers
 // while this step's are worked on; shared memory has two buffers, so a step has one barrier.  What bounds it: the FMA pipe (74
-// TFLOP/s) and the issue of what feeds it.  531 rows against 12,288 x 2,048 (gate and up of the 1.8B sizes): 606 us; 4 x 4 entries a
+// TFLOP/s) and the issue of what feeds it.  531 rows against 12,288 x 2,048 (gate and up of the 1.8B sizes): 597 us; 4 x 4 entries a
 // thread, one buffer and single-word reads, which this replaced, took 769.  Also measured there: plain FMAs 684, 8 x 8 entries
 // with 128 threads 650 to 700, 8 x 16 668, W stored twice for the pairs 838.
 template <typename TA, typename TW, typename TC, int EPI, int TILE_M, int TILE_N, int PM, int PN>
@@ -167,7 +167,7 @@ constexpr int ROWS_N = 16, ROWS_THREADS = 128, ROWS_BK = 128, ROWS_LD = ROWS_BK 
 
 __host__ __device__ constexpr int rows_stage_floats(int mp, int nb) { return (nb * ROWS_N + mp) * ROWS_LD; }
 __host__ __device__ constexpr int rows_stages(int mp, int nb) {
-    const int fit = 75 * 1024 / (4 * rows_stage_floats(mp, nb));      // three blocks an SM
+    const int fit = 75 * 1024 / (4 * rows_stage_floats(mp, nb));      // three blocks an SM, where three stages leave room for them
     return fit < 3 ? 3 : (fit > 8 ? 8 : fit);
 }
 
@@ -322,16 +322,28 @@ int launch_tiles(TC* C, const TA* A, const TW* W, int M, int N, int K, long lda,
     return hymt2_check_launch("gemm_simt");
 }
 
-// Few rows whose weights are streamed: 33 to 64 of them only while the weight rows' blocks are all resident
-// at twice an SM: 64 rows against 2,048 x 2,048 take 43 us there and 92 in tiles, against 12,288 x 2,048 195 and 125.
-inline bool rows_streamed(int M, int N) { return M <= 32 || (M <= ROWS_MAX_M && N <= 296 * ROWS_N); }
+// Few rows whose weights are streamed.  The time grows with every wave of weight rows' blocks (three of them fit an SM with up to 16
+// rows, two or three with 32, one with 64), where the tiles hardly notice rows of A and their waves are four times as wide.  us
+// streamed and in tiles, K = 2,048 (1,024 and 4,096 cross at the same widths):
+//   16 rows: 20,480 wide 103 123, 32,768 wide 165 157, 120,818 wide 540 498; gated 65,536 wide 458 542
+//   32 rows: 8,192 wide 99 93, 9,472 wide 102 94, 12,288 wide 105 101, 16,384 wide 145 102, 120,818 wide 812 506; gated 9,472 wide 95 100, 12,288 wide
+//     138 123
+//   64 rows: 4,736 wide 78 92, 4,800 wide 115 96; gated 2,368 wide 76 88, 3,072 wide 106 94
+inline bool rows_streamed(int M, int N, int epi) {
+    const int blocks = (N + ROWS_N - 1) / ROWS_N;
+    const bool gated = epi == EPI_SWIGLU;
+    if (M <= 8) return true;
+    if (M <= 16) return gated || blocks <= 1280;
+    if (M <= 32) return blocks <= 592;
+    return M <= ROWS_MAX_M && blocks <= (gated ? 148 : 296);
+}
 
 template <typename TA, typename TW, typename TC>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, long lda, long ldw, long ldc, int epi,
            cudaStream_t stream, int batch = 1, long a_bs = 0, long w_bs = 0, long c_bs = 0, GluRule glu = GluRule{}) {
     if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TC) == 4) {
         // (pieces of 16 bytes that lie on their boundaries)
-        if (rows_streamed(M, N) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
+        if (rows_streamed(M, N, epi) && batch == 1 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0) {
             float* c = (float*)C;
             const float *a = (const float*)A, *w = (const float*)W;
             if (epi == EPI_STORE) return launch_rows_for<EPI_STORE>(c, a, w, M, N, K, lda, ldw, ldc, glu, stream);
@@ -589,7 +601,7 @@ gemm_skinny_grouped_kernel(TC* __restrict__ C, const T* __restrict__ A, const T*
 // Which kernel a product takes: the number of its tiles above, or ROWS_STREAMED.  narrow: operands of 16 bits (one or both); aligned:
 // K and the rows' strides multiples of 4, both operands on 16 bytes.
 HYMT2_API int hymt2_gemm_simt_route(int M, int N, int epi, int batch, int narrow, int aligned) {
-    if (!narrow && aligned && batch == 1 && rows_streamed(M, N)) return ROWS_STREAMED;
+    if (!narrow && aligned && batch == 1 && rows_streamed(M, N, epi)) return ROWS_STREAMED;
     return pick_tile(M, N, epi == EPI_SWIGLU ? 2 : 1, batch, narrow != 0);
 }
 

@@ -44,6 +44,21 @@ def test_products_of_few_rows_and_in_tiles_agree_bit_for_bit(M, N, K):
             assert ((outs[0].double() - base.double() - ref[:, :N]).abs() <= bound[:, :N] + 2.0 ** -23 * (base.double().abs() + ref[:, :N].abs())).all()
 
 
+@pytest.mark.parametrize("M, N, epilogue", [(16, 20480, 0), (16, 20481, 0), (17, 9472, 1), (32, 9473, 1), (32, 9473, 2), (64, 4736, 0), (64, 4737, 0), (33, 2369, 2)])
+def test_products_at_the_line_between_streamed_rows_and_tiles(M, N, epilogue):
+    ops = _ops()
+    torch.manual_seed(M + N)
+    K = 260
+    a, w = torch.randn(M, K, device=DEV), torch.randn(2 * N if epilogue == ops.EPILOGUE_SWIGLU else N, K, device=DEV) / math.sqrt(K)
+    base = torch.randn(M, N, device=DEV)
+    outs = [base.clone(), base.clone()]
+    ops.gemm_simt(outs[0], a, w, epilogue)
+    for m in range(0, M, 8):                                                     # streamed, whatever the width
+        assert ops.gemm_simt_route(min(8, M - m), N, epilogue) == "rows"
+        ops.gemm_simt(outs[1][m:m + 8], a[m:m + 8], w, epilogue)
+    assert torch.equal(*outs)
+
+
 # sizes whose last tile is ragged in both directions, with the tiles that the rule picks for them
 _TILES = [(100, 5003, 0, False, "64x128"), (65, 4099, 2, False, "64x128"), (65, 4099, 0, False, "64x64"), (130, 1001, 2, False, "64x64"),
           (65, 131, 1, False, "32x64"), (67, 130, 2, False, "32x64"), (100, 5003, 1, True, "64x128"), (65, 4099, 2, True, "64x128"),

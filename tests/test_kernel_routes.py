@@ -18,3 +18,15 @@ def test_rows_are_filtered_and_drawn_by_one_block_where_a_cluster_would_be_slowe
     (531, 3072, 0, False, "64x64"), (531, 6144, 2, False, "64x128"), (129, 2048, 0, False, "64x64"), (65, 130, 0, False, "32x64")])
 def test_tiles_of_products_on_cuda_cores(rows, columns, epilogue, narrow, kernel):
     assert ops.gemm_simt_route(rows, columns, epilogue, narrow=narrow) == kernel
+
+
+@pytest.mark.parametrize("rows, widest, widest_gated", [(1, 10 ** 6, 10 ** 6), (8, 10 ** 6, 10 ** 6), (9, 20480, 10 ** 6), (16, 20480, 10 ** 6), (17, 9472, 9472),
+                                                        (32, 9472, 9472), (33, 4736, 2368), (64, 4736, 2368), (65, 0, 0)])
+def test_few_rows_stream_their_weights_as_far_as_that_is_faster(rows, widest, widest_gated):
+    for epilogue, last in ((ops.EPILOGUE_STORE, widest), (ops.EPILOGUE_ACCUMULATE, widest), (ops.EPILOGUE_SWIGLU, widest_gated)):
+        if last:
+            assert ops.gemm_simt_route(rows, last, epilogue) == "rows"
+        if last < 10 ** 6:
+            assert ops.gemm_simt_route(rows, last + 1, epilogue) != "rows"
+        assert ops.gemm_simt_route(rows, 64, epilogue, aligned=False) != "rows" and ops.gemm_simt_route(rows, 64, epilogue, batch=2) != "rows"
+        assert ops.gemm_simt_route(rows, 64, epilogue, narrow=True) != "rows"
