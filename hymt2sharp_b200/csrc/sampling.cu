@@ -366,8 +366,8 @@ struct FilterParams {
 // pass (from its own cache).  Thresholds are found by three radix passes over the keys (11, 11 and 10 bits): every block counts its
 // slice's keys per bin, a block adds up its share of the bins for all, and all walk the totals from the top.  After a top-k of up to
 // FEW entries the survivors go to the first block, which ranks them and settles min-p and top-p there.  What bounds it: the chain of
-// passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows, with top-k 20, top-p and penalty 31 us (one block a
-// row: 75), with top-p alone 58 (317), with min-p alone 13 (32).
+// passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows, with top-k 20, top-p and penalty 29 us (one block a
+// row: 75), with top-p alone 57 (317), with min-p alone 13 (32).
 constexpr int FEW = 1024, BINS = 2048;
 
 struct FilterShared {
@@ -394,6 +394,10 @@ struct RowBlocks {
         if constexpr (BLOCKS > 1) cg::this_cluster().sync();
         else __syncthreads();
     }
+    __device__ int rank() const {       // (asked of the hardware where it is needed: a copy in a register slowed the counting passes, 8 rows 29 -> 31 us)
+        if constexpr (BLOCKS > 1) return cg::this_cluster().block_rank();
+        else return 0;
+    }
     template <typename V> __device__ V* of(V* mine, int rank) const {       // block `rank`'s copy of a shared variable
         if constexpr (BLOCKS > 1) return cg::this_cluster().map_shared_rank(mine, rank);
         else return mine;
@@ -402,8 +406,8 @@ struct RowBlocks {
 
 // Adds up the blocks' bins: afterwards every block has the row's in `total`.  (In the order of the blocks: the same sum everywhere.)
 template <typename V, int BLOCKS>
-__device__ void gather_bins(RowBlocks<BLOCKS> blocks, FilterShared& s, int bins, int rank) {
-    const int share = bins / BLOCKS;
+__device__ void gather_bins(RowBlocks<BLOCKS> blocks, FilterShared& s, int bins) {
+    const int share = bins / BLOCKS, rank = blocks.rank();
     blocks.sync();
     for (int i = threadIdx.x; i < share; i += THREADS) {
         V sum = 0;
@@ -477,7 +481,7 @@ filter_kernel(FilterParams p) {
                 const uint32_t key = float_key(x[i] * inv_t);
                 if ((key & mask) == prefix) atomicAdd(&s.hist[(key >> shift) & (bins - 1)], 1);
             }
-            gather_bins<int>(blocks, s, bins, rank);
+            gather_bins<int>(blocks, s, bins);
             // from the top: the bin in which the remaining-th key lies
             const int per = bins / THREADS, top = bins - 1 - tid * per;
             int mine = 0;
@@ -595,7 +599,7 @@ filter_kernel(FilterParams p) {
                     const uint32_t key = float_key(v);
                     if ((key & mask) == prefix) atomicAdd(&bins_of<float>(s)[(key >> shift) & (bins - 1)], expf(v - mx));
                 }
-                gather_bins<float>(blocks, s, bins, rank);
+                gather_bins<float>(blocks, s, bins);
                 const float* mass = totals_of<float>(s);
                 const int per = bins / THREADS, top = bins - 1 - tid * per;
                 float mine = 0.f;
