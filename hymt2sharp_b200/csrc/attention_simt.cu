@@ -586,22 +586,29 @@ int plain_prompt_rows(AttnParams p, int batch, int max_new_tokens, cudaStream_t 
     const dim3 grid((max_new_tokens + p.tokens_per_tile - 1) / p.tokens_per_tile, p.nkv * p.head_chunks, batch);
     HYMT2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "attention: grid too large (batch %d)", batch);
     const size_t smem = sizeof(float) * ((size_t)(4 * KEY_TILE + 16 * RT) * (p.d + 4) + 16 * RT * PLAIN_P_LD);
-    if (p.d <= 32) return plain_launch(attention_plain_prompt_kernel<RT, 1>, grid, smem, stream, p);
-    if (p.d <= 64) return plain_launch(attention_plain_prompt_kernel<RT, 2>, grid, smem, stream, p);
     if constexpr (RT == 4) return plain_launch(attention_plain_prompt_kernel<RT, 4>, grid, smem, stream, p);
+    else if (p.d <= 32) return plain_launch(attention_plain_prompt_kernel<RT, 1>, grid, smem, stream, p);
+    else if (p.d <= 64) return plain_launch(attention_plain_prompt_kernel<RT, 2>, grid, smem, stream, p);
     else if (p.d <= 128) return plain_launch(attention_plain_prompt_kernel<RT, 4>, grid, smem, stream, p);
     else return plain_launch(attention_plain_prompt_kernel<RT, 8>, grid, smem, stream, p);
 }
 
-// Prompts: the more rows a block has, the fewer reads an FMA costs; 32 rows instead of 64 while the blocks would not fill the SMs twice
-// (two blocks fit an SM), and for heads whose outputs would not fit the registers.
+// Rows a block of the prompt kernel.  The more it has, the fewer reads an FMA costs: 64 instead of 32 for heads of 65 to 128 entries, from
+// where such blocks fill the SMs twice over (two fit an SM).  16 heads on 4 of 128: 531 tokens 154 us with 32 rows and 172 with 64, 1,300
+// tokens 581 and 505, 2,048 1,089 and 1,030, 4,096 4,044 and 3,014, with a window of 256 588 and 477; near the line a last wave that is
+// nearly empty can cost more than the reads (8 heads on 2, 2,400 tokens: 702 and 919).  Smaller heads have too few FMAs between a row's
+// softmax and the next (16 heads on 4, 1,300 tokens: of 64 260 and 320, of 32 134 and 160), wider ones' outputs do not fit the registers.
+inline int plain_prompt_block_rows(int tokens, int nh, int d) {
+    return d > 64 && d <= 128 && (long)tokens * nh >= 64L * 2 * 148 ? 64 : 32;
+}
+
 int plain_prompt(AttnParams p, int batch, int tokens, int max_new_tokens, cudaStream_t stream) {
     const int g = p.nh / p.nkv;
-    const int rt = p.d <= 128 && (long)tokens * p.nh >= 64L * 2 * 148 ? 4 : 2;
-    p.heads_per_tile = g < 16 * rt ? g : 16 * rt;
-    p.tokens_per_tile = 16 * rt / p.heads_per_tile;
+    const int rows = plain_prompt_block_rows(tokens, p.nh, p.d);
+    p.heads_per_tile = g < rows ? g : rows;
+    p.tokens_per_tile = rows / p.heads_per_tile;
     p.head_chunks = (g + p.heads_per_tile - 1) / p.heads_per_tile;
-    return rt == 4 ? plain_prompt_rows<4>(p, batch, max_new_tokens, stream) : plain_prompt_rows<2>(p, batch, max_new_tokens, stream);
+    return rows == 64 ? plain_prompt_rows<4>(p, batch, max_new_tokens, stream) : plain_prompt_rows<2>(p, batch, max_new_tokens, stream);
 }
 
 constexpr int MERGE_WEIGHTS = 128, MERGE_COLS = 4;
@@ -796,6 +803,9 @@ static int attention_simt_general(void* out, const void* q, const void* k_cache,
     });
     return rc;
 }
+
+// Rows a block of a float32 prompt's attention works on.
+HYMT2_API int hymt2_attention_prompt_rows(int tokens, int nh, int d) { return plain_prompt_block_rows(tokens, nh, d); }
 
 HYMT2_API int hymt2_attention_simt(void* out, const void* q, const void* k_cache, const void* v_cache, int dtype,
                                    const int* block_table, int table_stride, int block_tokens,

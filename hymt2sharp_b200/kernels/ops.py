@@ -675,6 +675,11 @@ def attention_simt_scratch(tokens: int, nh: int, d: int, max_splits: int) -> tup
     return tokens * nh * max_splits * d, tokens * nh * max_splits * 2
 
 
+def attention_prompt_rows(tokens: int, nh: int, d: int) -> int:
+    """Rows (token, head) of a block in attention_simt of float32 prompts (32 or 64).  Works without a GPU."""
+    return int(_lib().hymt2_attention_prompt_rows(c_int(tokens), c_int(nh), c_int(d)))
+
+
 def attention_simt(out: torch.Tensor, q: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tensor,
                    block_table: torch.Tensor, cu_seqlens: torch.Tensor, slot_ids: torch.Tensor,
                    kv_lens: torch.Tensor, batch: int, max_new_tokens: int, nh: int, nkv: int, d: int,

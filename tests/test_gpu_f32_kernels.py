@@ -1,7 +1,7 @@
-"""The kernels of the 32-bit path at the sizes where their tiles end: the products for few rows and in tiles, and the attention of
-its plain form.  Every sum keeps one
-order whichever kernel runs, so the kernels are compared with each other bit for bit, and with 64-bit sums within the bound of a
-chain of K float32 FMAs, K * 2^-24 * sum |a| |w| (twice that, for the add into the output)."""
+"""The kernels of the 32-bit path: the products of few rows and in every tile (bfloat16 operands too) at the sizes where their tiles end,
+and the attention of its plain form in every instance that a rule picks.  Every sum keeps one order whichever kernel runs, so the
+kernels are compared with each other bit for bit, and with 64-bit sums within the bound of a chain of K float32 FMAs,
+K * 2^-24 * sum |a| |w| (twice that, for the add into the output)."""
 import math
 
 import numpy as np
@@ -156,3 +156,23 @@ def test_a_row_does_not_know_values_of_tiles_it_cannot_see(nh, nkv, d, window):
             assert torch.equal(outs[0][p], outs[1][p]), p
         if any(low <= at <= p for at in (40, 150, 199)):
             assert not outs[1][p].isfinite().any(), p
+
+
+@pytest.mark.parametrize("nh, nkv, d, rows", [(16, 4, 128, 64), (12, 4, 104, 64), (16, 16, 72, 64), (40, 1, 128, 64), (16, 4, 64, 32), (16, 4, 24, 32), (16, 8, 136, 32)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_long_prompts_are_the_general_kernels_bit_for_bit(nh, nkv, d, rows, window):
+    """The blocks of 64 rows, several tokens each, with windows and parts of prompts; heads and tokens that do not fill a block."""
+    ops = _ops()
+    torch.manual_seed(nh * 100 + d)
+    news, lens = [1001, 3, 613], [1001, 90, 900]
+    T = sum(news)
+    assert ops.attention_prompt_rows(T, nh, d) == rows
+    kp, vp, table = _paged([torch.randn(L, nkv, d, device=DEV) for L in lens], [torch.randn(L, nkv, d, device=DEV) for L in lens], 64, torch.float32)
+    q = torch.randn(T, nh * d, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    outs = []
+    for x in (q, _shifted(q)):       # (the second takes the general kernel)
+        out = torch.full((T, nh * d), 5.0, device=DEV)
+        ops.attention_simt(out, x, kp, vp, table, i32([0, 1001, 1004, 1617]), i32([0, 1, 2]), i32(lens), 3, 1001, nh, nkv, d, 1 / math.sqrt(d), window)
+        outs.append(out)
+    assert torch.equal(*outs)
