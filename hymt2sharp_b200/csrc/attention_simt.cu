@@ -593,13 +593,14 @@ int plain_prompt_rows(AttnParams p, int batch, int max_new_tokens, cudaStream_t 
     else return plain_launch(attention_plain_prompt_kernel<RT, 8>, grid, smem, stream, p);
 }
 
-// Rows a block of the prompt kernel.  The more it has, the fewer reads an FMA costs: 64 instead of 32 for heads of 65 to 128 entries, from
+// Rows a block of the prompt kernel.  The more it has, the fewer reads an FMA costs: 64 instead of 32 for heads of 96 to 128 entries, from
 // where such blocks fill the SMs twice over (two fit an SM).  16 heads on 4 of 128: 531 tokens 154 us with 32 rows and 172 with 64, 1,300
 // tokens 581 and 505, 2,048 1,089 and 1,030, 4,096 4,044 and 3,014, with a window of 256 588 and 477; near the line a last wave that is
 // nearly empty can cost more than the reads (8 heads on 2, 2,400 tokens: 702 and 919).  Smaller heads have too few FMAs between a row's
-// softmax and the next (16 heads on 4, 1,300 tokens: of 64 260 and 320, of 32 134 and 160), wider ones' outputs do not fit the registers.
+// softmax and the next (16 heads on 4, 1,300 and 4,096 tokens: of 96 399 and 428, 2,776 and 2,562; of 72 365 and 446, 2,257 and 2,351; of 64
+// 260 and 320, 1,643 and 1,732), wider ones' outputs do not fit the registers.
 inline int plain_prompt_block_rows(int tokens, int nh, int d) {
-    return d > 64 && d <= 128 && (long)tokens * nh >= 64L * 2 * 148 ? 64 : 32;
+    return d >= 96 && d <= 128 && (long)tokens * nh >= 64L * 2 * 148 ? 64 : 32;
 }
 
 int plain_prompt(AttnParams p, int batch, int tokens, int max_new_tokens, cudaStream_t stream) {

@@ -32,7 +32,7 @@ def test_few_rows_stream_their_weights_as_far_as_that_is_faster(rows, widest, wi
         assert ops.gemm_simt_route(rows, 64, epilogue, narrow=True) != "rows"
 
 
-@pytest.mark.parametrize("tokens, heads, d, rows", [(531, 16, 128, 32), (1183, 16, 128, 32), (1184, 16, 128, 64), (4096, 16, 72, 64), (4096, 16, 64, 32),
+@pytest.mark.parametrize("tokens, heads, d, rows", [(531, 16, 128, 32), (1183, 16, 128, 32), (1184, 16, 128, 64), (4096, 16, 96, 64), (4096, 16, 88, 32), (4096, 16, 64, 32),
                                                     (4096, 16, 24, 32), (4096, 16, 136, 32), (18944, 1, 128, 64)])
 def test_rows_a_block_of_32_bit_prompt_attention(tokens, heads, d, rows):
     assert ops.attention_prompt_rows(tokens, heads, d) == rows
