@@ -2,8 +2,9 @@
 // Both operands are K-contiguous (W is stored [out][in], the layout of
 // src/HyMT2Sharp/HunyuanDenseModel.cs:586-587).  Products and sums are float32
 // FMAs in ascending K order, so an output element does not depend on M or on
-// its row's place in the batch.  This is the whole of the 32-bit path and the
-// fallback of the bfloat16 path for shapes that the tensor-core kernels refuse.
+// its row's place in the batch.  This is the path of small and misaligned 32-bit
+// weights (the others go to gemm_f32_tc.cu), of 32-bit batches, and of bfloat16
+// shapes that the tensor-core kernels refuse.
 //
 // Epilogues:
 //   0 store      C = acc

@@ -36,7 +36,8 @@ _library = None
 # thirty.  A short prompt's step is as long as the host takes to launch it.  p: address, i: int, l: long, f: float.
 _DECLARED = {"hymt2_gemm_tc_norm": "pippiiilllipl" "pippp" "iifppip" "iffp",
              "hymt2_gemm_tc_rope_kv": "ppiillpppp" "iipppppipp" "ifiiipppiif",
-             "hymt2_attention_prefill_tc": "pppplpiipppiiiiiifipp"}
+             "hymt2_attention_prefill_tc": "pppplpiipppiiiiiifipp",
+             "hymt2_gemm_f32_tc": "pppiiillliplpp" "iffp"}
 
 
 def _lib():
@@ -366,6 +367,62 @@ def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int
                                   _ptr(w), c_int(dtype_code(w.dtype)), c_int(M), c_int(N), c_int(K),
                                   c_long(a.stride(0)), c_long(w.stride(0)), c_long(out.stride(0)),
                                   c_int(epilogue), *_glu_arguments(glu, glu_bias, N, epilogue), _stream()), "gemm_simt")
+
+
+# float32 products from these sizes of the weight on go to the tensor cores, whatever the number of rows, so that a row's sums do not depend
+# on it.  us on CUDA cores and there, 1 row / 8 / 32 / 531: 512 x 512 3.4 5.4 / 3.9 5.3 / 7.0 6.4 / 23 14; 1,536 x 512 gated 4.9 5.9 / 5.7 6.2 /
+# 9.5 7.4 / 33 19; 1,024 x 1,024 5.7 6.0 / 7.0 6.2 / 14 7.6 / 48 26; 2,048 x 2,048 10.3 10.2 / 13.0 10.4 / 24 13 / 127 45.
+F32_TC_MIN_SIDE, F32_TC_MIN_ENTRIES = 512, 1 << 20
+_f32_plans: dict = {}
+
+
+def gemm_f32_tc_plan(rows: int, columns: int, inner: int, epilogue: int = EPILOGUE_STORE, aligned: bool = True) -> tuple:
+    """(whether a kernel in front cuts the rows into pieces, tokens of a tile, stages of the ring, parts of the inner dimension,
+    bytes of scratch) of a gemm_f32_tc.  Works without a GPU."""
+    key = (rows, columns, inner, epilogue, aligned)
+    hit = _f32_plans.get(key)
+    if hit is None:
+        out = (c_long * 5)()
+        _check(_lib().hymt2_gemm_f32_tc_plan(c_int(rows), c_int(columns), c_int(inner), c_int(epilogue), c_int(aligned), out), "gemm_f32_tc_plan", 0)
+        if len(_f32_plans) > 4096:
+            _f32_plans.clear()
+        hit = _f32_plans[key] = tuple(out)
+    return hit
+
+
+def gemm_f32_tc_supported(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int) -> bool:
+    """Whether the float32 product on tensor cores takes these operands: all float32, rows of w on 16 bytes, a weight that is large
+    enough to be worth its start."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32:
+        return False
+    if a.dim() != 2 or w.dim() != 2 or out.dim() != 2 or a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
+        return False
+    if min(w.shape) < F32_TC_MIN_SIDE or w.numel() < F32_TC_MIN_ENTRIES:
+        return False
+    return w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
+
+
+def gemm_f32_tc(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int, status: torch.Tensor, glu: GluRule | None = None,
+                glu_bias: torch.Tensor | None = None) -> None:
+    """out[M, N] = epilogue(a[M, K] @ w[N, K]^T), float32, on the tcgen05 tensor cores: every operand as three bfloat16 pieces whose
+    products are exact, the sums in float32.  Not further from the exact product than a chain of float32 FMAs, and the same bit
+    for bit for a row whatever other rows there are.  With EPILOGUE_SWIGLU w has 2N rows."""
+    M, N = out.shape
+    K = a.shape[1]
+    rows_w = 2 * N if epilogue == EPILOGUE_SWIGLU else N
+    for t, n in ((out, "out"), (a, "a"), (w, "w")):
+        if not t.is_cuda or t.dim() != 2 or t.stride(1) != 1 or t.dtype != torch.float32:
+            raise KernelError(f"gemm_f32_tc: {n} must be a float32 CUDA matrix with contiguous rows")
+    if a.shape[0] != M or w.shape != (rows_w, K) or K == 0 or w.stride(0) % 4 or w.data_ptr() % 16:
+        raise KernelError(f"gemm_f32_tc: operands out {tuple(out.shape)} a {tuple(a.shape)} w {tuple(w.shape)} epilogue {epilogue} are not taken")
+    if M == 0 or N == 0:
+        return
+    lda = a.stride(0)
+    planes, _, _, _, scratch_bytes = gemm_f32_tc_plan(M, N, K, epilogue, a.data_ptr() % 16 == 0 and lda % 4 == 0)
+    scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=out.device) if planes else None
+    _check(_lib().hymt2_gemm_f32_tc(out.data_ptr(), a.data_ptr(), w.data_ptr(), M, N, K, lda, w.stride(0), out.stride(0), epilogue,
+                                    _address(scratch), scratch_bytes, status.data_ptr(), _raw_stream(),
+                                    *_glu_arguments(glu, glu_bias, N, epilogue)), "gemm_f32_tc", 2 if planes else 1)
 
 
 def gemm_simt_route(rows: int, columns: int, epilogue: int = EPILOGUE_STORE, batch: int = 1, narrow: bool = False, aligned: bool = True) -> str:

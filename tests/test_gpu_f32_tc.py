@@ -1,0 +1,99 @@
+"""The float32 product on tensor cores (three bfloat16 pieces an operand): against 64-bit sums, at the sizes where its tiles, chunks and
+parts of K end, and bit for bit the same for a row whatever other rows there are.
+
+The bound, times sum |a| |w|: the dropped pieces of a product 2^-24; in a chunk of 64 entries four additions of the sum's own size, each
+cut off at 2^-22 of what it has reached at most; an addition of float32 a chunk and a part, rounded at 2^-24."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, _ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(a, w, K):
+    return (1 + 16 + -(-K // 64) + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 1e-12
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65, 97, 200])
+@pytest.mark.parametrize("N, K", [(512, 512), (520, 516), (131, 64), (900, 1100), (2000, 132)])
+@pytest.mark.parametrize("narrow", [False, True])
+def test_products_in_every_form(M, N, K, narrow):
+    ops = _ops()
+    torch.manual_seed(M + N + K)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    a, w = torch.randn(M, K, device=DEV), torch.randn(2 * N, K, device=DEV) / math.sqrt(K)
+    if narrow:                      # a bfloat16 checkpoint's weights: only their first pieces are multiplied
+        w = w.bfloat16().float()
+    shifted = torch.empty(M * K + 1, device=DEV)[1:].view(M, K).copy_(a)      # rows that do not start on 16 bytes: the form with planes
+    for epilogue, rows in ((ops.EPILOGUE_STORE, N), (ops.EPILOGUE_ACCUMULATE, N), (ops.EPILOGUE_SWIGLU, 2 * N)):
+        base, outs = torch.randn(M, N, device=DEV), []
+        for x in (a, shifted):
+            out = base.clone()
+            ops.gemm_f32_tc(out, x, w[:rows], epilogue, status)
+            outs.append(out)
+        assert torch.equal(*outs)
+        one = base[M - 1:].clone()
+        ops.gemm_f32_tc(one, a[M - 1:].contiguous(), w[:rows], epilogue, status)
+        assert torch.equal(one, outs[0][M - 1:])
+        ref, bound = a.double() @ w[:rows].double().T, _bound(a, w[:rows], K)
+        if epilogue == ops.EPILOGUE_SWIGLU:
+            g, u = ref[:, :N], ref[:, N:]
+            silu = g / (1 + torch.exp(-g))
+            want = silu * u
+            # |silu'| <= 1.1; the exponential and the division are within a few units of 2^-24
+            bound = 1.1 * bound[:, :N] * (u.abs() + bound[:, N:]) + silu.abs() * bound[:, N:] + 2.0 ** -20 * want.abs()
+        else:
+            want = ref + base.double() if epilogue == ops.EPILOGUE_ACCUMULATE else ref
+            bound = bound + 2.0 ** -23 * (want.abs() + ref.abs())
+        assert ((outs[0].double() - want).abs() <= bound + 1e-12).all()
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("N, K, epilogue", [(1024, 2048, 0), (2048, 6144, 1), (3072, 2048, 2), (640, 8192, 0)])
+def test_a_row_does_not_depend_on_the_others_and_is_nearer_than_a_chain(N, K, epilogue):
+    """Long sums over several parts of K, in tiles of every width; and further from the exact product than a chain of FMAs it must not be."""
+    ops = _ops()
+    torch.manual_seed(N)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    M = 531
+    a, w = torch.randn(M, K, device=DEV), torch.randn(2 * N if epilogue == 2 else N, K, device=DEV) / math.sqrt(K)
+    base = torch.randn(M, N, device=DEV)
+    whole = base.clone()
+    ops.gemm_f32_tc(whole, a, w, epilogue, status)
+    for m in (1, 16, 32, 64, 129, 300):
+        part = base[M - m:].clone()
+        ops.gemm_f32_tc(part, a[M - m:], w, epilogue, status)
+        assert torch.equal(part, whole[M - m:]), m
+    if epilogue == 0:
+        chain = torch.empty_like(base)
+        ops.gemm_simt(chain, a, w, epilogue)
+        ref = a.double() @ w.double().T
+        assert (whole.double() - ref).norm() <= (chain.double() - ref).norm()
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M", [8, 150])
+def test_entries_at_the_ends_of_the_range(M):
+    """Infinities, NaN and entries whose first piece rounds to infinity give what the chain of FMAs gives; tiny ones lose nothing."""
+    ops = _ops()
+    torch.manual_seed(M)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    N, K = 512, 1024
+    for epilogue in (ops.EPILOGUE_STORE, ops.EPILOGUE_SWIGLU):
+        a, w = torch.randn(M, K, device=DEV), torch.randn(2 * N if epilogue == ops.EPILOGUE_SWIGLU else N, K, device=DEV) / math.sqrt(K)
+        a[3, 5], a[5, 9], w[11, 17], a[M - 1, 0], w[len(w) - 1, 3] = math.inf, math.nan, -math.inf, 3.4e38, 1e30
+        a[6] *= 1e-30
+        w[100] *= 1e-20
+        bound = _bound(a.nan_to_num(0, 0, 0), w.nan_to_num(0, 0, 0), K)[:, :N] + K * 2.0 ** -24 * (a.nan_to_num(0, 0, 0).double().abs() @ w.nan_to_num(0, 0, 0).double().abs().T)[:, :N]
+        got, want = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+        ops.gemm_f32_tc(got, a, w, epilogue, status)
+        ops.gemm_simt(want, a, w, epilogue)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        assert (got[got.isinf()] == want[want.isinf()]).all()
+        ok = want.isfinite()
+        if epilogue == ops.EPILOGUE_STORE:          # (the chain's own error is K * 2^-24 * sum |a| |w|)
+            assert ((got.double() - want.double()).abs() <= bound + 1e-44)[ok].all()
+    assert status.tolist() == [0, 0, 0, 0]
