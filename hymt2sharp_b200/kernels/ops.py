@@ -1707,6 +1707,36 @@ def gemm_grouped(kernel: str, out: torch.Tensor, a: torch.Tensor, w: torch.Tenso
                "gemm_tc_grouped")
 
 
+# The grouped product of few rows goes to the tensor cores from this many weight entries on that a step may touch (pairs of token and choice
+# times a matrix's entries): below, the start of its clusters is longer than the reading.  us, CUDA cores / tensor cores: 4.2 M entries 4.1 6.6
+# and 7.3 6.9; 8.4 M 7.3 7.3 and 6.6 9.3; 16.8 M 12.4 9.8, 12.3 9.7 and 13.6 11.2; 67 M 36 27 and 40 27; 134 M 53 33.
+FEW_MIN_ENTRIES = 12 << 20
+
+
+def gemm_grouped_few_supported(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
+    """Whether `pairs` (token, choice) pairs' grouped product runs on the tensor cores in tiles of 8 rows: bfloat16, rows on 16 bytes, the
+    inner size a multiple of 256 up to 4,096, and enough of the matrices in use to be worth it."""
+    K = a.shape[1]
+    return a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 256 == 0 and K <= 4096 and a.stride(1) == 1 and a.stride(0) % 8 == 0 \
+        and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous() and min(pairs, w.shape[0]) * w.shape[1] * K >= FEW_MIN_ENTRIES
+
+
+def gemm_grouped_few(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, row_token: torch.Tensor, gather: bool,
+                     epilogue: int = EPILOGUE_STORE, glu: GluRule | None = None) -> None:
+    """gemm_grouped's "skinny" on the tcgen05 tensor cores: bfloat16 operands, the inner size a multiple of 256 up to 4,096."""
+    _need(out, "out", None, 2); _need(a, "a", torch.bfloat16, 2); _need(w, "w", torch.bfloat16, 3)
+    _need(tile_group, "tile_group", torch.int32, 1); _need(row_token, "row_token", torch.int32, 1)
+    tiles, tile = tile_group.numel() - 1, gemm_group_tile("skinny")
+    gated = epilogue == EPILOGUE_SWIGLU
+    N, K = w.shape[1] // (2 if gated else 1), w.shape[2]
+    if (gated and w.shape[1] % 2) or out.shape != (tiles * tile, N) or a.shape[1] != K or row_token.numel() < tiles * tile or (not gather and a.shape[0] < tiles * tile):
+        raise KernelError(f"gemm_grouped_few: shapes out {tuple(out.shape)} a {tuple(a.shape)} w {tuple(w.shape)} tiles {tiles} of {tile}")
+    _check(_lib().hymt2_gemm_grouped_few(_ptr(out), c_int(dtype_code(out.dtype)), _ptr(a), _ptr(w), _ptr(tile_group), _ptr(row_token), c_int(1 if gather else 0),
+                                         c_int(tiles), c_int(w.shape[0]), c_int(N), c_int(K), c_long(a.stride(0)), c_long(out.stride(0)), c_int(epilogue),
+                                         *_glu_arguments(glu, None, 0, epilogue, with_bias=False), _ptr(device_status(out.device)), _stream()),
+           "gemm_grouped_few")
+
+
 def gemm_simt_grouped(out, a, w, tile_group, row_token, gather: bool, epilogue: int = EPILOGUE_STORE) -> None:
     gemm_grouped("simt", out, a, w, tile_group, row_token, gather, epilogue)
 

@@ -164,13 +164,17 @@ class RoutedExperts:
         if kernel == "tc":     # its tiles come by TMA, which reads rows side by side
             rows, gather = torch.empty((tiles * tile, self.hidden), dtype=x.dtype, device=dev), False
             ops.moe_gather(rows, x, row_token)
+        # (one rule for both products: tiles of 8 rows go where the reading is worth the start)
+        few = kernel == "skinny" and self.intermediate % 256 == 0 and self.intermediate <= 4096 \
+            and ops.gemm_grouped_few_supported(x, self.up, T * self.top)
+        grouped = ops.gemm_grouped_few if few else lambda *args: ops.gemm_grouped(kernel, *args)
         ops.tag = "experts_up"
         if self.gated and self.activation in ("silu", "clamped") and kernel != "simt":
             act = torch.empty((tiles * tile, self.intermediate), dtype=x.dtype, device=dev)
-            ops.gemm_grouped(kernel, act, rows, self.up, tile_group, row_token, gather, ops.EPILOGUE_SWIGLU, self.glu)
+            grouped(act, rows, self.up, tile_group, row_token, gather, ops.EPILOGUE_SWIGLU, self.glu)
         elif self.gated:
             both = torch.empty((tiles * tile, 2 * self.intermediate), dtype=x.dtype, device=dev)
-            ops.gemm_grouped(kernel, both, rows, self.up, tile_group, row_token, gather, ops.EPILOGUE_STORE)
+            grouped(both, rows, self.up, tile_group, row_token, gather, ops.EPILOGUE_STORE)
             act = torch.empty((tiles * tile, self.intermediate), dtype=x.dtype, device=dev)
             # (rows of tiles not in use hold whatever was there: nobody reads them)
             if self.activation == "clamped":
@@ -179,10 +183,10 @@ class RoutedExperts:
                 ops.gated_act(act, both, GATED_ACTIVATIONS[self.activation])
         else:
             act = torch.empty((tiles * tile, self.intermediate), dtype=x.dtype, device=dev)
-            ops.gemm_grouped(kernel, act, rows, self.up, tile_group, row_token, gather, ACTIVATIONS[self.activation])
+            grouped(act, rows, self.up, tile_group, row_token, gather, ACTIVATIONS[self.activation])
         y = torch.empty((tiles * tile, self.hidden), dtype=torch.float32, device=dev)
         ops.tag = "experts_down"
-        ops.gemm_grouped(kernel, y, act, self.down, tile_group, row_token, False, ops.EPILOGUE_STORE)
+        grouped(y, act, self.down, tile_group, row_token, False, ops.EPILOGUE_STORE)
         ops.tag = None
         return y, pair_row, weight, z
 
