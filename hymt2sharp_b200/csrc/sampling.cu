@@ -25,11 +25,11 @@ constexpr int THREADS = 1024;
 
 __global__ void __launch_bounds__(THREADS)
 argmax_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_stride, int vocab,
-              const int* __restrict__ row_map) {
+              const int* __restrict__ row_map, const int* __restrict__ drawn) {
     __shared__ float sval[32];
     __shared__ int sidx[32];
     const int row = blockIdx.x;
-    if (row_map && row_map[row] < 0) return;
+    if ((row_map && row_map[row] < 0) || (drawn && drawn[row])) return;
     const float* x = logits + (size_t)row * row_stride;
     float best = -INFINITY;
     int best_i = 0x7fffffff;
@@ -65,13 +65,13 @@ constexpr int ARGMAX_PIECE = 4096;
 
 __global__ void __launch_bounds__(256)
 argmax_pieces_kernel(float* __restrict__ piece_val, int* __restrict__ piece_idx, const float* __restrict__ logits,
-                     long row_stride, int vocab, const int* __restrict__ row_map) {
+                     long row_stride, int vocab, const int* __restrict__ row_map, const int* __restrict__ drawn) {
     __shared__ float sval[8];
     __shared__ int sidx[8];
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.y, piece = blockIdx.x;
-    if (row_map && row_map[row] < 0) return;
+    if ((row_map && row_map[row] < 0) || (drawn && drawn[row])) return;
     const float* x = logits + (size_t)row * row_stride;
     const int begin = piece * ARGMAX_PIECE, end = min(vocab, begin + ARGMAX_PIECE);
     float best = -INFINITY;
@@ -98,11 +98,12 @@ argmax_pieces_kernel(float* __restrict__ piece_val, int* __restrict__ piece_idx,
 }
 
 __global__ void argmax_final_kernel(int* __restrict__ out, const float* __restrict__ piece_val,
-                                    const int* __restrict__ piece_idx, int pieces, const int* __restrict__ row_map) {
+                                    const int* __restrict__ piece_idx, int pieces, const int* __restrict__ row_map,
+                                    const int* __restrict__ drawn) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x;
-    if (row_map && row_map[row] < 0) return;
+    if ((row_map && row_map[row] < 0) || (drawn && drawn[row])) return;
     float best = -INFINITY;
     int best_i = 0x7fffffff;
     for (int i = threadIdx.x; i < pieces; i += 32) {
@@ -180,14 +181,14 @@ __device__ __forceinline__ V block_exclusive_scan(V v, V* warp_totals, V* total)
 __global__ void __launch_bounds__(THREADS)
 sample_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_stride, int vocab,
               const float* __restrict__ inv_temperature, uint64_t* __restrict__ rng_states,
-              const int* __restrict__ row_map) {
+              const int* __restrict__ row_map, const int* __restrict__ drawn) {
     __shared__ float scratch[33];
     __shared__ float warp_totals[32];
     __shared__ float total_s;
     __shared__ int pick_s, owner_s;
     const int row = blockIdx.x;
     const int srow = row_map ? row_map[row] : row;  // the sequence's row in the per-sequence arrays
-    if (srow < 0) return;
+    if (srow < 0 || (drawn && drawn[row])) return;
     const float* x = logits + (size_t)row * row_stride;
     const float inv_t = inv_temperature[srow];
     if (!(inv_t > 0.f)) return;  // a greedy row: argmax has written its token
@@ -257,7 +258,8 @@ constexpr int CLUSTER = 8, CLUSTER_PIECES = THREADS / CLUSTER;
 
 __global__ void __launch_bounds__(THREADS)
 sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, long row_stride, int vocab,
-                      const float* __restrict__ inv_temperature, uint64_t* __restrict__ rng_states, const int* __restrict__ row_map) {
+                      const float* __restrict__ inv_temperature, uint64_t* __restrict__ rng_states, const int* __restrict__ row_map,
+                      const int* __restrict__ drawn) {
     extern __shared__ float values[];          // [CLUSTER_PIECES][piece, made odd]
     __shared__ float scratch[33], warp_totals[32], parts[THREADS], maxima[CLUSTER];
     __shared__ float total_s, u_s;
@@ -266,7 +268,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, l
     pdl_wait();
     const int row = blockIdx.x / CLUSTER, rank = blockIdx.x % CLUSTER;
     const int srow = row_map ? row_map[row] : row;
-    if (srow < 0) return;
+    if (srow < 0 || (drawn && drawn[row])) return;
     const float inv_t = inv_temperature[srow];
     if (!(inv_t > 0.f)) return;                // a greedy row: argmax has written its token (all of its blocks leave alike)
     cluster.sync();                            // (every block of the row runs: its shared memory may be written to)
@@ -360,14 +362,23 @@ struct FilterParams {
     const int* history;            // [sequence, history_stride] recent tokens, -1 = empty
     int history_stride;
     const int* row_map;            // logits row -> sequence row, < 0 = skip
+    // where the token can be drawn from the few survivors of a row at once (all null: it is not)
+    int* out;                      // [rows] the token
+    uint64_t* rng_states;          // per sequence
+    int* drawn;                    // [rows] whether it was
 };
 
 // A row is filtered by one block or a cluster of them, each with a contiguous slice of the vocabulary, which it reads again in every
 // pass (from its own cache).  Thresholds are found by three radix passes over the keys (11, 11 and 10 bits): every block counts its
-// slice's keys per bin, a block adds up its share of the bins for all, and all walk the totals from the top.  After a top-k of up to
-// FEW entries the survivors go to the first block, which ranks them and settles min-p and top-p there.  What bounds it: the chain of
-// passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows, with top-k 20, top-p and penalty 29 us (one block a
-// row: 75), with top-p alone 57 (317), with min-p alone 13 (32).
+// slice's keys per bin, a block adds up its share of the bins for all, and all walk the totals from the top.  What bounds it: the chain of
+// passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows: with top-p alone 57 us (one block a row: 317), with
+// min-p alone 13 (32).
+//
+// A top-k of up to FEW entries with min-p or top-p behind it needs one pass over the bins, of the threads' largest keys alone: the
+// lower edge of the bin that holds the k-th largest of them cannot lie above the k-th largest key of the row.  What reaches that
+// edge (a few more than k entries, as a rule) goes to the first block, which ranks it, keeps k, settles min-p and top-p and, asked
+// to, draws the token as the kernels above would.  With more than FEW such entries the row goes the long way.  120,818 logits, 8 rows,
+// top-k 20, top-p and penalty: 20 us with the draw; three passes over all keys took 25 us, and the draw's own pass over the row 20 more.
 constexpr int FEW = 1024, BINS = 2048;
 
 struct FilterShared {
@@ -378,10 +389,13 @@ struct FilterShared {
     int at[FEW];
     int warp_i[32];
     float warp_f[32], scratch[33];
+    int order[FEW];              // the kept survivors in the order of their indices
+    float parts[THREADS];
     int counts[CLUSTER];         // a number of every block's
     float floats[CLUSTER];
     int total_i, bin, need, n_few;
-    float total_f, above;
+    float total_f, above, u;
+    int owner, last;
 };
 
 template <typename V> __device__ __forceinline__ V* bins_of(FilterShared& s) { return reinterpret_cast<V*>(s.hist); }
@@ -424,14 +438,120 @@ __device__ __forceinline__ void swap_values(RowBlocks<BLOCKS> blocks, V* mine, i
     blocks.sync();
 }
 
+// The bin, counted from the top of `bins` in s.total, in which the remaining-th key lies, and how many of it are needed (s.bin, s.need).
+__device__ __forceinline__ void find_bin(FilterShared& s, int bins, int remaining) {
+    const int per = bins / THREADS, top = bins - 1 - (int)threadIdx.x * per;
+    int mine = 0;
+    for (int i = 0; i < per; i++) mine += s.total[top - i];
+    int before = block_exclusive_scan<int>(mine, s.warp_i, &s.total_i);
+    if (before < remaining && before + mine >= remaining) {
+        int i = 0;
+        while (before + s.total[top - i] < remaining) before += s.total[top - i++];
+        s.bin = top - i;
+        s.need = remaining - before;
+    }
+    __syncthreads();
+}
+
+// The token of a row of which `kept` of the first block's threads hold one survivor each: its value v = logit * inv_t and its index.
+// What sample_kernel makes of the row with everything else at -inf, bit for bit: its pieces' sums hold the same terms in the order
+// of their indices, and zeros.  False (nothing drawn): a value is not finite.
+__device__ __forceinline__ bool draw_from(FilterShared& s, const FilterParams& p, int row, int srow, bool kept, float v, int index) {
+    const int tid = threadIdx.x;
+    if (__syncthreads_or(kept && !isfinite(v))) return false;
+    const float mx = block_max(kept ? v : -INFINITY, s.scratch);
+    const float pr = kept ? expf(v - mx) : 0.f;
+    // the survivors in the order of their indices
+    s.at[tid] = kept ? index : 0x7fffffff;
+    s.parts[tid] = 0.f;
+    if (tid == 0) {
+        uint64_t* state = p.rng_states + (size_t)srow * 4;
+        s.u = (float)(xoshiro_next(state) >> 40) * (1.0f / 16777216.0f);
+        s.owner = 0x7fffffff;
+        s.last = -1;
+    }
+    const int n = __syncthreads_count(kept);
+    int place = 0;
+    if (kept)
+        for (int j = 0; j < FEW && j < s.n_few; j++) place += s.at[j] < index;
+    __syncthreads();
+    if (kept) {
+        s.sorted[place] = pr;
+        s.order[place] = index;
+    }
+    __syncthreads();
+    const int piece = (p.vocab + THREADS - 1) / THREADS;
+    if (tid < n) {
+        const int mine = s.order[tid] / piece;
+        if (tid == 0 || s.order[tid - 1] / piece != mine) {
+            float part = 0.f;
+            for (int j = tid; j < n && s.order[j] / piece == mine; j++) part += s.sorted[j];
+            s.parts[mine] = part;
+        }
+    }
+    __syncthreads();
+    const float part = s.parts[tid];
+    const float before = block_exclusive_scan<float>(part, s.warp_f, &s.total_f);
+    const float r = s.u * s.total_f;
+    if (part > 0.f && before + part >= r) atomicMin(&s.owner, tid);
+    if (tid < n && s.sorted[tid] > 0.f) atomicMax(&s.last, s.order[tid]);
+    __syncthreads();
+    if (tid == s.owner) {
+        float acc = before;
+        int pick = -1, last = -1;
+        for (int j = 0; j < n; j++) {
+            if (s.order[j] / piece != tid || s.sorted[j] <= 0.f) continue;
+            last = s.order[j];
+            acc += s.sorted[j];
+            if (acc >= r) { pick = last; break; }
+        }
+        p.out[row] = pick >= 0 ? pick : last;
+    }
+    if (tid == 0 && s.owner == 0x7fffffff) p.out[row] = s.last >= 0 ? s.last : 0;
+    return true;
+}
+
+// The n entries in s.few are what a row's k largest are among: the first k of them stay (ties in index order), min-p and top-p take
+// some of those away, and the token may be drawn.  One block.
+__device__ __forceinline__ void settle_few(FilterShared& s, const FilterParams& p, int row, int srow, float* x, float inv_t, int n, int k,
+                                           float top_p, float min_p) {
+    const int tid = threadIdx.x;
+    // ranks by key, ties by index; the mass before an entry is then a scan
+    const unsigned long long mine = tid < n ? s.few[tid] : 0ull;
+    int place = 0;
+    for (int j = 0; j < n; j++) place += s.few[j] > mine;
+    if (tid < n) {
+        const int i = (int)~(uint32_t)mine;
+        if (place < k) {
+            s.sorted[place] = x[i] * inv_t;
+            s.at[place] = i;
+        } else x[i] = -INFINITY;
+    }
+    __syncthreads();
+    const int stay = min(n, k);
+    const float v = tid < stay ? s.sorted[tid] : -INFINITY;
+    const int index = tid < stay ? s.at[tid] : 0;
+    const float mx = block_max(v, s.scratch);
+    const float pr = v == -INFINITY ? 0.f : expf(v - mx);
+    const float before = block_exclusive_scan<float>(pr, s.warp_f, &s.total_f);
+    const float limit = top_p * s.total_f;      // a share of the mass from before min-p (Sampling.cs:272-274)
+    const bool dropped = (min_p > 0.f && pr < min_p) || (top_p < 1.f && before >= limit);
+    if (tid < stay && dropped) x[index] = -INFINITY;
+    if (p.drawn) {
+        __syncthreads();
+        if (draw_from(s, p, row, srow, tid < stay && !dropped, v, index) && tid == 0) p.drawn[row] = 1;
+    }
+}
+
 template <int BLOCKS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1)
 filter_kernel(FilterParams p) {
     __shared__ FilterShared s;
     const RowBlocks<BLOCKS> blocks;
     pdl_wait();
     const int row = blockIdx.x / BLOCKS, rank = blockIdx.x % BLOCKS, tid = threadIdx.x;
     const int srow = p.row_map ? p.row_map[row] : row;
+    if (p.drawn && rank == 0 && tid == 0) p.drawn[row] = 0;
     if (srow < 0) return;
     float* x = p.logits + (size_t)row * p.row_stride;
     const int vocab = p.vocab, slice = (vocab + BLOCKS - 1) / BLOCKS;
@@ -469,6 +589,42 @@ filter_kernel(FilterParams p) {
     const bool by_mass = top_p < 1.f || min_p > 0.f;
     const bool by_rank = k > 0 && k < vocab, few = by_rank && k <= FEW && by_mass;
 
+    if (few) {
+        // a lower edge of the k-th largest key, from the threads' largest
+        for (int i = tid; i < BINS; i += THREADS) s.hist[i] = 0;
+        uint32_t largest = 0;
+#pragma unroll 8
+        for (int i = begin + tid; i < end; i += THREADS) largest = max(largest, float_key(x[i] * inv_t));
+        __syncthreads();
+        if (begin + tid < end) atomicAdd(&s.hist[largest >> 21], 1);
+        gather_bins<int>(blocks, s, BINS);
+        if (tid == 0) s.bin = 0;                    // (fewer threads than k hold an entry: everything reaches the edge)
+        __syncthreads();
+        find_bin(s, BINS, k);
+        const uint32_t edge = (uint32_t)s.bin << 21, lowest = float_key(-INFINITY);
+        int* n_few = blocks.of(&s.n_few, 0);
+        unsigned long long* list = blocks.of(s.few, 0);
+        // what lies below the edge is dropped whichever way the row goes on
+#pragma unroll 8
+        for (int i = begin + tid; i < end; i += THREADS) {
+            const uint32_t key = float_key(x[i] * inv_t);
+            if (key < edge) x[i] = -INFINITY;
+            else if (key > lowest) {
+                const int at = atomicAdd(n_few, 1);
+                if (at < FEW) list[at] = (unsigned long long)key << 32 | (uint32_t)~i;
+            } else x[i] = -INFINITY;
+        }
+        blocks.sync();
+        const int n = *n_few;
+        if (n <= FEW) {
+            if (rank == 0) settle_few(s, p, row, srow, x, inv_t, n, k, top_p, min_p);
+            blocks.sync();     // (the first block stays until the others have read its count)
+            return;
+        }
+        blocks.sync();         // (everyone has read the count)
+        if (rank == 0 && tid == 0) s.n_few = 0;
+    }
+
     if (by_rank) {
         uint32_t prefix = 0, mask = 0;
         int remaining = k, shift = 32;
@@ -482,18 +638,7 @@ filter_kernel(FilterParams p) {
                 if ((key & mask) == prefix) atomicAdd(&s.hist[(key >> shift) & (bins - 1)], 1);
             }
             gather_bins<int>(blocks, s, bins);
-            // from the top: the bin in which the remaining-th key lies
-            const int per = bins / THREADS, top = bins - 1 - tid * per;
-            int mine = 0;
-            for (int i = 0; i < per; i++) mine += s.total[top - i];
-            int before = block_exclusive_scan<int>(mine, s.warp_i, &s.total_i);
-            if (before < remaining && before + mine >= remaining) {
-                int i = 0;
-                while (before + s.total[top - i] < remaining) before += s.total[top - i++];
-                s.bin = top - i;
-                s.need = remaining - before;
-            }
-            __syncthreads();
+            find_bin(s, bins, remaining);      // from the top: the bin in which the remaining-th key lies
             prefix |= (uint32_t)s.bin << shift;
             mask |= (uint32_t)(bins - 1) << shift;
             remaining = s.need;
@@ -522,28 +667,9 @@ filter_kernel(FilterParams p) {
             else if (few && key > lowest) list[atomicAdd(n_few, 1)] = (unsigned long long)key << 32 | (uint32_t)~i;
         }
     }
-
     if (few) {
         blocks.sync();
-        if (rank != 0) return;
-        // ranks by key, ties by index; the mass before an entry is then a scan
-        const int n = s.n_few;
-        const unsigned long long mine = tid < n ? s.few[tid] : 0ull;
-        int place = 0;
-        for (int j = 0; j < n; j++) place += s.few[j] > mine;
-        if (tid < n) {
-            const int i = (int)~(uint32_t)mine;
-            s.sorted[place] = x[i] * inv_t;
-            s.at[place] = i;
-        }
-        __syncthreads();
-        if (n == 0) return;
-        const float v = tid < n ? s.sorted[tid] : -INFINITY;
-        const float mx = block_max(v, s.scratch);
-        const float pr = v == -INFINITY ? 0.f : expf(v - mx);
-        const float before = block_exclusive_scan<float>(pr, s.warp_f, &s.total_f);
-        const float limit = top_p * s.total_f;      // a share of the mass from before min-p (Sampling.cs:272-274)
-        if (tid < n && ((min_p > 0.f && pr < min_p) || (top_p < 1.f && before >= limit))) x[s.at[tid]] = -INFINITY;
+        if (rank == 0) settle_few(s, p, row, srow, x, inv_t, s.n_few, k, top_p, min_p);
         return;
     }
 
@@ -691,21 +817,22 @@ HYMT2_API int hymt2_record_history(int* history, int* counts, int stride, const 
     return hymt2_check_launch("record_history");
 }
 
+// `drawn` (or null): rows that hymt2_filter_logits drew, which are passed over.
 // piece_val / piece_idx: scratch of rows * ceil(vocab / 4096) entries each, or null.  With scratch
 // and a vocabulary above 2 * 4096 the scan is spread over many blocks per row.
 HYMT2_API int hymt2_argmax(int* out, const float* logits, long row_stride, int rows, int vocab,
-                           const int* row_map, float* piece_val, int* piece_idx, cudaStream_t stream) {
+                           const int* row_map, float* piece_val, int* piece_idx, const int* drawn, cudaStream_t stream) {
     if (rows == 0) return HYMT2_OK;
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "argmax: bad sizes rows=%d vocab=%d", rows, vocab);
     if (piece_val && piece_idx && vocab > 2 * ARGMAX_PIECE && rows <= 65535) {
         const int pieces = (vocab + ARGMAX_PIECE - 1) / ARGMAX_PIECE;
-        launch_pdl(argmax_pieces_kernel, dim3(pieces, rows), dim3(256), 0, stream, piece_val, piece_idx, logits, row_stride, vocab, row_map);
+        launch_pdl(argmax_pieces_kernel, dim3(pieces, rows), dim3(256), 0, stream, piece_val, piece_idx, logits, row_stride, vocab, row_map, drawn);
         int rc = hymt2_check_launch("argmax (pieces)");
         if (rc != HYMT2_OK) return rc;
-        launch_pdl(argmax_final_kernel, dim3(rows), dim3(32), 0, stream, out, (const float*)piece_val, (const int*)piece_idx, pieces, row_map);
+        launch_pdl(argmax_final_kernel, dim3(rows), dim3(32), 0, stream, out, (const float*)piece_val, (const int*)piece_idx, pieces, row_map, drawn);
         return hymt2_check_launch("argmax (final)");
     }
-    argmax_kernel<<<rows, THREADS, 0, stream>>>(out, logits, row_stride, vocab, row_map);
+    argmax_kernel<<<rows, THREADS, 0, stream>>>(out, logits, row_stride, vocab, row_map, drawn);
     return hymt2_check_launch("argmax");
 }
 
@@ -738,7 +865,7 @@ HYMT2_API int hymt2_filter_blocks(int rows, int vocab) {
 }
 
 HYMT2_API int hymt2_sample(int* out, const float* logits, long row_stride, int rows, int vocab,
-                           const float* inv_temperature, uint64_t* rng_states, const int* row_map,
+                           const float* inv_temperature, uint64_t* rng_states, const int* row_map, const int* drawn,
                            cudaStream_t stream) {
     if (rows == 0) return HYMT2_OK;
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "sample: bad sizes rows=%d vocab=%d", rows, vocab);
@@ -747,22 +874,25 @@ HYMT2_API int hymt2_sample(int* out, const float* logits, long row_stride, int r
         cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SHARED);
         if (e != cudaSuccess) { hymt2_set_error("sample: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
         launch_clusters(sample_cluster_kernel, rows, sample_shared(vocab), stream, out, logits, row_stride, vocab, inv_temperature, rng_states,
-                        row_map);
+                        row_map, drawn);
         return hymt2_check_launch("sample");
     }
     sample_kernel<<<rows, THREADS, 0, stream>>>(out, logits, row_stride, vocab, inv_temperature, rng_states,
-                                                row_map);
+                                                row_map, drawn);
     return hymt2_check_launch("sample");
 }
 
+// `drawn` (or null) [rows]: rows left with few entries draw their token at once, into out[row] with the sequence's stream, and say so
+// there; argmax and sample, given the same `drawn`, pass over such rows.
 HYMT2_API int hymt2_filter_logits(float* logits, long row_stride, int rows, int vocab, const float* inv_temperature,
                                   const int* top_k, const float* top_p, const float* min_p, const float* penalty,
-                                  const int* history, int history_stride, const int* row_map,
-                                  cudaStream_t stream) {
+                                  const int* history, int history_stride, const int* row_map, int* out, uint64_t* rng_states,
+                                  int* drawn, cudaStream_t stream) {
     if (rows == 0) return HYMT2_OK;
     HYMT2_REQUIRE(rows > 0 && vocab > 0 && row_stride >= vocab, "filter: bad sizes rows=%d vocab=%d", rows, vocab);
     FilterParams p{logits, row_stride, vocab, inv_temperature, top_k, top_p, min_p, penalty, history,
-                   history_stride, row_map};
+                   history_stride, row_map, out, rng_states, drawn};
+    HYMT2_REQUIRE(!drawn || (out && rng_states), "filter: a draw needs the tokens' place and the random streams");
     if (hymt2_filter_blocks(rows, vocab) == CLUSTER) launch_clusters(filter_kernel<CLUSTER>, rows, 0, stream, p);
     else launch_pdl(filter_kernel<1>, dim3(rows), dim3(THREADS), 0, stream, p);
     return hymt2_check_launch("filter_logits");

@@ -889,8 +889,8 @@ ARGMAX_PIECE = 4096
 
 
 def argmax(out: torch.Tensor, logits: torch.Tensor, row_map: torch.Tensor | None = None,
-           scratch: tuple | None = None) -> None:
-    """out[r] = first index of the maximum of logits[r]; rows with row_map[r] < 0 are skipped.
+           scratch: tuple | None = None, drawn: torch.Tensor | None = None) -> None:
+    """out[r] = first index of the maximum of logits[r]; rows with row_map[r] < 0 are skipped, and rows that filter_logits has drawn (`drawn`).
     `scratch` = (float32, int32) tensors of rows * ceil(vocab / 4096) entries lets a wide
     vocabulary be scanned by many blocks per row."""
     _need(out, "out", torch.int32, 1)
@@ -898,14 +898,14 @@ def argmax(out: torch.Tensor, logits: torch.Tensor, row_map: torch.Tensor | None
     rows, vocab = logits.shape
     val = idx = None
     if scratch is not None:
-        val, idx = scratch
+        val, idx = scratch[:2]
         need = rows * (-(-vocab // ARGMAX_PIECE))
         _need(val, "scratch values", torch.float32); _need(idx, "scratch indices", torch.int32)
         if val.numel() < need or idx.numel() < need:
             raise KernelError("argmax: the scratch is too small")
     two_stage = scratch is not None and vocab > 2 * ARGMAX_PIECE
     _check(_lib().hymt2_argmax(_ptr(out), _ptr(logits), c_long(logits.stride(0)), c_int(rows), c_int(vocab),
-                               _ptr(row_map), _ptr(val), _ptr(idx), _stream()), "argmax", 2 if two_stage else 1)
+                               _ptr(row_map), _ptr(val), _ptr(idx), _ptr(drawn), _stream()), "argmax", 2 if two_stage else 1)
 
 
 def seed_rng(states: torch.Tensor, rows: torch.Tensor, seeds: torch.Tensor) -> None:
@@ -915,16 +915,17 @@ def seed_rng(states: torch.Tensor, rows: torch.Tensor, seeds: torch.Tensor) -> N
 
 
 def sample(out: torch.Tensor, logits: torch.Tensor, inv_temperature: torch.Tensor, rng_states: torch.Tensor,
-           row_map: torch.Tensor | None = None) -> None:
+           row_map: torch.Tensor | None = None, drawn: torch.Tensor | None = None) -> None:
     """Temperature sampling of one token for every logits row whose sequence has a temperature
     above 0; advances that sequence's random stream by one draw.  row_map[r] is the row of the
-    per-sequence arrays (inv_temperature, rng_states) that logits row r belongs to; < 0 skips."""
+    per-sequence arrays (inv_temperature, rng_states) that logits row r belongs to; < 0 skips.  Rows that filter_logits has drawn
+    (`drawn`) are passed over."""
     _need(out, "out", torch.int32, 1); _need(inv_temperature, "inv_temperature", torch.float32, 1)
     _need(rng_states, "rng_states", torch.int64, 2)
     _logits_ok(logits, "sample")
     rows, vocab = logits.shape
     _check(_lib().hymt2_sample(_ptr(out), _ptr(logits), c_long(logits.stride(0)), c_int(rows), c_int(vocab),
-                               _ptr(inv_temperature), _ptr(rng_states), _ptr(row_map), _stream()), "sample")
+                               _ptr(inv_temperature), _ptr(rng_states), _ptr(row_map), _ptr(drawn), _stream()), "sample")
 
 
 def sample_blocks(rows: int, vocab: int) -> int:
@@ -939,18 +940,24 @@ def filter_blocks(rows: int, vocab: int) -> int:
 
 def filter_logits(logits: torch.Tensor, inv_temperature: torch.Tensor, top_k: torch.Tensor | None,
                   top_p: torch.Tensor | None, min_p: torch.Tensor | None, penalty: torch.Tensor | None,
-                  history: torch.Tensor | None, row_map: torch.Tensor | None = None) -> None:
+                  history: torch.Tensor | None, row_map: torch.Tensor | None = None, draw: tuple | None = None) -> None:
     """In place: repetition penalty, then (temperature > 0 only) top-k / min-p / top-p drops;
-    dropped entries become -inf."""
+    dropped entries become -inf.  `draw` = (out [rows] int32, rng_states, drawn [rows] int32): a row whose top-k left few entries draws
+    its token at once, as `sample` would, into out, and says so in drawn (1, else 0), which argmax and sample then want."""
     _logits_ok(logits, "filter")
     rows, vocab = logits.shape
     hs = 0
     if history is not None:
         _need(history, "history", torch.int32, 2)
         hs = history.shape[1]
+    out, rng, drawn = draw or (None, None, None)
+    if draw is not None:
+        _need(out, "out", torch.int32, 1); _need(rng, "rng_states", torch.int64, 2); _need(drawn, "drawn", torch.int32, 1)
+        if out.shape[0] < rows or drawn.shape[0] < rows:
+            raise KernelError("filter: a draw needs a place for every row's token")
     _check(_lib().hymt2_filter_logits(_ptr(logits), c_long(logits.stride(0)), c_int(rows), c_int(vocab),
                                       _ptr(inv_temperature), _ptr(top_k), _ptr(top_p), _ptr(min_p), _ptr(penalty),
-                                      _ptr(history), c_int(hs), _ptr(row_map), _stream()), "filter_logits")
+                                      _ptr(history), c_int(hs), _ptr(row_map), _ptr(out), _ptr(rng), _ptr(drawn), _stream()), "filter_logits")
 
 
 def record_history(history: torch.Tensor, counts: torch.Tensor, tokens: torch.Tensor,

@@ -67,12 +67,15 @@ class BatchSampler:
         rows = logits.shape[0]
         if out is None:
             out = torch.empty(rows, dtype=torch.int32, device=self.device)
+        scratch, drawn = self.ensure_argmax_scratch(rows, logits.shape[1]), None
         if self.any_filter:
+            draw = None if self.all_greedy else (out, self.rng, scratch[2])
+            drawn = None if draw is None else draw[2]          # the rows whose token the filters draw on the way
             ops.filter_logits(logits, self.inv_temperature, self.top_k, self.top_p, self.min_p, self.penalty,
-                              self.history, row_map)
-        ops.argmax(out, logits, row_map, self.ensure_argmax_scratch(rows, logits.shape[1]))
+                              self.history, row_map, draw)
+        ops.argmax(out, logits, row_map, scratch, drawn)
         if not self.all_greedy:
-            ops.sample(out, logits, self.inv_temperature, self.rng, row_map)
+            ops.sample(out, logits, self.inv_temperature, self.rng, row_map, drawn)
         if self.any_filter and self.history is not None:
             ops.record_history(self.history, self.counts, out, row_map, rows)
         return out
@@ -100,9 +103,10 @@ class BatchSampler:
 
     def ensure_argmax_scratch(self, rows: int, vocab: int):
         need = rows * (-(-vocab // ops.ARGMAX_PIECE))
-        if self._argmax_scratch is None or self._argmax_scratch[0].numel() < need:
+        if self._argmax_scratch is None or self._argmax_scratch[0].numel() < need or self._argmax_scratch[2].numel() < rows:
             self._argmax_scratch = (torch.empty(need, dtype=torch.float32, device=self.device),
-                                    torch.empty(need, dtype=torch.int32, device=self.device))
+                                    torch.empty(need, dtype=torch.int32, device=self.device),
+                                    torch.empty(rows, dtype=torch.int32, device=self.device))      # rows that the filters drew
         return self._argmax_scratch
 
     def snapshot(self):
