@@ -42,6 +42,8 @@ __host__ __device__ constexpr int tile_issuers(int bn, int epi) {
 }
 __host__ __device__ constexpr int tile_threads(int bn, int epi) { return tile_issuers(bn, epi) > 1 ? 224 : 192; }
 constexpr int A_TILE_BYTES = TILE_M * BLOCK_K * 2;
+// cycles of a k block of a pair's tile (fixed, and a column), of the start of a grid of pairs, and of a product from which on pairs are asked at all
+constexpr double PAIR_FIXED = 251.0, PAIR_COLUMN = 2.0, PAIR_START = 4500.0, PAIR_LEAST = 140e3;
 constexpr int PERSISTENT_BN = 256;   // tile width of the persistent kernel for many tokens
 
 // EPI_GLU is EPI_SWIGLU with another rule than silu(gate) * up, or with biases: an instance of its own, so that the plain one keeps
@@ -201,6 +203,81 @@ __device__ __forceinline__ bool umma_block_looking_ahead(uint32_t tmem_d, uint64
         : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_bar), "r"(next_parity)
         : "memory");
     return seen != 0;
+}
+// ---- the same for a pair of CTAs (cta_group::2): the even CTA's barriers, and MMAs that both SMs work on ------------------------
+constexpr uint32_t EVEN_CTA = 0xFEFFFFFFu;      // an address of this CTA's shared memory, turned to the pair's even CTA
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t even_bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"((uint64_t)map), "r"(even_bar), "r"(x), "r"(y) : "memory");
+}
+// tma_stage_looking_ahead of one CTA of a pair: its rows of both operands, of one or two k blocks (`two`; the second `a2`, `b2` bytes behind the
+// first), counted at the even CTA's barrier, which the even CTA arms with both CTAs' bytes (`arm`).
+__device__ __forceinline__ bool tma_pair_stage_looking_ahead(uint32_t bar, uint32_t arm, uint32_t bytes, uint32_t a_dst, const CUtensorMap* map_a, int x,
+                                                             int ay, uint32_t b_dst, const CUtensorMap* map_b, int by, uint32_t b2, uint32_t two,
+                                                             uint32_t next_bar, uint32_t next_parity) {
+    uint32_t seen;
+    asm volatile(
+        "{\n\t.reg .pred look, even, second;\n\t.reg .b32 x2, a2, b2;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 look, [%10], %11;\n\t"
+        "setp.ne.b32 even, %2, 0;\n\t"
+        "setp.ne.b32 second, %14, 0;\n\t"
+        "add.u32 x2, %6, 64;\n\tadd.u32 a2, %4, 16384;\n\tadd.u32 b2, %7, %15;\n\t"
+        "@even mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %3;\n\t"
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%7], [%8, {%6, %9}], [%12];\n\t"
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%4], [%5, {%6, %13}], [%12];\n\t"
+        "@second cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [b2], [%8, {x2, %9}], [%12];\n\t"
+        "@second cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [a2], [%5, {x2, %13}], [%12];\n\t"
+        "selp.u32 %0, 1, 0, look;\n\t}"
+        : "=r"(seen)
+        : "r"(bar), "r"(arm), "r"(bytes), "r"(a_dst), "l"((uint64_t)map_a), "r"(x), "r"(b_dst), "l"((uint64_t)map_b), "r"(by), "r"(next_bar),
+          "r"(next_parity), "r"(bar & EVEN_CTA), "r"(ay), "r"(two), "r"(b2)
+        : "memory");
+    static_assert(A_TILE_BYTES == 16384, "the second k block's activations lie behind the first's");
+    return seen != 0;
+}
+// umma_block_looking_ahead for the pair, of one or two k blocks (`two`; descriptors of the second `a2`, `b2` units behind the first); the stage is
+// given back to both CTAs.
+__device__ __forceinline__ bool umma_pair_blocks_looking_ahead(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                               uint64_t a2, uint64_t b2, uint32_t two, uint32_t empty_bar, uint32_t next_bar,
+                                                               uint32_t next_parity) {
+    uint32_t seen;
+    asm volatile(
+        "{\n\t.reg .pred look, first, yes, second;\n\t.reg .b64 a, b, c, d;\n\t.reg .b16 both;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 look, [%7], %8;\n\t"
+        "setp.ne.b32 first, %5, 0;\n\t"
+        "setp.ne.b32 second, %11, 0;\n\t"
+        "setp.eq.u32 yes, 1, 1;\n\t"
+        "mov.b16 both, 3;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %4, first;\n\t"
+        "add.u64 a, %2, 2;\n\tadd.u64 b, %3, 2;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "add.u64 a, %2, 4;\n\tadd.u64 b, %3, 4;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "add.u64 a, %2, 6;\n\tadd.u64 b, %3, 6;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "add.u64 c, %2, %9;\n\tadd.u64 d, %3, %10;\n\t"
+        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], c, d, %4, yes;\n\t"
+        "add.u64 a, c, 2;\n\tadd.u64 b, d, 2;\n\t"
+        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "add.u64 a, c, 4;\n\tadd.u64 b, d, 4;\n\t"
+        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "add.u64 a, c, 6;\n\tadd.u64 b, d, 6;\n\t"
+        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], both;\n\t"
+        "selp.u32 %0, 1, 0, look;\n\t}"
+        : "=r"(seen)
+        : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_bar), "r"(next_parity), "l"(a2), "l"(b2), "r"(two)
+        : "memory");
+    return seen != 0;
+}
+__device__ __forceinline__ void mbar_arrive_even(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar & EVEN_CTA) : "memory");
+}
+__device__ __forceinline__ void umma_pair_commit(uint32_t bar) {      // the barrier at this place in both CTAs
+    asm volatile(
+        "{\n\t.reg .b16 both;\n\tmov.b16 both, 3;\n\t"
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n\t}" ::"r"(bar) : "memory");
 }
 template <int N>
 __device__ __forceinline__ void tmem_load(uint32_t taddr, float* v);
@@ -864,18 +941,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // runs on across tiles, and two accumulators in tensor memory alternate: while the epilogue
 // warps drain one, the MMA thread already fills the other with the next tile.
 // --------------------------------------------------------------------------------------------
-template <int BN, int EPI, typename TC>
+template <int BN, int EPI, typename TC, bool PAIR>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmTcParams p) {
     // BN is the widest tile (the accumulators lie BN columns apart); the width in use comes with the launch, chosen so
     // that the tiles fill whole waves of SMs
     constexpr bool SPLIT_B = is_gated(EPI);
     const int bn = p.bn;
-    const int B_TILE_BYTES = bn * BLOCK_K * 2;
-    const int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
+    const int B_TILE_BYTES = bn * BLOCK_K * (PAIR ? 1 : 2);     // (a CTA of a pair holds half of the tile's weight rows)
+    // A look at a barrier takes the issuing threads some 500 cycles whatever hides in front of it, as long as a pair's MMAs of a k block:
+    // a pair's stage holds two k blocks.
+    constexpr int BLOCKS = PAIR ? 2 : 1;
+    const int STAGE_BYTES = BLOCKS * (A_TILE_BYTES + B_TILE_BYTES);
     constexpr int TMEM_COLS = 2 * BN;                       // 256 or 512
+    constexpr int CTAS = PAIR ? 2 : 1, TILE_ROWS = CTAS * TILE_M;
     const int OUT_COLS = SPLIT_B ? bn / 2 : bn;
-    const uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
+    const uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TILE_ROWS >> 4) << 24);
+    const int unit = blockIdx.x / CTAS, units = gridDim.x / CTAS;      // what walks tiles: a CTA or a pair
+    const int rank = blockIdx.x % CTAS;                                // the CTA's place in its pair
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4];
@@ -889,9 +972,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     const uint32_t acc_full0 = smem_u32(&bars[2 * MAX_STAGES]), acc_empty0 = acc_full0 + 16;
     volatile int* abort_flag = &abort_s;
     const int num_k_blocks = (p.K + BLOCK_K - 1) / BLOCK_K;
-    int tiles_m = (p.T + TILE_M - 1) / TILE_M;
+    int tiles_m = (p.T + TILE_ROWS - 1) / TILE_ROWS;
     const int tiles_n = (p.N + OUT_COLS - 1) / OUT_COLS;
-    if (p.tile_group) {
+    if (!PAIR && p.tile_group) {
         // a grouped product: the row tiles in use come first, and their number stands behind the last tile's entry (written by
         // the kernel before, so every role waits for it here)
         pdl_wait();
@@ -907,17 +990,23 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(acc_full0 + 8 * b, 1);
-            mbar_init(acc_empty0 + 8 * b, 128);
+            mbar_init(acc_empty0 + 8 * b, PAIR ? 8 : 128);      // threads, or warps of both CTAs
         }
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync_all();       // both CTAs' barriers and tensor memory are there
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
 
@@ -927,31 +1016,49 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         // were issued (the stages of the first round are free anyway).
         uint32_t s = 0, round = 0;
         bool first = true, looked = true;
-        if (p.tile_group) pdl_wait();   // which weights a tile meets was written by the kernel before
-        for (int tile = blockIdx.x; tile < num_tiles && !*abort_flag; tile += gridDim.x) {
-            const int a_row0 = (tile % tiles_m) * TILE_M;
+        if (!PAIR && p.tile_group) pdl_wait();   // which weights a tile meets was written by the kernel before
+        for (int tile = unit; tile < num_tiles && !*abort_flag; tile += units) {
+            const int a_row0 = (tile % tiles_m) * TILE_ROWS + rank * TILE_M;
             int b_row0 = (tile / tiles_m) * OUT_COLS;
-            if (p.tile_group) {
+            if (!PAIR && p.tile_group) {
                 const int group = p.tile_group[tile % tiles_m];
                 b_row0 += (int)((group > 0 ? group : 0) * p.group_rows);
             }
-            for (int kb = 0; kb < num_k_blocks; kb++) {
+            // (a pair's tile: the even CTA brings the first half of the weight rows, the odd one the second; of gated rows the gates and the ups)
+            if (PAIR) b_row0 += rank * (SPLIT_B ? p.N : bn / 2);
+            for (int kb = 0; kb < num_k_blocks; kb += BLOCKS) {
                 if (round > 0 && !looked && !mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, abort_flag, p.status, 101)) break;
-                const uint32_t bar = full0 + 8 * s, a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + A_TILE_BYTES;
+                const uint32_t bar = full0 + 8 * s, a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + BLOCKS * A_TILE_BYTES;
+                const uint32_t two = PAIR && kb + 1 < num_k_blocks ? 1u : 0u;
+                const uint32_t pair_bytes = 2 * (1 + two) * (A_TILE_BYTES + B_TILE_BYTES);
                 const int k = kb * BLOCK_K;
                 const uint32_t s_next = s + 1 == (uint32_t)stages ? 0 : s + 1, round_next = s_next ? round : round + 1;
                 if (first) {
-                    mbar_expect_tx(bar, STAGE_BYTES);
-                    tma_load_2d(b_dst, &map_b, bar, k, b_row0);
-                    if (SPLIT_B) tma_load_2d(b_dst + B_TILE_BYTES / 2, &map_b, bar, k, p.N + b_row0);
-                    pdl_wait();   // the activations come from the kernel before
-                    tma_load_2d(a_dst, &map_a, bar, k, a_row0);
+                    if constexpr (PAIR) {
+                        if (rank == 0) mbar_expect_tx(bar, pair_bytes);
+                        tma_load_2d_pair(b_dst, &map_b, bar & EVEN_CTA, k, b_row0);
+                        if (two) tma_load_2d_pair(b_dst + B_TILE_BYTES, &map_b, bar & EVEN_CTA, k + BLOCK_K, b_row0);
+                        pdl_wait();
+                        tma_load_2d_pair(a_dst, &map_a, bar & EVEN_CTA, k, a_row0);
+                        if (two) tma_load_2d_pair(a_dst + A_TILE_BYTES, &map_a, bar & EVEN_CTA, k + BLOCK_K, a_row0);
+                    } else {
+                        mbar_expect_tx(bar, STAGE_BYTES);
+                        tma_load_2d(b_dst, &map_b, bar, k, b_row0);
+                        if (SPLIT_B) tma_load_2d(b_dst + B_TILE_BYTES / 2, &map_b, bar, k, p.N + b_row0);
+                        pdl_wait();   // the activations come from the kernel before
+                        tma_load_2d(a_dst, &map_a, bar, k, a_row0);
+                    }
                     first = false;
                     looked = round_next == 0;
                 } else {
-                    const bool seen = tma_stage_looking_ahead(bar, STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, k, b_row0,
-                                                              b_dst + B_TILE_BYTES / 2, p.N + b_row0, SPLIT_B ? 1u : 0u,
-                                                              empty0 + 8 * s_next, (round_next & 1) ^ 1);
+                    bool seen;
+                    if constexpr (PAIR)
+                        seen = tma_pair_stage_looking_ahead(bar, rank == 0 ? 1u : 0u, pair_bytes, a_dst, &map_a, k, a_row0, b_dst, &map_b, b_row0, B_TILE_BYTES, two,
+                                                            empty0 + 8 * s_next, (round_next & 1) ^ 1);
+                    else
+                        seen = tma_stage_looking_ahead(bar, STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, k, b_row0,
+                                                       b_dst + B_TILE_BYTES / 2, p.N + b_row0, SPLIT_B ? 1u : 0u,
+                                                       empty0 + 8 * s_next, (round_next & 1) ^ 1);
                     looked = round_next == 0 || seen;
                 }
                 s = s_next;
@@ -959,32 +1066,46 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
         }
         if (first) pdl_wait();
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer: the stage's descriptor is carried along, see gemm_tc_kernel --------------
+        if (rank == 0 && *abort_flag) {
+            // copies in flight (of a pair: both CTAs', counted here) must land before the shared memory goes away
+            for (int back = 0; back < stages && (round > 0 || s > 0); back++) {
+                if (s == 0) { s = stages; round--; }
+                s--;
+                for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(full0 + 8 * s, round & 1); t++) {}
+            }
+        }
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+        // ---- MMA issuer (of a pair: the even CTA's): the stage's descriptor is carried along, see gemm_tc_kernel --------------
         const uint64_t desc0 = desc_k_major(tiles);
         uint64_t adesc = desc0;
         uint32_t s = 0, phase = 0;
         bool looked = false;   // whether the stage's barrier was already seen complete
         int j = 0;
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, j++) {
+        for (int tile = unit; tile < num_tiles; tile += units, j++) {
             const int buf = j & 1;
             if (j >= 2 && !mbar_wait(acc_empty0 + 8 * buf, (uint32_t)((((j >> 1) - 1) & 1)), abort_flag, p.status, 104)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             bool ok = true;
             const uint32_t acc_at = tmem_base + buf * BN;
-            for (int kb = 0; kb < num_k_blocks; kb++) {
+            for (int kb = 0; kb < num_k_blocks; kb += BLOCKS) {
                 if (!looked && !(ok = mbar_wait(full0 + 8 * s, phase, abort_flag, p.status, 102))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t s_next = s + 1 == (uint32_t)stages ? 0 : s + 1, phase_next = s_next ? phase : phase ^ 1;
                 // a look at a stage that will never be filled (behind the last one) is thrown away by the loops' ends
-                looked = umma_block_looking_ahead(acc_at, adesc, adesc + (A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, empty0 + 8 * s,
-                                                  full0 + 8 * s_next, phase_next);
+                if constexpr (PAIR)
+                    looked = umma_pair_blocks_looking_ahead(acc_at, adesc, adesc + (2 * A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, A_TILE_BYTES >> 4,
+                                                            (uint64_t)(B_TILE_BYTES >> 4), kb + 1 < num_k_blocks ? 1u : 0u, empty0 + 8 * s,
+                                                            full0 + 8 * s_next, phase_next);
+                else
+                    looked = umma_block_looking_ahead(acc_at, adesc, adesc + (A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, empty0 + 8 * s,
+                                                      full0 + 8 * s_next, phase_next);
                 s = s_next;
                 phase = phase_next;
                 adesc = s ? adesc + (uint64_t)(STAGE_BYTES >> 4) : desc0;
             }
             if (!ok) break;
-            umma_commit(acc_full0 + 8 * buf);
+            if constexpr (PAIR) umma_pair_commit(acc_full0 + 8 * buf);
+            else umma_commit(acc_full0 + 8 * buf);
         }
     } else if (warp >= 2) {
         // ---- epilogue ---------------------------------------------------------------------------------
@@ -1003,7 +1124,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         // (The helper reads a barrier it has not followed.  When it gets there it has drained tile last - 1, whose
         // MMAs were issued after those of tile last - 2 were complete, so the barrier of the last tile's accumulator is in
         // the last tile's own phase or past it, never one behind: the parity cannot be taken for an older one.)
-        const int my_tiles = (int)blockIdx.x < num_tiles ? (num_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        const int my_tiles = unit < num_tiles ? (num_tiles - 1 - unit) / units + 1 : 0;
         const int last = my_tiles - 1;
         const int split_at = EPI == EPI_ROPE_KV ? (bn / TILE_M / 2) * TILE_M : ((OUT_COLS / 16 + 1) / 2) * 16;   // whole heads, whole chunks
         const bool can_share = split_at > 0 && split_at < OUT_COLS;
@@ -1017,9 +1138,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             } else if (my_tiles > 0 && can_share && (last & 1) != group && group + EPILOGUE_GROUPS * (item - 1) < my_tiles && !*abort_flag) {
                 j = last; own = false; c_begin = split_at;
             } else break;
-            const int tile = blockIdx.x + j * gridDim.x;
+            const int tile = unit + j * units;
             const int buf = j & 1;
-            const int a_row0 = (tile % tiles_m) * TILE_M, b_row0 = (tile / tiles_m) * OUT_COLS;
+            const int a_row0 = (tile % tiles_m) * TILE_ROWS + rank * TILE_M, b_row0 = (tile / tiles_m) * OUT_COLS;
             // (the threads of a warp leave the wait at different times; what follows reads tensor memory warp-wide, so the
             // warp comes together first, and gives up together)
             const int m = a_row0 + row;
@@ -1107,15 +1228,24 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
             if (!own) break;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(acc_empty0 + 8 * buf);   // this thread has taken its row out of the accumulator
+            // this thread (a pair's: this warp) has taken its row out of the accumulator
+            if constexpr (PAIR) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_even(acc_empty0 + 8 * buf);
+            } else mbar_arrive(acc_empty0 + 8 * buf);
         }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) {
+        __syncwarp();
+        cluster_sync_all();             // neither CTA leaves while the other may still arrive at its barriers
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -1261,32 +1391,101 @@ bool make_plan(int T, int N, int K, int epilogue, int sm_count, Plan* plan, bool
     return true;
 }
 
-template <int BN, int EPI, typename TC>
+// Pairs of CTAs (cta_group::2) on tiles of 256 tokens: a CTA holds its 128 tokens and half of the tile's weight rows, so a k block brings
+// 16 KB + bn / 2 rows into each SM's shared memory and the MMAs read as much, where a CTA by itself brings and reads all bn rows.  That
+// traffic is what bounds the kernel of single CTAs (96 KB a k block at bn = 256, 128 bytes a cycle: 750 of its 821 cycles, the tensor
+// core needs 512).
+struct PairPlan {
+    bool use;
+    int bn, stages, pairs;
+    size_t smem;
+};
+
+PairPlan plan_pairs(int T, int N, int K, int epilogue, const Plan& single) {
+    PairPlan pp{};
+    if (!single.persistent || single.sm_count < 2) return pp;
+    const int k_blocks = (K + BLOCK_K - 1) / BLOCK_K, pairs = single.sm_count / 2;
+    // costs in cycles as in make_plan: waves of tiles, and the epilogue behind the last one
+    const double epilogue_cycles = epilogue == EPI_ROPE_KV ? 60.0 : epilogue == EPI_ACCUMULATE ? 30.0 : 15.0;
+    const long single_tiles = (long)single.grid.x * single.grid.y;
+    const double alone = (double)((single_tiles + single.sm_count - 1) / single.sm_count) * k_blocks * (350.0 + 1.84 * single.bn) + epilogue_cycles * single.bn;
+    const int step = epilogue == EPI_ROPE_KV ? TILE_M : 32;       // an MMA of a pair takes widths in steps of 32
+    double best = 0;
+    for (int bn = PERSISTENT_BN; bn >= 128; bn -= step) {
+        const int out = epilogue == EPI_SWIGLU ? bn / 2 : bn;
+        const long tiles = (long)((T + 2 * TILE_M - 1) / (2 * TILE_M)) * ((N + out - 1) / out);
+        const double cost = (double)((tiles + pairs - 1) / pairs) * k_blocks * (PAIR_FIXED + PAIR_COLUMN * bn) + epilogue_cycles * bn;
+        if (bn == PERSISTENT_BN || cost < best) {
+            best = cost;
+            pp.bn = bn;
+            pp.pairs = (int)(tiles < pairs ? tiles : pairs);
+        }
+    }
+    pp.use = alone >= PAIR_LEAST && best + PAIR_START < alone;
+    const int stage = 2 * (A_TILE_BYTES + pp.bn * BLOCK_K);         // two k blocks
+    pp.stages = 224 * 1024 / stage > MAX_STAGES ? MAX_STAGES : 224 * 1024 / stage;
+    pp.smem = (size_t)pp.stages * stage + 1024;
+    return pp;
+}
+
+template <int EPI, typename TC, bool PAIR>
 int launch_persistent_one(const CUtensorMap& ma, const CUtensorMap& mb, const GemmTcParams& p, int ctas, size_t smem,
                           cudaStream_t stream) {
-    auto kernel = gemm_tc_persistent_kernel<BN, EPI, TC>;
+    auto kernel = gemm_tc_persistent_kernel<PERSISTENT_BN, EPI, TC, PAIR>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         if (e != cudaSuccess) { hymt2_set_error("gemm_tc: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
         configured = true;
     }
-    cudaError_t e = launch_pdl(kernel, dim3(ctas), dim3(NUM_THREADS), smem, stream, ma, mb, p);
+    cudaError_t e;
+    if constexpr (PAIR) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(NUM_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = hymt2_pdl_enabled() ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
+    } else {
+        e = launch_pdl(kernel, dim3(ctas), dim3(NUM_THREADS), smem, stream, ma, mb, p);
+    }
     if (e != cudaSuccess) { hymt2_set_error("gemm_tc: %s", cudaGetErrorString(e)); return HYMT2_ERR_LAUNCH; }
     return hymt2_check_launch("gemm_tc (persistent)");
 }
 
-int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmTcParams& p, const Plan& pl, int epilogue,
+template <bool PAIR>
+int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmTcParams& p, int ctas, size_t smem, int epilogue,
                       int c_dtype, cudaStream_t stream) {
-    const int ctas = pl.tiles < pl.sm_count ? pl.tiles : pl.sm_count;
-    if (epilogue == EPI_STORE && c_dtype == HYMT2_BF16) return launch_persistent_one<PERSISTENT_BN, EPI_STORE, __nv_bfloat16>(ma, mb, p, ctas, pl.smem, stream);
-    if (epilogue == EPI_STORE && c_dtype == HYMT2_F32) return launch_persistent_one<PERSISTENT_BN, EPI_STORE, float>(ma, mb, p, ctas, pl.smem, stream);
-    if (epilogue == EPI_ACCUMULATE && c_dtype == HYMT2_F32) return launch_persistent_one<PERSISTENT_BN, EPI_ACCUMULATE, float>(ma, mb, p, ctas, pl.smem, stream);
-    if (epilogue == EPI_SWIGLU && c_dtype == HYMT2_BF16 && !plain_rule(p.glu)) return launch_persistent_one<PERSISTENT_BN, EPI_GLU, __nv_bfloat16>(ma, mb, p, ctas, pl.smem, stream);
-    if (epilogue == EPI_SWIGLU && c_dtype == HYMT2_BF16) return launch_persistent_one<PERSISTENT_BN, EPI_SWIGLU, __nv_bfloat16>(ma, mb, p, ctas, pl.smem, stream);
+    if (epilogue == EPI_ROPE_KV) return launch_persistent_one<EPI_ROPE_KV, __nv_bfloat16, PAIR>(ma, mb, p, ctas, smem, stream);
+    if (epilogue == EPI_STORE && c_dtype == HYMT2_BF16) return launch_persistent_one<EPI_STORE, __nv_bfloat16, PAIR>(ma, mb, p, ctas, smem, stream);
+    if (epilogue == EPI_STORE && c_dtype == HYMT2_F32) return launch_persistent_one<EPI_STORE, float, PAIR>(ma, mb, p, ctas, smem, stream);
+    if (epilogue == EPI_ACCUMULATE && c_dtype == HYMT2_F32) return launch_persistent_one<EPI_ACCUMULATE, float, PAIR>(ma, mb, p, ctas, smem, stream);
+    if (epilogue == EPI_SWIGLU && c_dtype == HYMT2_BF16 && !plain_rule(p.glu)) return launch_persistent_one<EPI_GLU, __nv_bfloat16, PAIR>(ma, mb, p, ctas, smem, stream);
+    if (epilogue == EPI_SWIGLU && c_dtype == HYMT2_BF16) return launch_persistent_one<EPI_SWIGLU, __nv_bfloat16, PAIR>(ma, mb, p, ctas, smem, stream);
     hymt2_set_error("gemm_tc: epilogue %d with output type %d is not built", epilogue, c_dtype);
     return HYMT2_ERR_ARGUMENT;
 }
+
+// The product by pairs of CTAs; `p` as for the kernel of single ones.
+int launch_pairs(const CUtensorMap& ma, const void* W, long w_rows, long ldw, GemmTcParams p, const PairPlan& pp, int epilogue, int c_dtype,
+                 cudaStream_t stream) {
+    CUtensorMap mb;
+    HYMT2_REQUIRE(make_map(&mb, W, w_rows, p.K, ldw, pp.bn / 2), "gemm_tc: cuTensorMapEncodeTiled refused the operands");
+    p.bn = pp.bn;
+    p.stages = pp.stages;
+    return launch_persistent<true>(ma, mb, p, 2 * pp.pairs, pp.smem, epilogue, c_dtype, stream);
+}
+
+inline int single_ctas(const Plan& pl) { return pl.tiles < pl.sm_count ? pl.tiles : pl.sm_count; }
 
 int sm_count_of_current_device() {
     static int cached[64] = {};
@@ -1333,6 +1532,18 @@ HYMT2_API int hymt2_gemm_tc_describe(int T, int N, int K, int epilogue, int sm_c
     out[5] = pl.cluster ? 1 : 0;
     out[6] = pl.tiles;
     out[7] = pl.persistent ? (pl.tiles < pl.sm_count ? pl.tiles : pl.sm_count) : (int)(pl.grid.x * pl.grid.y * pl.grid.z);
+    return HYMT2_OK;
+}
+
+// Whether pairs of CTAs run a product that hymt2_gemm_tc_describe says is the persistent kernel's (what it says of widths and CTAs is then
+// what single CTAs would do): out[0] whether, [1] the tile's width (of 256 tokens), [2] stages of the ring, [3] pairs.
+HYMT2_API int hymt2_gemm_tc_describe_pairs(int T, int N, int K, int epilogue, int sm_count, int* out) {
+    HYMT2_REQUIRE(T > 0 && N > 0 && K > 0 && epilogue >= 0 && epilogue <= 3 && out, "gemm_tc_describe_pairs: bad arguments");
+    Plan pl;
+    make_plan(T, N, K, epilogue, sm_count > 0 ? sm_count : sm_count_of_current_device(), &pl);
+    const PairPlan pp = plan_pairs(T, N, K, epilogue, pl);
+    out[0] = pp.use ? 1 : 0;
+    out[1] = pp.bn; out[2] = pp.stages; out[3] = pp.pairs;
     return HYMT2_OK;
 }
 
@@ -1393,7 +1604,9 @@ int run_gemm_tc(void* C, int c_dtype, const void* X, const void* W, int T, int N
             default: return dispatch_epilogue<128>(ma, mb, p, pl.grid, pl.smem, epilogue, c_dtype, stream);
         }
     }
-    return launch_persistent(ma, mb, p, pl, epilogue, c_dtype, stream);
+    const PairPlan pp = plan_pairs(T, N, K, epilogue, pl);
+    if (pp.use) return launch_pairs(ma, W, w_rows, ldw, p, pp, epilogue, c_dtype, stream);
+    return launch_persistent<false>(ma, mb, p, single_ctas(pl), pl.smem, epilogue, c_dtype, stream);
 }
 }  // namespace
 
@@ -1432,7 +1645,7 @@ HYMT2_API int hymt2_gemm_tc_grouped(void* C, int c_dtype, const void* X, const v
     p.group_rows = rows_w;
     p.act = act == 1 ? 1 : 0;
     p.glu = GluRule{glu_kind, glu_limit, glu_alpha, nullptr};
-    return launch_persistent(ma, mb, p, pl, epi, c_dtype, stream);
+    return launch_persistent<false>(ma, mb, p, single_ctas(pl), pl.smem, epi, c_dtype, stream);
 }
 
 // hymt2_gemm_tc with an RMSNorm folded in (see NormSide).  As a consumer (ss_in): the activations X are bf16(x * gain) and the sums
@@ -1524,8 +1737,9 @@ HYMT2_API int hymt2_gemm_tc_rope_kv(const void* X, const void* W, int T, int K, 
     GemmTcParams p{nullptr, 0, T, N, K, pl.stages, pl.bn, pl.splits, pl.k_blocks_per_split, pl.cluster ? 1 : 0, nullptr, nullptr, status, rope,
                    WAIT_LIMIT, -1, NormSide{nullptr, nullptr, 0, nullptr, 0, ss_in, ss_in_tiles, ss_width, ss_eps}};
     if (pl.persistent) {
-        const int ctas = pl.tiles < pl.sm_count ? pl.tiles : pl.sm_count;
-        return launch_persistent_one<PERSISTENT_BN, EPI_ROPE_KV, __nv_bfloat16>(ma, mb, p, ctas, pl.smem, stream);
+        const PairPlan pp = plan_pairs(T, N, K, EPI_ROPE_KV, pl);
+        if (pp.use) return launch_pairs(ma, W, N, ldw, p, pp, EPI_ROPE_KV, HYMT2_BF16, stream);
+        return launch_persistent<false>(ma, mb, p, single_ctas(pl), pl.smem, EPI_ROPE_KV, HYMT2_BF16, stream);
     }
     switch (pl.bn) {
         case 16: return launch<16, EPI_ROPE_KV, __nv_bfloat16>(ma, mb, p, pl.grid, pl.smem, stream);

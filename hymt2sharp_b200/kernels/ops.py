@@ -646,8 +646,8 @@ def gemm_tc_rope_kv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pla
 
 
 def gemm_tc_describe(tokens: int, out_features: int, inner: int, epilogue: int, sm_count: int = 0) -> dict:
-    """How the tensor-core kernel would run this product (nothing is launched; works without a GPU when sm_count
-    is given): orientation, kernel, tile width, ring depth, splits of K and how they fold, tiles and CTAs.
+    """How the tensor-core kernel would run this product on single CTAs (what gemm_tc_pairs says goes first; nothing is
+    launched; works without a GPU when sm_count is given): orientation, kernel, tile width, ring depth, splits of K and how they fold, tiles and CTAs.
     epilogue: EPILOGUE_STORE / _ACCUMULATE / _SWIGLU, or 3 for the q/k/v projection with rotation."""
     out = (ctypes.c_int * 8)()
     rc = _lib().hymt2_gemm_tc_describe(c_int(tokens), c_int(out_features), c_int(inner), c_int(epilogue), c_int(sm_count), out)
@@ -655,6 +655,14 @@ def gemm_tc_describe(tokens: int, out_features: int, inner: int, epilogue: int, 
         raise KernelError(f"gemm_tc_describe failed ({rc}): {_lib().hymt2_last_error().decode(errors='replace')}")
     keys = ("swapped", "persistent", "tile_width", "stages", "k_splits", "cluster", "tiles", "ctas")
     return {k: (bool(v) if k in ("swapped", "persistent", "cluster") else int(v)) for k, v in zip(keys, out)}
+
+
+def gemm_tc_pairs(tokens: int, out_features: int, inner: int, epilogue: int, sm_count: int = 0) -> dict:
+    """Whether pairs of CTAs run a product of more than 128 tokens (`pairs` of them, 0: single CTAs do, as gemm_tc_describe says), the
+    width of their tiles of 256 tokens and the stages of their ring.  Nothing is launched; works without a GPU when sm_count is given."""
+    out = (ctypes.c_int * 4)()
+    _check(_lib().hymt2_gemm_tc_describe_pairs(c_int(tokens), c_int(out_features), c_int(inner), c_int(epilogue), c_int(sm_count), out), "gemm_tc_describe_pairs", 0)
+    return {"pairs": int(out[3]) if out[0] else 0, "tile_width": int(out[1]), "stages": int(out[2])}
 
 
 def protocol_numbers() -> dict:
