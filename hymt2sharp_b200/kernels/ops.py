@@ -2288,3 +2288,60 @@ def delta_scan(out: torch.Tensor, qn: torch.Tensor, kn: torch.Tensor, decay: tor
                                    c_int(dtype_code(v.dtype)), _ptr(state), c_long(state_offset), c_long(state.stride(0)), _ptr(cu_seqlens),
                                    _ptr(slot_ids), _ptr(kv_lens), c_int(batch), c_int(max_new_tokens), c_int(heads), c_int(kv_heads), c_int(dk),
                                    c_int(dv), _stream()), "delta_scan")
+
+
+# -- a dense block's step by one call ---------------------------------------------------------------------------------------------
+class _DenseBlock(ctypes.Structure):
+    """csrc/dense_block.cu: Hymt2DenseBlock, in the order of its members."""
+    _fields_ = ([(n, c_void_p) for n in ("x", "ss_in", "residual", "w_qkv", "w_o", "w_gate_up", "w_down", "q_gain", "k_gain", "norm2_gain",
+                                         "next_gain", "q", "att", "act", "normed", "ss", "k_plane", "v_plane", "block_table", "token_seq",
+                                         "token_pos", "slot_ids", "cu_seqlens", "kv_lens", "inv_freq", "angles", "workspace", "counters", "status")]
+                + [(n, c_long) for n in ("cache_blocks", "workspace_floats", "ldx")]
+                + [(n, c_int) for n in ("T", "hidden", "inner", "nh", "nkv", "batch", "max_new_tokens", "table_stride", "block_tokens", "rope_dim",
+                                        "write_kv", "window", "gain_dtype", "norm2_dtype", "next_dtype", "ss_in_tiles", "ss_tiles", "num_counters")]
+                + [(n, c_float) for n in ("qk_eps", "norm1_eps", "norm2_eps", "scale")])
+
+
+_dense_tiles: dict = {}
+
+
+def dense_block_tiles(tokens: int, hidden: int, nh: int, nkv: int, inner: int, rope_dim: int) -> int:
+    """Partial sums of squares a row between the products of a dense block that one call launches; 0: the kernels do not take these
+    sizes that way."""
+    key = (tokens, hidden, nh, nkv, inner, rope_dim)
+    hit = _dense_tiles.get(key)
+    if hit is None:
+        lib = _lib()
+        taken = hidden % 8 == 0 and inner % 8 == 0 and lib.hymt2_dense_block_bytes() == ctypes.sizeof(_DenseBlock) and \
+            bool(lib.hymt2_gemm_tc_rope_kv_supported(c_int(tokens), c_int((nh + 2 * nkv) * 128), c_int(hidden), c_int(rope_dim)))
+        tiles = gemm_tc_norm_tiles(tokens, hidden, nh * 128, EPILOGUE_ACCUMULATE) if taken else 0
+        if tiles != (gemm_tc_norm_tiles(tokens, hidden, inner, EPILOGUE_ACCUMULATE) if taken else 0):
+            tiles = 0
+        if len(_dense_tiles) > 4096:
+            _dense_tiles.clear()
+        hit = _dense_tiles[key] = tiles
+    return hit
+
+
+def dense_block(x, pre, residual, w_qkv, w_o, w_gate_up, w_down, q_gain, k_gain, norm2, following, q, att, act, normed, ss, k_plane, v_plane,
+                block_table, ctx, inv_freq, angles, rope_dim: int, nh: int, nkv: int, inner: int, write_kv: bool, window: int, qk_eps: float,
+                scale: float) -> None:
+    """The five kernels of a dense block's prompt step (parts.dense, which has checked the operands): x [T, hidden] is the first norm's
+    output, or with `pre` (parts.base.Prenormed) its first piece; `following`: the norm whose input the last product leaves in
+    (normed, ss), or None.  The buffers q, att, act, normed and ss are the step's own."""
+    T, hidden = residual.shape
+    floats, counters = _plan_scratch(T, inner, hidden, EPILOGUE_SWIGLU)
+    ws, cnt = _tc_workspace(residual.device, floats, counters) if floats else (None, None)
+    if (q_gain is None) != (k_gain is None) or (q_gain is not None and (q_gain.dtype != k_gain.dtype or q_gain.numel() != 128 or k_gain.numel() != 128)):
+        raise KernelError("dense_block: the gains of q and k hold 128 entries of one type each")
+    a = _address
+    block = _DenseBlock(
+        a(x), a(pre.ss) if pre else 0, a(residual), a(w_qkv), a(w_o), a(w_gate_up), a(w_down), a(q_gain), a(k_gain), a(norm2.gain),
+        a(following.gain) if following is not None else 0, a(q), a(att), a(act), a(normed), a(ss), a(k_plane), a(v_plane), a(block_table),
+        a(ctx.token_seq), a(ctx.token_pos), a(ctx.slot_ids), a(ctx.cu_seqlens), a(ctx.kv_lens), a(inv_freq), a(angles), a(ws), a(cnt), a(ctx.status),
+        k_plane.shape[0], ws.numel() if ws is not None else 0, x.stride(0),
+        T, hidden, inner, nh, nkv, ctx.num_seqs, ctx.max_new_tokens, block_table.stride(0), k_plane.shape[2], rope_dim, 1 if write_kv else 0, window,
+        dtype_code(q_gain.dtype) if q_gain is not None else F32, dtype_code(norm2.gain.dtype),
+        dtype_code(following.gain.dtype) if following is not None else F32, pre.ss.shape[1] if pre else 0, ss.shape[1],
+        cnt.numel() if cnt is not None else 0, qk_eps, pre.eps if pre else 0.0, norm2.eps, scale)
+    _check(_lib().hymt2_dense_block(ctypes.byref(block), _stream()), "dense_block", 5, timed=False)

@@ -4,6 +4,7 @@ float32; the normed activations have the engine's compute type."""
 from __future__ import annotations
 
 from ..kernels import ops
+from . import dense
 from .base import PartSpec, Prenormed, build_part, register_part
 
 
@@ -13,6 +14,7 @@ class PreNormBlock:
         self.mixer = build_part("mixer", mixer)
         self.norm2 = build_part("norm", norm2)
         self.feed_forward = build_part("feed_forward", feed_forward)
+        self.dense = dense.takes(self)         # whether a prompt's step may be launched by one call
 
     def parts(self):
         return (self.norm1, self.mixer, self.norm2, self.feed_forward)
@@ -47,6 +49,8 @@ class PreNormBlock:
         x = self.norm1.forward(residual, ctx, ctx.dtype)      # what the block before left behind, or the norm's own kernel
         if isinstance(x, Prenormed) and not getattr(self.mixer, "takes_prenormed", False):
             x = x.materialize(ctx)
+        if self.dense and dense.try_block(self, x, residual, ctx, slots[0]):
+            return
         # what the feed-forward streams first, for a mixer whose last kernel can ask for it ahead of time
         ctx.weights_ahead = getattr(self.feed_forward, "first_weights", lambda: None)()
         # the norm that comes next, for a mixer whose last product can prepare it
