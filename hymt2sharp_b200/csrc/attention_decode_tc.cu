@@ -246,9 +246,9 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 __syncwarp();
                 if (lane < 10) load_box(it, s, lane);
             }
-        } else if (warp == 1 && lane == 0) {
+        } else if (warp == 1 && elect_one()) {
             // ---- MMAs of the scores: S^T(n) = K(n) Q^T as soon as the keys have landed and the accumulator pair of
-            // n's parity is free.  (A thread that issues MMAs is slow at it: an MMA costs it ~56 cycles and a look
+            // n's parity is free.  (A thread that issues MMAs is slow at it: an MMA costs it ~31 cycles and a look
             // at a barrier ~190, so the two kinds of product have a thread each.  The descriptors of stage 0 are
             // built once; per instruction only constants are added: the address sits in the low bits in units of
             // 16 bytes, and shared memory is too small to carry out of them.)
@@ -269,7 +269,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
                 umma_commit(s_done + 8 * t);
             }
-        } else if (warp == 10 && lane == 0) {
+        } else if (warp == 10 && elect_one()) {
             // ---- MMAs of the weighted sums: O^T(n) = V(n)^T P^T(n) once P^T is written and the values have landed
             const uint64_t p_desc0 = desc_k_major(p_of(0)), v_desc0 = desc_mn_major(v_of(0), BOX);
             constexpr uint64_t STAGE_STEP = STAGE_BYTES >> 4;

@@ -210,7 +210,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     bool ok = true;             // softmax threads: no wait gave up
     float l = 0.f;              // and the sum of their row's numerators
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- producer: Q with K(0), then K(i + 1) with V(i) ---------------------------------------
         const int* table = p.block_table + (size_t)slot * p.table_stride;
         auto cache_row = [&](int tile) { return (table[tile_begin + tile] * p.nkv + kvh) * KEY_TILE; };
@@ -239,7 +239,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             for (int i = max(0, issued - KV_STAGES); i < issued; i++)
                 for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(kv_full + 8 * (i % KV_STAGES), (i / KV_STAGES) & 1); t++) {}
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- first MMA issuer: the scores, one tile ahead of the softmax warps ---------------------------
         // Two threads issue, each with a wait or two and a dozen instructions a tile: one thread doing both was
         // the slowest link of the chain.
@@ -277,7 +277,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             issue_scores(i + 1);
         }
-    } else if (warp == 2 && lane == 0) {
+    } else if (warp == 2 && elect_one()) {
         // ---- second MMA issuer: O += P V once the softmax warps have written P (and rescaled O where a maximum rose)
         const uint64_t p_desc0 = desc_k_major(k_smem), v_desc0 = desc_mn_major(v_smem, KEY_TILE * 128);
         constexpr uint64_t K_STEP = K_SLOT_BYTES >> 4, V_STEP = V_TILE_BYTES >> 4;

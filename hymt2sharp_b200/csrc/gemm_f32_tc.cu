@@ -216,7 +216,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (warp < WARP_CONVERT) {
     if constexpr (Regs::SPLIT) fewer_registers<Regs::MISC>();
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- copies: the first ring of W before the wait for the kernel in front, then the tokens ----
             auto load_w = [&](int tile, int c, int s) {
                 const uint32_t bar = full0 + 8 * s, dst = ring + s * stage_bytes;
@@ -250,7 +250,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(full0 + 8 * (i % stages), (i / stages) & 1); t++) {}
         }
     } else if (warp == WARP_PLANES) {
-        if (PLANES && lane == 0) {
+        if (PLANES && elect_one()) {
             // ---- planes: chunk i's two stages into slot i % PLANE_SLOTS, free again with its MMAs ----
             pdl_wait();
             uint32_t issued = 0;
@@ -270,7 +270,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(planes_full0 + 8 * (i % PLANE_SLOTS), (i / PLANE_SLOTS) & 1); t++) {}
         }
     } else {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer g: the chunks g, g + 2, ... of this CTA, counted through all tiles ----
             const int g = warp - WARP_ISSUER;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);

@@ -127,7 +127,7 @@ gemm_grouped_few_kernel(const __grid_constant__ CUtensorMap map_w, FewParams p) 
     const int begin = (int)(items * me / clusters), end = (int)(items * (me + 1) / clusters);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- weights: the ring runs on from item to item ----
             uint32_t s = 0, round = 0, issued = 0;
             bool ok = true;
@@ -150,7 +150,7 @@ gemm_grouped_few_kernel(const __grid_constant__ CUtensorMap map_w, FewParams p) 
                     for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(full0 + 8 * (i % stages), (i / stages) & 1); t++) {}
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMAs: block j into accumulator j % ACCS, the rows of the q-th row tile from buffer q & 1 ----
             const uint64_t w0 = desc_k_major(ring), x0 = desc_k_major(rows0);
             uint32_t s = 0, phase = 0;

@@ -434,7 +434,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer -------------------------------------------------------------------
         // Weights do not depend on the kernel before this one: the first ring of weight tiles is
         // requested at once, then the producer waits for that kernel and requests the activations.
@@ -477,7 +477,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int i = max(0, issued - stages); i < issued; i++)
                 for (uint32_t t = 0; t < tries && !mbar_try_wait(full0 + 8 * (i % stages), (i / stages) & 1); t++) {}
         }
-    } else if ((warp == 1 || (warp >= 6 && warp - 5 < ISSUERS)) && lane == 0) {
+    } else if ((warp == 1 || (warp >= 6 && warp - 5 < ISSUERS)) && elect_one()) {
         // ---- MMA issuers: warp 1 is issuer 0, warp 6 is issuer 1 ------------------------------------
         // The loop carries the stage's descriptor along (the address sits in the low bits, in units of 16 bytes,
         // and the ring is far too small to carry out of them) and adds constants: a chain of address arithmetic
@@ -1010,7 +1010,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_s;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- producer: the first stage's weights (B) before the wait, then everything in order ----
         // Stage and phase are counted along; whether the next stage is free was looked up while this one's copies
         // were issued (the stages of the first round are free anyway).
@@ -1074,7 +1074,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 for (uint32_t t = 0; t < (1u << 16) && !mbar_try_wait(full0 + 8 * s, round & 1); t++) {}
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0 && elect_one()) {
         // ---- MMA issuer (of a pair: the even CTA's): the stage's descriptor is carried along, see gemm_tc_kernel --------------
         const uint64_t desc0 = desc_k_major(tiles);
         uint64_t adesc = desc0;

@@ -67,6 +67,15 @@ __device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr, uint32_t mn_gro
            (2ull << 61);
 }
 
+// True in one thread of the (converged) warp: the thread that a role of one thread runs in.  By the instruction for it, and not by
+// `lane == 0`: the compiler then knows that one thread is there and keeps descriptors and addresses in uniform registers.  Cycles that an MMA
+// takes its issuer, elected / lane 0: 31 / 68, a commit 60 / 91; the tensor core itself takes 32 with 64 columns and 64 with 128.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(chosen));
+    return chosen != 0;
+}
+
 // D[tmem] (+)= A[smem] · B[smem], bfloat16 operands, float32 accumulator; issued by ONE thread.
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
