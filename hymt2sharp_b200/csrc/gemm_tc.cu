@@ -42,8 +42,11 @@ __host__ __device__ constexpr int tile_issuers(int bn, int epi) {
 }
 __host__ __device__ constexpr int tile_threads(int bn, int epi) { return tile_issuers(bn, epi) > 1 ? 224 : 192; }
 constexpr int A_TILE_BYTES = TILE_M * BLOCK_K * 2;
-// cycles of a k block of a pair's tile (fixed, and a column), of the start of a grid of pairs, and of a product from which on pairs are asked at all
-constexpr double PAIR_FIXED = 251.0, PAIR_COLUMN = 2.0, PAIR_START = 4500.0, PAIR_LEAST = 140e3;
+// Cycles of a k block of a pair's tile and of a single CTA's (fixed, and a column), of the start of a grid of pairs, and of a product from which
+// on pairs are asked at all.  Full power, 128 k blocks, us, single / pair: 128 columns 70 / 74, 192 95 / 94, 256 117 / 115.5 (the same operands
+// full of zeros 100 / 84: near the power limit the wider traffic costs little).  With these numbers the rule's choice was the best or within 1 %
+// of it at 23 of 24 products measured (1,000 to 4,096 tokens of the 1.8B and 4B sizes), and within 4 % at the other.
+constexpr double PAIR_FIXED = 150.0, PAIR_COLUMN = 2.41, SINGLE_FIXED = 171.0, SINGLE_COLUMN = 2.73, PAIR_START = 2500.0, PAIR_LEAST = 50e3;
 constexpr int PERSISTENT_BN = 256;   // tile width of the persistent kernel for many tokens
 
 // EPI_GLU is EPI_SWIGLU with another rule than silu(gate) * up, or with biases: an instance of its own, so that the plain one keeps
@@ -211,42 +214,34 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"((uint64_t)map), "r"(even_bar), "r"(x), "r"(y) : "memory");
 }
-// tma_stage_looking_ahead of one CTA of a pair: its rows of both operands, of one or two k blocks (`two`; the second `a2`, `b2` bytes behind the
-// first), counted at the even CTA's barrier, which the even CTA arms with both CTAs' bytes (`arm`).
+// tma_stage_looking_ahead of one CTA of a pair: its rows of both operands, counted at the even CTA's barrier, which the even CTA arms with both
+// CTAs' bytes (`arm`).
 __device__ __forceinline__ bool tma_pair_stage_looking_ahead(uint32_t bar, uint32_t arm, uint32_t bytes, uint32_t a_dst, const CUtensorMap* map_a, int x,
-                                                             int ay, uint32_t b_dst, const CUtensorMap* map_b, int by, uint32_t b2, uint32_t two,
-                                                             uint32_t next_bar, uint32_t next_parity) {
+                                                             int ay, uint32_t b_dst, const CUtensorMap* map_b, int by, uint32_t next_bar,
+                                                             uint32_t next_parity) {
     uint32_t seen;
     asm volatile(
-        "{\n\t.reg .pred look, even, second;\n\t.reg .b32 x2, a2, b2;\n\t"
+        "{\n\t.reg .pred look, even;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 look, [%10], %11;\n\t"
         "setp.ne.b32 even, %2, 0;\n\t"
-        "setp.ne.b32 second, %14, 0;\n\t"
-        "add.u32 x2, %6, 64;\n\tadd.u32 a2, %4, 16384;\n\tadd.u32 b2, %7, %15;\n\t"
         "@even mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %3;\n\t"
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%7], [%8, {%6, %9}], [%12];\n\t"
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%4], [%5, {%6, %13}], [%12];\n\t"
-        "@second cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [b2], [%8, {x2, %9}], [%12];\n\t"
-        "@second cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [a2], [%5, {x2, %13}], [%12];\n\t"
         "selp.u32 %0, 1, 0, look;\n\t}"
         : "=r"(seen)
         : "r"(bar), "r"(arm), "r"(bytes), "r"(a_dst), "l"((uint64_t)map_a), "r"(x), "r"(b_dst), "l"((uint64_t)map_b), "r"(by), "r"(next_bar),
-          "r"(next_parity), "r"(bar & EVEN_CTA), "r"(ay), "r"(two), "r"(b2)
+          "r"(next_parity), "r"(bar & EVEN_CTA), "r"(ay)
         : "memory");
-    static_assert(A_TILE_BYTES == 16384, "the second k block's activations lie behind the first's");
     return seen != 0;
 }
-// umma_block_looking_ahead for the pair, of one or two k blocks (`two`; descriptors of the second `a2`, `b2` units behind the first); the stage is
-// given back to both CTAs.
-__device__ __forceinline__ bool umma_pair_blocks_looking_ahead(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
-                                                               uint64_t a2, uint64_t b2, uint32_t two, uint32_t empty_bar, uint32_t next_bar,
-                                                               uint32_t next_parity) {
+// umma_block_looking_ahead for the pair; the stage is given back to both CTAs.
+__device__ __forceinline__ bool umma_pair_block_looking_ahead(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                              uint32_t empty_bar, uint32_t next_bar, uint32_t next_parity) {
     uint32_t seen;
     asm volatile(
-        "{\n\t.reg .pred look, first, yes, second;\n\t.reg .b64 a, b, c, d;\n\t.reg .b16 both;\n\t"
+        "{\n\t.reg .pred look, first, yes;\n\t.reg .b64 a, b;\n\t.reg .b16 both;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 look, [%7], %8;\n\t"
         "setp.ne.b32 first, %5, 0;\n\t"
-        "setp.ne.b32 second, %11, 0;\n\t"
         "setp.eq.u32 yes, 1, 1;\n\t"
         "mov.b16 both, 3;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %4, first;\n\t"
@@ -256,18 +251,10 @@ __device__ __forceinline__ bool umma_pair_blocks_looking_ahead(uint32_t tmem_d, 
         "tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
         "add.u64 a, %2, 6;\n\tadd.u64 b, %3, 6;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
-        "add.u64 c, %2, %9;\n\tadd.u64 d, %3, %10;\n\t"
-        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], c, d, %4, yes;\n\t"
-        "add.u64 a, c, 2;\n\tadd.u64 b, d, 2;\n\t"
-        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
-        "add.u64 a, c, 4;\n\tadd.u64 b, d, 4;\n\t"
-        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
-        "add.u64 a, c, 6;\n\tadd.u64 b, d, 6;\n\t"
-        "@second tcgen05.mma.cta_group::2.kind::f16 [%1], a, b, %4, yes;\n\t"
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], both;\n\t"
         "selp.u32 %0, 1, 0, look;\n\t}"
         : "=r"(seen)
-        : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_bar), "r"(next_parity), "l"(a2), "l"(b2), "r"(two)
+        : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(empty_bar), "r"(next_bar), "r"(next_parity)
         : "memory");
     return seen != 0;
 }
@@ -949,10 +936,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     constexpr bool SPLIT_B = is_gated(EPI);
     const int bn = p.bn;
     const int B_TILE_BYTES = bn * BLOCK_K * (PAIR ? 1 : 2);     // (a CTA of a pair holds half of the tile's weight rows)
-    // A look at a barrier takes the issuing threads some 500 cycles whatever hides in front of it, as long as a pair's MMAs of a k block:
-    // a pair's stage holds two k blocks.
-    constexpr int BLOCKS = PAIR ? 2 : 1;
-    const int STAGE_BYTES = BLOCKS * (A_TILE_BYTES + B_TILE_BYTES);
+    const int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
     constexpr int TMEM_COLS = 2 * BN;                       // 256 or 512
     constexpr int CTAS = PAIR ? 2 : 1, TILE_ROWS = CTAS * TILE_M;
     const int OUT_COLS = SPLIT_B ? bn / 2 : bn;
@@ -1026,21 +1010,17 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
             // (a pair's tile: the even CTA brings the first half of the weight rows, the odd one the second; of gated rows the gates and the ups)
             if (PAIR) b_row0 += rank * (SPLIT_B ? p.N : bn / 2);
-            for (int kb = 0; kb < num_k_blocks; kb += BLOCKS) {
+            for (int kb = 0; kb < num_k_blocks; kb++) {
                 if (round > 0 && !looked && !mbar_wait(empty0 + 8 * s, (round & 1) ^ 1, abort_flag, p.status, 101)) break;
-                const uint32_t bar = full0 + 8 * s, a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + BLOCKS * A_TILE_BYTES;
-                const uint32_t two = PAIR && kb + 1 < num_k_blocks ? 1u : 0u;
-                const uint32_t pair_bytes = 2 * (1 + two) * (A_TILE_BYTES + B_TILE_BYTES);
+                const uint32_t bar = full0 + 8 * s, a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + A_TILE_BYTES;
                 const int k = kb * BLOCK_K;
                 const uint32_t s_next = s + 1 == (uint32_t)stages ? 0 : s + 1, round_next = s_next ? round : round + 1;
                 if (first) {
                     if constexpr (PAIR) {
-                        if (rank == 0) mbar_expect_tx(bar, pair_bytes);
+                        if (rank == 0) mbar_expect_tx(bar, 2 * STAGE_BYTES);
                         tma_load_2d_pair(b_dst, &map_b, bar & EVEN_CTA, k, b_row0);
-                        if (two) tma_load_2d_pair(b_dst + B_TILE_BYTES, &map_b, bar & EVEN_CTA, k + BLOCK_K, b_row0);
                         pdl_wait();
                         tma_load_2d_pair(a_dst, &map_a, bar & EVEN_CTA, k, a_row0);
-                        if (two) tma_load_2d_pair(a_dst + A_TILE_BYTES, &map_a, bar & EVEN_CTA, k + BLOCK_K, a_row0);
                     } else {
                         mbar_expect_tx(bar, STAGE_BYTES);
                         tma_load_2d(b_dst, &map_b, bar, k, b_row0);
@@ -1053,7 +1033,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 } else {
                     bool seen;
                     if constexpr (PAIR)
-                        seen = tma_pair_stage_looking_ahead(bar, rank == 0 ? 1u : 0u, pair_bytes, a_dst, &map_a, k, a_row0, b_dst, &map_b, b_row0, B_TILE_BYTES, two,
+                        seen = tma_pair_stage_looking_ahead(bar, rank == 0 ? 1u : 0u, 2 * STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, b_row0,
                                                             empty0 + 8 * s_next, (round_next & 1) ^ 1);
                     else
                         seen = tma_stage_looking_ahead(bar, STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, k, b_row0,
@@ -1087,15 +1067,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             bool ok = true;
             const uint32_t acc_at = tmem_base + buf * BN;
-            for (int kb = 0; kb < num_k_blocks; kb += BLOCKS) {
+            for (int kb = 0; kb < num_k_blocks; kb++) {
                 if (!looked && !(ok = mbar_wait(full0 + 8 * s, phase, abort_flag, p.status, 102))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t s_next = s + 1 == (uint32_t)stages ? 0 : s + 1, phase_next = s_next ? phase : phase ^ 1;
                 // a look at a stage that will never be filled (behind the last one) is thrown away by the loops' ends
                 if constexpr (PAIR)
-                    looked = umma_pair_blocks_looking_ahead(acc_at, adesc, adesc + (2 * A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, A_TILE_BYTES >> 4,
-                                                            (uint64_t)(B_TILE_BYTES >> 4), kb + 1 < num_k_blocks ? 1u : 0u, empty0 + 8 * s,
-                                                            full0 + 8 * s_next, phase_next);
+                    looked = umma_pair_block_looking_ahead(acc_at, adesc, adesc + (A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, empty0 + 8 * s,
+                                                           full0 + 8 * s_next, phase_next);
                 else
                     looked = umma_block_looking_ahead(acc_at, adesc, adesc + (A_TILE_BYTES >> 4), IDESC, kb > 0 ? 1u : 0u, empty0 + 8 * s,
                                                       full0 + 8 * s_next, phase_next);
@@ -1348,7 +1327,8 @@ bool make_plan(int T, int N, int K, int epilogue, int sm_count, Plan* plan, bool
         pl.bn = 128;
         {
             // The tile's width: the one whose tiles fill whole waves of SMs best.  A k block of a tile bn wide
-            // costs about 350 + 1.84 bn cycles (measured at 192 to 256), and a wave lasts as long as one tile; behind
+            // costs about 350 + 1.84 bn cycles (measured at 192 to 256 when its issue took 270; 171 + 2.73 bn now, which puts the widths
+            // in nearly the same order: the best of them or within 3 % at 24 products), and a wave lasts as long as one tile; behind
             // the last wave one epilogue stands alone, which costs about 60 cycles a column where it rotates and
             // norms heads (measured: tiles of one head win up to a few thousand tokens, of two heads beyond), 30
             // where it adds into float32, 15 else.
@@ -1393,8 +1373,8 @@ bool make_plan(int T, int N, int K, int epilogue, int sm_count, Plan* plan, bool
 
 // Pairs of CTAs (cta_group::2) on tiles of 256 tokens: a CTA holds its 128 tokens and half of the tile's weight rows, so a k block brings
 // 16 KB + bn / 2 rows into each SM's shared memory and the MMAs read as much, where a CTA by itself brings and reads all bn rows.  That
-// traffic is what bounds the kernel of single CTAs (96 KB a k block at bn = 256, 128 bytes a cycle: 750 of its 821 cycles, the tensor
-// core needs 512).
+// traffic is what bounds the kernel of single CTAs as long as power does not: operands full of zeros, 128 k blocks, take it 443 cycles a k block
+// of 32 KB (128 columns) and 740 of 48 KB (256 columns), a pair 622 of 32 KB (256 columns); the tensor core needs 256 and 512.
 struct PairPlan {
     bool use;
     int bn, stages, pairs;
@@ -1408,7 +1388,7 @@ PairPlan plan_pairs(int T, int N, int K, int epilogue, const Plan& single) {
     // costs in cycles as in make_plan: waves of tiles, and the epilogue behind the last one
     const double epilogue_cycles = epilogue == EPI_ROPE_KV ? 60.0 : epilogue == EPI_ACCUMULATE ? 30.0 : 15.0;
     const long single_tiles = (long)single.grid.x * single.grid.y;
-    const double alone = (double)((single_tiles + single.sm_count - 1) / single.sm_count) * k_blocks * (350.0 + 1.84 * single.bn) + epilogue_cycles * single.bn;
+    const double alone = (double)((single_tiles + single.sm_count - 1) / single.sm_count) * k_blocks * (SINGLE_FIXED + SINGLE_COLUMN * single.bn) + epilogue_cycles * single.bn;
     const int step = epilogue == EPI_ROPE_KV ? TILE_M : 32;       // an MMA of a pair takes widths in steps of 32
     double best = 0;
     for (int bn = PERSISTENT_BN; bn >= 128; bn -= step) {
@@ -1422,7 +1402,7 @@ PairPlan plan_pairs(int T, int N, int K, int epilogue, const Plan& single) {
         }
     }
     pp.use = alone >= PAIR_LEAST && best + PAIR_START < alone;
-    const int stage = 2 * (A_TILE_BYTES + pp.bn * BLOCK_K);         // two k blocks
+    const int stage = A_TILE_BYTES + pp.bn * BLOCK_K;
     pp.stages = 224 * 1024 / stage > MAX_STAGES ? MAX_STAGES : 224 * 1024 / stage;
     pp.smem = (size_t)pp.stages * stage + 1024;
     return pp;

@@ -10,7 +10,8 @@ from test_gpu_kernels import DEV, _ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T, N, K, epilogue", [(8192, 3072, 2048, 0), (8000, 2504, 3080, 0), (10001, 4096, 4096, 1), (8200, 4104, 3072, 2), (16001, 1000, 4104, 0)])
+@pytest.mark.parametrize("T, N, K, epilogue", [(8192, 3072, 2048, 0), (8000, 2504, 3080, 0), (10001, 4096, 4096, 1), (8200, 4104, 3072, 2), (16001, 1000, 4104, 0),
+                                               (1025, 4104, 3080, 0), (1700, 2048, 4104, 1), (1000, 8192, 1024, 2)])
 def test_pairs_give_the_bits_of_single_ctas(T, N, K, epilogue):
     ops = _ops()
     assert ops.gemm_tc_pairs(T, N, K, epilogue)["pairs"] > 0
@@ -25,7 +26,7 @@ def test_pairs_give_the_bits_of_single_ctas(T, N, K, epilogue):
     out, after = base.clone(), sums(T)
     ops.gemm_tc(out, x, w, epilogue, status, row_scale=None if scale is None else (scale, K, 1e-5), norm_after=after)
     step = 400
-    for at in list(range(0, T, step))[:3] + [T - 300]:
+    for at in list(range(0, T, step))[:3] + [T - 300]:        # (parts of more than 128 rows: fewer run on another kernel, whose sums are split)
         part = base[at:at + step].clone()
         n = part.shape[0]
         assert ops.gemm_tc_pairs(n, N, K, epilogue)["pairs"] == 0
