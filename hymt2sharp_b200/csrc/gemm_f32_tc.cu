@@ -19,14 +19,14 @@
 //
 //   few rows: the tokens' float32 rows come by TMA beside W and are cut into pieces in the same kernel; K is cut over a cluster, which
 //             adds the parts through distributed shared memory.  Bound by the weights' way from memory where they are many (120,818 x
-//             2,048, 8 rows: 183 us, 5.4 TB/s; a kernel of FMA chains took 412), by start, fill and fold (4 to 5 us) where they are few.
-//             8 rows of the 1.8B sizes, us before and now: q/k/v 21 and 10, O 13 and 10, gate and up 44 and 29, down 36 and 22;
-//             1 row: 12.5 and 10, 10.3 and 10.2, 27 and 29, 28 and 22.
+//             2,048, 8 rows: 174 us, 5.7 TB/s; a kernel of FMA chains took 412), by start, fill and fold (4 to 5 us) where they are few.
+//             8 rows of the 1.8B sizes, us before and now: q/k/v 21 and 9.6, O 13 and 9.4, gate and up 44 and 25, down 36 and 19;
+//             1 row: 12.4 and 9.3, 10.3 and 8.9, 27 and 25, 28 and 18.
 //   many rows (PLANES): a kernel in front writes the tokens' pieces once (three planes), the product brings them by TMA; persistent, a
 //             CTA walks tiles of 128 weight rows x bn tokens, parts of K one after the other.  531 rows of the 1.8B sizes, before (tiles
-//             on CUDA cores, 44 TFLOP/s) and now: q/k/v 171 and 47, O 127 and 45, gate and up 596 and 186 (144 TFLOP/s of float32
-//             products), down 365 and 120.  Half the MMAs took 190 of 204 us: they are not the
-//             bound; a chunk's way around (cut, multiply, drain) takes a CTA 2,700 cycles.
+//             on CUDA cores, 44 TFLOP/s) and now: q/k/v 172 and 41, O 128 and 38, gate and up 598 and 157 (171 TFLOP/s of float32
+//             products), down 366 and 96.  Not bound by the MMAs (24 of 48 cycles a chunk at 96 columns) but by a stage's way through its
+//             converters: 1,500 to 1,800 cycles (a look 250, loads 200, cutting 600, stores and arrival 220), two stages at a time.
 //
 // Results that are not finite are computed again as the plain chain of FMAs: an infinity's pieces are not numbers, and a finite entry
 // near the largest float32 can round to an infinite hi.
@@ -42,8 +42,12 @@ enum { EPI_STORE = 0, EPI_ACCUMULATE = 1, EPI_SWIGLU = 2 };
 constexpr int ROWS = 128, STAGE_K = 32, CHUNK = 2 * STAGE_K, PIECE_COLS = STAGE_K / 2, A_COLS = 3 * PIECE_COLS;
 constexpr int W_BYTES = ROWS * STAGE_K * 4;
 constexpr int MAX_STAGES = 12, MAX_PARTS = 8, PLANES_BN = 96;
+constexpr int MEET = 4;           // columns of sums that meet their gates at a time
 constexpr int PLANE_SLOTS = 4;    // chunks of the tokens' planes in flight
-constexpr int BUFFERS = 4;        // of a stage's pieces: two chunks' worth, one multiplied while the other is written
+// Chunks of W's pieces in tensor memory: cut, multiplied and (where two blocks do not share an SM's tensor memory) one more.  A buffer's way around
+// (cut, a look, the MMAs, their completion, a look) takes 3,000 cycles.
+__host__ __device__ constexpr int buffers(bool planes, int bn) { return planes || bn > 32 ? 3 : 2; }
+constexpr int MAX_BUFFERS = 3;
 
 // Groups of four warps that cut stages into pieces, stage i by group i % groups: with up to 32 tokens two, of 64 registers a thread, so
 // that two blocks share an SM (the next product's first stages come in while this one's last are folded); with tiles of 64 tokens four.
@@ -159,20 +163,20 @@ __global__ void __launch_bounds__(threads_of(PLANES, BN), BN <= 32 ? 2 : 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_t, F32Params p) {
     constexpr int CONVERTERS = converters(PLANES, BN), WARP_DRAIN = warp_drain(PLANES, BN);
     constexpr int DRAIN_WARPS = drain_warps(PLANES), OWN = BN / drain_groups(PLANES);      // columns of the accumulator that a drain thread may own
-    constexpr int A_AT = (PLANES ? 3 : 2) * BN, TOTAL_AT = 2 * BN;
-    constexpr int USED = A_AT + BUFFERS * A_COLS, TMEM_COLS = USED <= 128 ? 128 : USED <= 256 ? 256 : 512;
+    constexpr int A_AT = 2 * BN;
+    constexpr int BUFFERS = buffers(PLANES, BN), USED = A_AT + 2 * BUFFERS * A_COLS, TMEM_COLS = USED <= 128 ? 128 : USED <= 256 ? 256 : 512;
     constexpr int OUT_ROWS = EPI == EPI_SWIGLU ? ROWS / 2 : ROWS;
     static_assert(USED <= 512, "tensor memory has 512 columns");
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 6 + 2 * PLANE_SLOTS];
+    __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4 + 2 * MAX_BUFFERS + 2 * PLANE_SLOTS];
     __shared__ uint32_t tmem_base_s;
-    __shared__ int abort_s, rich_s[BUFFERS];
+    __shared__ int abort_s, rich_s[2 * BUFFERS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bn = PLANES ? p.bn : BN, stages = p.stages;
     const int stage_bytes = W_BYTES + (PLANES ? 0 : token_bytes(false, bn)), plane_bytes = token_bytes(true, bn);
-    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, after_ring = ring + stages * stage_bytes;   // few rows: the buffers of the tokens' pieces; planes: their ring, and up sums on their way to their gates
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, after_ring = ring + stages * stage_bytes;   // few rows: the buffers of the tokens' pieces; planes: their ring, and sums on their way to be gated
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES]);
-    const uint32_t ready0 = smem_u32(&bars[2 * MAX_STAGES]), done0 = ready0 + 16, drained0 = done0 + 16, planes_full0 = drained0 + 16, planes_empty0 = planes_full0 + 8 * PLANE_SLOTS;
+    const uint32_t ready0 = smem_u32(&bars[2 * MAX_STAGES]), freed0 = ready0 + 8 * MAX_BUFFERS, done0 = freed0 + 8 * MAX_BUFFERS, drained0 = done0 + 16, planes_full0 = drained0 + 16, planes_empty0 = planes_full0 + 8 * PLANE_SLOTS;
     volatile int* abort_flag = &abort_s;
     // few rows: this CTA's part of K; planes: all of it, tile after tile.  (Of a chunk that K ends in, the second stage is zeros.)
     const int all_chunks = (p.K + CHUNK - 1) / CHUNK;
@@ -189,13 +193,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 4);         // the warps of a group of converters
         }
-        for (int b = 0; b < BUFFERS; b++) rich_s[b] = 0;
+        for (int b = 0; b < 2 * BUFFERS; b++) rich_s[b] = 0;
+        for (int b = 0; b < BUFFERS; b++) {
+            mbar_init(ready0 + 8 * b, 8);         // the warps of the converters of a chunk's two stages
+            mbar_init(freed0 + 8 * b, 1);
+        }
         for (int b = 0; b < PLANE_SLOTS; b++) {
             mbar_init(planes_full0 + 8 * b, 1);
             mbar_init(planes_empty0 + 8 * b, 1);
         }
         for (int g = 0; g < 2; g++) {
-            mbar_init(ready0 + 8 * g, 8);         // the warps of the converters of a chunk's two stages
             mbar_init(done0 + 8 * g, 1);
             mbar_init(drained0 + 8 * g, DRAIN_WARPS);
         }
@@ -274,26 +281,27 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             // ---- MMA issuer g: the chunks g, g + 2, ... of this CTA, counted through all tiles ----
             const int g = warp - WARP_ISSUER;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
-            const uint32_t d = tmem + g * BN, a0 = tmem + A_AT + 2 * g * A_COLS;
+            const uint32_t d = tmem + g * BN;
             const uint32_t plane_step = (uint32_t)(bn * (PLANES ? CHUNK : STAGE_K) * 2) >> 4;
             const long total = first_tile < tiles ? (long)((tiles - 1 - first_tile) / stride + 1) * chunks : 0;
             uint32_t use = 0;
             for (long j = g; j < total; j += 2, use++) {
+                const uint32_t buf = (uint32_t)j % BUFFERS, round = (uint32_t)j / BUFFERS, a0 = tmem + A_AT + 2 * buf * A_COLS;
                 // its planes' slot, which no other issuer looks at
                 const uint32_t slot = (uint32_t)j % PLANE_SLOTS, planes = planes_full0 + 8 * slot, planes_parity = (uint32_t)(j / PLANE_SLOTS) & 1;
                 static_assert(PLANE_SLOTS % 2 == 0, "a slot belongs to one issuer, who sees every phase of its barrier");
                 bool ok = !PLANES || use > 0 || mbar_wait(planes, planes_parity, abort_flag, p.status, 139);
                 if (PLANES && use > 0) ok = mbar_wait_both(planes, planes_parity, drained0 + 8 * g, (use - 1) & 1, abort_flag, p.status, 139);
-                ok = ok && (PLANES || use == 0 ? mbar_wait(ready0 + 8 * g, use & 1, abort_flag, p.status, 132)
-                                               : mbar_wait_both(ready0 + 8 * g, use & 1, drained0 + 8 * g, (use - 1) & 1, abort_flag, p.status, 132));
+                ok = ok && (PLANES || use == 0 ? mbar_wait(ready0 + 8 * buf, round & 1, abort_flag, p.status, 132)
+                                               : mbar_wait_both(ready0 + 8 * buf, round & 1, drained0 + 8 * g, (use - 1) & 1, abort_flag, p.status, 132));
                 if (!ok) break;
                 // whether W has more than its first pieces here
-                const bool rich = *(volatile int*)&rich_s[2 * g] == (int)(use + 1) || *(volatile int*)&rich_s[2 * g + 1] == (int)(use + 1);
+                const bool rich = *(volatile int*)&rich_s[2 * buf] == (int)(round + 1) || *(volatile int*)&rich_s[2 * buf + 1] == (int)(round + 1);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint64_t b[2];
                 // (planes: rows of 128 bytes, a chunk's entries; few rows: rows of 64 bytes, a stage's)
-                b[0] = PLANES ? desc_k_major(after_ring + 2 * slot * plane_bytes) : desc_rows_of_64(after_ring + 2 * g * plane_bytes);
-                b[1] = PLANES ? b[0] + 4 : desc_rows_of_64(after_ring + (2 * g + 1) * plane_bytes);
+                b[0] = PLANES ? desc_k_major(after_ring + 2 * slot * plane_bytes) : desc_rows_of_64(after_ring + 2 * buf * plane_bytes);
+                b[1] = PLANES ? b[0] + 4 : desc_rows_of_64(after_ring + (2 * buf + 1) * plane_bytes);
                 constexpr int HI = 0, MID = 1, LO = 2;
                 auto mma = [&](int wp, int tp, int k16, uint32_t acc) {
                     umma_ts(d, a0 + (k16 / 2) * A_COLS + wp * PIECE_COLS + (k16 % 2) * 8, b[k16 / 2] + tp * plane_step + (k16 % 2) * 2, idesc, acc);
@@ -311,6 +319,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                 for (int k16 = 0; k16 < CHUNK / 16; k16++) mma(HI, HI, k16, 1);
                 if (PLANES) umma_commit(planes_empty0 + 8 * slot);
+                umma_commit(freed0 + 8 * buf);
                 umma_commit(done0 + 8 * g);
             }
         }
@@ -321,33 +330,38 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int g = (warp - WARP_CONVERT) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
         const int member = (warp - WARP_CONVERT - 4 * g) * 32 + lane;           // of the group's 128 threads
         const long total = first_tile < tiles ? (long)((tiles - 1 - first_tile) / stride + 1) * steps : 0;
-        uint32_t s = g % stages;
+        uint32_t s = g, phase = 0;       // (stages are a multiple of the groups)
         for (long i = g; i < total; i += CONVERTERS) {
-            const uint32_t buf = (uint32_t)i % BUFFERS, use = (uint32_t)(i / BUFFERS);      // the buffer, and its uses so far
+            const uint32_t buf = (uint32_t)i % (2 * BUFFERS), use = (uint32_t)i / (2 * BUFFERS);      // the half of a buffer, and its uses so far
             const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + A_AT + buf * A_COLS;
-            // the stage's copies, and the buffer's last readers, the MMAs two chunks back
-            const bool ok = use > 0 ? mbar_wait_both(full0 + 8 * s, (i / stages) & 1, done0 + 8 * (buf >> 1), (use - 1) & 1, abort_flag, p.status, 135)
-                                    : mbar_wait(full0 + 8 * s, (i / stages) & 1, abort_flag, p.status, 135);
+            // the stage's copies, and the buffer's last readers
+            const bool ok = use > 0 ? mbar_wait_both(full0 + 8 * s, phase, freed0 + 8 * (buf >> 1), (use - 1) & 1, abort_flag, p.status, 135)
+                                    : mbar_wait(full0 + 8 * s, phase, abort_flag, p.status, 135);
             if (!__all_sync(0xffffffffu, ok)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t w_at = ring + s * stage_bytes + row * 128;
-            uint32_t hi[PIECE_COLS], mid[PIECE_COLS], lo[PIECE_COLS], more = 0;
+            // (all loads first, then half of the entries at a time: with all 48 registers of pieces alive the loads came one by one)
+            float4 v[STAGE_K / 4];
 #pragma unroll
-            for (int j = 0; j < STAGE_K / 4; j++) {
-                const float4 v = lds128(w_at + ((j ^ (row & 7)) << 4));
-                cut(v.x, v.y, hi[2 * j], mid[2 * j], lo[2 * j]);
-                cut(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
-                more |= mid[2 * j] | mid[2 * j + 1];       // (lo is only there where mid is)
+            for (int j = 0; j < STAGE_K / 4; j++) v[j] = lds128(w_at + ((j ^ (row & 7)) << 4));
+            uint32_t more = 0;
+#pragma unroll
+            for (int h = 0; h < PIECE_COLS; h += 8) {
+                uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float4 q = v[h / 2 + j];
+                    cut(q.x, q.y, hi[2 * j], mid[2 * j], lo[2 * j]);
+                    cut(q.z, q.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
+                    more |= mid[2 * j] | mid[2 * j + 1];       // (lo is only there where mid is)
+                }
+                tmem_store8(a + h, hi);
+                tmem_store8(a + PIECE_COLS + h, mid);
+                tmem_store8(a + 2 * PIECE_COLS + h, lo);
             }
             if (PLANES) {                             // the stage has been read
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty0 + 8 * s);
-            }
-#pragma unroll
-            for (int h = 0; h < PIECE_COLS; h += 8) {
-                tmem_store8(a + h, hi + h);
-                tmem_store8(a + PIECE_COLS + h, mid + h);
-                tmem_store8(a + 2 * PIECE_COLS + h, lo + h);
             }
             if (!PLANES) {
                 const uint32_t t_at = ring + s * stage_bytes + W_BYTES, b_at = after_ring + buf * plane_bytes;
@@ -375,7 +389,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 mbar_arrive(ready0 + 8 * (buf >> 1));
             }
             s += CONVERTERS;
-            while (s >= (uint32_t)stages) s -= stages;
+            if (s >= (uint32_t)stages) { s = g; phase ^= 1; }
         }
     } else {
         if constexpr (Regs::SPLIT) more_registers<Regs::DRAIN>();
@@ -387,7 +401,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t i = 0;
         bool ok = true;
         for (int tile = first_tile; tile < tiles && ok; tile += stride) {
-            float acc[OWN];
+            float acc[OWN], total[PLANES ? OWN : 1];
 #pragma unroll
             for (int j = 0; j < OWN; j++) acc[j] = 0.f;
             int in_part = 0, part = 0;
@@ -397,10 +411,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if constexpr (PLANES) {
-                    float v[OWN];
-                    tmem_loads(lanes + g * BN, v, own);
 #pragma unroll
-                    for (int j = 0; j < OWN; j++) acc[j] = in_part ? acc[j] + v[j] : v[j];
+                    for (int j = 0; j < OWN; j += 8) {
+                        if (j >= own) break;
+                        float v[8];
+                        tmem_loads(lanes + g * BN + j, v, 8);
+#pragma unroll
+                        for (int q = 0; q < 8; q++) acc[j + q] = in_part ? acc[j + q] + v[q] : v[q];
+                    }
                 } else {
 #pragma unroll
                     for (int j = 0; j < OWN; j += 16) {
@@ -415,17 +433,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (lane == 0) mbar_arrive(drained0 + 8 * g);
                 in_part++;
                 if (PLANES && p.parts > 1 && in_part == p.chunks_per_part && c + 1 < chunks) {
-                    // a part of K is through: it joins the parts before it, which wait in tensor memory
-                    if (part > 0) {
-                        float v[OWN];
-                        tmem_loads(lanes + TOTAL_AT, v, own);
+                    // a part of K is through: it joins the parts before it
 #pragma unroll
-                        for (int j = 0; j < OWN; j++) acc[j] = v[j] + acc[j];
-                    }
-#pragma unroll
-                    for (int j = 0; j < OWN; j += 8)
-                        if (j < own) tmem_store8(lanes + TOTAL_AT + j, reinterpret_cast<const uint32_t*>(acc) + j);
-                    tmem_store_wait();
+                    for (int j = 0; j < OWN; j++) total[j] = part ? total[j] + acc[j] : acc[j];
                     part++;
                     in_part = 0;
                 }
@@ -434,51 +444,45 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if constexpr (PLANES) {
                 const int m0 = tile_t(tile) + col0, cols = min(own, p.M - m0);
                 if (part > 0) {
-                    float v[OWN];
-                    tmem_loads(lanes + TOTAL_AT, v, own);
 #pragma unroll
-                    for (int j = 0; j < OWN; j++) acc[j] = v[j] + acc[j];
+                    for (int j = 0; j < OWN; j++) acc[j] = total[j] + acc[j];
                 }
                 // (sums that are not finite are left out here and computed again behind the others)
                 uint64_t odd = 0;
 #pragma unroll
                 for (int j = 0; j < OWN; j++) odd |= (uint64_t)(!is_finite(acc[j]) && j < cols) << j;
                 if constexpr (EPI == EPI_SWIGLU) {
-                    // the up sums (lanes 64 to 127) go to their gates' threads through shared memory, 8 columns at a time, [column][row]
-                    constexpr int UP_STEP = (ROWS / 2) * 4;
-                    const uint32_t up = after_ring + 2 * PLANE_SLOTS * plane_bytes + share * 8 * UP_STEP + (row & 63) * 4;
-                    const int n = tile_w(tile) * OUT_ROWS + (row & 63);
+                    // sums meet in shared memory, [column][row], MEET columns at a time; then a thread gates half of them
+                    constexpr int STEP = ROWS * 4, HALF = MEET / 2;
+                    const uint32_t sums = after_ring + 2 * PLANE_SLOTS * plane_bytes + share * MEET * STEP;
+                    const int n = tile_w(tile) * OUT_ROWS + (row & 63), first = row < 64 ? 0 : HALF;
+                    const long w_row = (row < 64 ? 0L : (long)p.N) + n;
                     if (n >= p.N) odd = 0;
-                    float* dst = p.C + (size_t)m0 * p.ldc + n;
-                    auto up_at = [&](int j) {
-                        float u;
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(u) : "r"(up + (j & 7) * UP_STEP) : "memory");
-                        return u;
-                    };
+                    float* dst = p.C + (size_t)(m0 + first) * p.ldc + n;
 #pragma unroll
-                    for (int j0 = 0; j0 < OWN; j0 += 8) {
+                    for (int j0 = 0; j0 < OWN; j0 += MEET, dst += MEET * p.ldc) {
                         if (j0 >= own) break;
-                        uint32_t left = (uint32_t)(odd >> j0) & 0xffu;
-                        if (row >= 64) {
 #pragma unroll
-                            for (int j = j0; j < j0 + 8; j++) asm volatile("st.shared.f32 [%0], %1;" ::"r"(up + (j & 7) * UP_STEP), "f"(acc[j]) : "memory");
-                            for (; left; left &= left - 1) {
-                                const int j = __ffs((int)left) - 1;
-                                asm volatile("st.shared.f32 [%0], %1;" ::"r"(up + j * UP_STEP),
-                                             "f"(fma_chain(p.A + (size_t)(m0 + j0 + j) * p.lda, p.W + ((long)p.N + n) * p.ldw, p.K)) : "memory");
-                            }
+                        for (int j = 0; j < MEET; j++) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + j * STEP + row * 4), "f"(acc[j0 + j]) : "memory");
+                        for (uint32_t left = (uint32_t)(odd >> j0) & ((1u << MEET) - 1); left; left &= left - 1) {
+                            const int j = __ffs((int)left) - 1;
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + j * STEP + row * 4),
+                                         "f"(fma_chain(p.A + (size_t)(m0 + j0 + j) * p.lda, p.W + w_row * p.ldw, p.K)) : "memory");
                         }
                         asm volatile("bar.sync %0, 128;" ::"r"(1 + share) : "memory");
-                        if (row < 64 && n < p.N) {
+                        float g[HALF], u[HALF];
 #pragma unroll
-                            for (int j = j0; j < j0 + 8; j++, dst += p.ldc)
-                                if (j < cols) *dst = glu_at(p.glu, acc[j], up_at(j), n, p.N);
-                            for (; left; left &= left - 1) {
-                                const int j = j0 + __ffs((int)left) - 1;
-                                p.C[(size_t)(m0 + j) * p.ldc + n] = glu_at(p.glu, fma_chain(p.A + (size_t)(m0 + j) * p.lda, p.W + (long)n * p.ldw, p.K), up_at(j), n, p.N);
-                            }
+                        for (int q = 0; q < HALF; q++) {
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(g[q]) : "r"(sums + (first + q) * STEP + (row & 63) * 4) : "memory");
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(u[q]) : "r"(sums + (first + q) * STEP + (64 + (row & 63)) * 4) : "memory");
                         }
                         asm volatile("bar.sync %0, 128;" ::"r"(1 + share) : "memory");
+                        if (n < p.N) {
+#pragma unroll
+                            for (int q = 0; q < HALF; q++) g[q] = glu_at(p.glu, g[q], u[q], n, p.N);
+#pragma unroll
+                            for (int q = 0; q < HALF; q++) if (j0 + first + q < cols) dst[q * p.ldc] = g[q];
+                        }
                     }
                 } else {
                     const int n = tile_w(tile) * OUT_ROWS + row;
@@ -638,7 +642,7 @@ void plan_f32(int M, int N, int K, int epi, bool aligned, F32Plan* out) {
     pl.bn = pl.planes ? bn : few_bn;
     pl.tiles_m = (M + pl.bn - 1) / pl.bn;
     const int stage = W_BYTES + (pl.planes ? 0 : token_bytes(false, pl.bn));
-    const int behind = (pl.planes ? 2 * PLANE_SLOTS : BUFFERS) * token_bytes(true, pl.bn) + (pl.planes && epi == EPI_SWIGLU ? drain_groups(true) * 8 * (ROWS / 2) * 4 : 0);
+    const int behind = 2 * (pl.planes ? PLANE_SLOTS : buffers(false, pl.bn)) * token_bytes(true, pl.bn) + (pl.planes && epi == EPI_SWIGLU ? drain_groups(true) * MEET * ROWS * 4 : 0);
     const int room = (!pl.planes && pl.bn <= 32 ? 113 : 224) * 1024 - 1024 - behind;       // two blocks an SM with up to 32 tokens
     // a multiple of the groups of converters: a stage then belongs to one of them, which sees every phase of its barrier
     const int groups = converters(pl.planes, pl.bn);
