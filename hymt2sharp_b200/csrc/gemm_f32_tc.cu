@@ -25,7 +25,7 @@
 //   many rows (PLANES): a kernel in front writes the tokens' pieces once (three planes), the product brings them by TMA; persistent, a
 //             CTA walks tiles of 128 weight rows x bn tokens, parts of K one after the other.  531 rows of the 1.8B sizes, before (tiles
 //             on CUDA cores, 44 TFLOP/s) and now: q/k/v 172 and 41, O 128 and 38, gate and up 598 and 157 (171 TFLOP/s of float32
-//             products), down 366 and 96.  Not bound by the MMAs (24 of 48 cycles a chunk at 96 columns) but by a stage's way through its
+//             products), down 366 and 96.  Not bound by the MMAs (a chunk has 24, of 48 cycles at 96 columns) but by a stage's way through its
 //             converters: 1,500 to 1,800 cycles (a look 250, loads 200, cutting 600, stores and arrival 220), two stages at a time.
 //
 // Results that are not finite are computed again as the plain chain of FMAs: an infinity's pieces are not numbers, and a finite entry
@@ -131,7 +131,7 @@ __host__ __device__ constexpr int token_bytes(bool planes, int bn) { return plan
 // Warp 0 brings W's stages (and with few rows the tokens'), warp 3 the planes, in a ring of their own: a stage of W is free again when it
 // is cut, planes when they are multiplied.  Groups of four warps cut W's (and, with few rows, the tokens') entries of stage after stage into
 // pieces (a stage takes a group 2,400 cycles, most of them latency: looks at barriers, shared memory, conversions, tensor memory), warps 1
-// and 2 issue the MMAs of the even and the odd chunks (an accumulator and two buffers of pieces each), the rest drains accumulators and
+// and 2 issue the MMAs of the even and the odd chunks (an accumulator each), the rest drains accumulators and
 // writes C.  A look at a barrier takes hundreds of cycles, and an accumulator's way around (MMAs, drain, MMAs) holds three of them: chunks of
 // 32 took 1,650 cycles whatever the MMAs in them, so a chunk is two stages.
 
