@@ -55,6 +55,10 @@ constexpr int MAX_BUFFERS = 3;
 // group's 2,400 cycles with 48 columns a warp) is what a tile's next chunk but one waits for (531 rows, gate and up: two groups 218 us, four 186).
 constexpr int WARP_ISSUER = 1, WARP_PLANES = 3, WARP_CONVERT = 4;
 __host__ __device__ constexpr int converters(bool planes, int bn) { return !planes && bn > 32 ? 4 : 2; }
+// Four groups take chunks in turns, and a group then meets a buffer's `freed` barrier in every other phase.  What keeps its parity from being an
+// old one is the ring: with four stages, a stage is copied only when the one two chunks before it was cut, behind that barrier's phase before.
+// With eight it is not (explored: seven chunks are enough for a wrong pass), so such a ring has four stages, however much room there is.
+__host__ __device__ constexpr int most_stages(bool planes, int bn) { return converters(planes, bn) > 2 ? 4 : MAX_STAGES; }
 __host__ __device__ constexpr int warp_drain(bool planes, int bn) { return WARP_CONVERT + 4 * converters(planes, bn); }
 
 struct F32Params {
@@ -135,7 +139,8 @@ __host__ __device__ constexpr int token_bytes(bool planes, int bn) { return plan
 // writes C.  A look at a barrier takes hundreds of cycles, and an accumulator's way around (MMAs, drain, MMAs) holds three of them: chunks of
 // 32 took 1,650 cycles whatever the MMAs in them, so a chunk is two stages.
 
-// Waits for two barriers, looking at both at once first (a look takes hundreds of cycles; the two then take one look's time).
+// Waits for two barriers, `a` and then `b`, looking at both behind one another first (a look takes hundreds of cycles; the two then take one
+// look's time).  Where b's parity means something only once a is through, this order sees to it: the second look comes behind the first.
 __device__ __forceinline__ bool mbar_wait_both(uint32_t a, uint32_t parity_a, uint32_t b, uint32_t parity_b, volatile int* abort_flag, int* status, int code) {
     uint32_t both;
     asm volatile(
@@ -290,10 +295,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 // its planes' slot, which no other issuer looks at
                 const uint32_t slot = (uint32_t)j % PLANE_SLOTS, planes = planes_full0 + 8 * slot, planes_parity = (uint32_t)(j / PLANE_SLOTS) & 1;
                 static_assert(PLANE_SLOTS % 2 == 0, "a slot belongs to one issuer, who sees every phase of its barrier");
-                bool ok = !PLANES || use > 0 || mbar_wait(planes, planes_parity, abort_flag, p.status, 139);
-                if (PLANES && use > 0) ok = mbar_wait_both(planes, planes_parity, drained0 + 8 * g, (use - 1) & 1, abort_flag, p.status, 139);
-                ok = ok && (PLANES || use == 0 ? mbar_wait(ready0 + 8 * buf, round & 1, abort_flag, p.status, 132)
-                                               : mbar_wait_both(ready0 + 8 * buf, round & 1, drained0 + 8 * g, (use - 1) & 1, abort_flag, p.status, 132));
+                // Its own accumulator's drain is waited for BEFORE the pieces.  It is taken out of tensor memory chunk after chunk, so chunk
+                // j - 2 drained means chunk j - 3 multiplied, whose pieces stood in this buffer: an issuer meets a buffer's barrier in every
+                // other phase only, and looked at first its parity could still be that of the phase before the last one.
+                const uint32_t pieces = ready0 + 8 * buf, drained = drained0 + 8 * g, drained_parity = (use - 1) & 1;
+                bool ok;
+                if constexpr (PLANES) {
+                    ok = use > 0 ? mbar_wait_both(planes, planes_parity, drained, drained_parity, abort_flag, p.status, 139)
+                                 : mbar_wait(planes, planes_parity, abort_flag, p.status, 139);
+                    ok = ok && mbar_wait(pieces, round & 1, abort_flag, p.status, 132);
+                } else {
+                    ok = use > 0 ? mbar_wait_both(drained, drained_parity, pieces, round & 1, abort_flag, p.status, 132)
+                                 : mbar_wait(pieces, round & 1, abort_flag, p.status, 132);
+                }
                 if (!ok) break;
                 // whether W has more than its first pieces here
                 const bool rich = *(volatile int*)&rich_s[2 * buf] == (int)(round + 1) || *(volatile int*)&rich_s[2 * buf + 1] == (int)(round + 1);
@@ -645,8 +659,8 @@ void plan_f32(int M, int N, int K, int epi, bool aligned, F32Plan* out) {
     const int behind = 2 * (pl.planes ? PLANE_SLOTS : buffers(false, pl.bn)) * token_bytes(true, pl.bn) + (pl.planes && epi == EPI_SWIGLU ? drain_groups(true) * MEET * ROWS * 4 : 0);
     const int room = (!pl.planes && pl.bn <= 32 ? 113 : 224) * 1024 - 1024 - behind;       // two blocks an SM with up to 32 tokens
     // a multiple of the groups of converters: a stage then belongs to one of them, which sees every phase of its barrier
-    const int groups = converters(pl.planes, pl.bn);
-    pl.stages = (room / stage > MAX_STAGES ? MAX_STAGES : room / stage) / groups * groups;
+    const int groups = converters(pl.planes, pl.bn), most = most_stages(pl.planes, pl.bn);
+    pl.stages = (room / stage > most ? most : room / stage) / groups * groups;
     pl.smem = (size_t)pl.stages * stage + behind + 1024;
     const long tiles = (long)pl.tiles_m * pl.tiles_n;
     pl.ctas = pl.planes ? (int)(tiles < SMS ? tiles : SMS) : 0;
@@ -697,6 +711,14 @@ int launch_width(const CUtensorMap& mw, const CUtensorMap& mt, const F32Params& 
 inline bool rows_on_16(const void* A, long lda) { return (uintptr_t)A % 16 == 0 && lda % 4 == 0; }
 
 }  // namespace
+
+// The numbers of the kernel's barrier protocol: out[0] groups of converters and [1] buffers of pieces with up to 32 tokens, [2], [3] with tiles of 64,
+// [4], [5] with planes, [6] slots of planes, [7] 1: an issuer waits for its accumulator before it looks at the pieces
+HYMT2_API int hymt2_gemm_f32_tc_protocol(int* out) {
+    out[0] = converters(false, 32); out[1] = buffers(false, 32); out[2] = converters(false, 64); out[3] = buffers(false, 64);
+    out[4] = converters(true, PLANES_BN); out[5] = buffers(true, PLANES_BN); out[6] = PLANE_SLOTS; out[7] = 1;
+    return HYMT2_OK;
+}
 
 // How a product would be run: out[0] 1 where a kernel in front writes the tokens' pieces, [1] the tile's tokens, [2] stages, [3] parts of K,
 // [4] bytes of scratch for the pieces.  `aligned`: rows of A start on 16 bytes.  Nothing is launched.

@@ -1,6 +1,6 @@
 """The barrier protocols of the tcgen05 kernels, restated as little programs and explored over EVERY interleaving,
 without a GPU.  First and in most detail the prefill attention kernel (hymt2sharp_b200/csrc/attention_prefill_tc.cu);
-the decode attention and the persistent matrix product follow at the end.
+the decode attention and the matrix products follow at the end.
 
 Why: a wait on an mbarrier names a parity, and a parity cannot tell a phase from the one two later.  A reader that
 falls two phases behind its barrier waits for ever; one that is a phase early passes at once.  Whether that can
@@ -249,3 +249,63 @@ def test_issuers_that_own_their_stages_never_misread_a_barrier(blocks, stages, i
 def test_three_issuers_taking_turns_over_five_stages_did():
     """The version that ended two launches with a fault: an issuer took a stage whose copy had not landed."""
     assert "passes its wait" in tile_gemm(32, 5, 3, own=False)
+
+
+# ---- the float32 product (hymt2sharp_b200/csrc/gemm_f32_tc.cu): stages of W are cut into pieces, two stages a chunk ----
+#   producer        for every stage i: wait "stage free" (the stage a ring earlier), copy the stage
+#   converter g     for the stages i = g, g + groups, ...: wait the stage, wait "buffer free" (the chunk `buffers` earlier is
+#                   multiplied), free the stage, announce half of chunk i div 2 (two arrivals complete it)
+#   planes          (where the tokens' pieces come ready) for every chunk j: wait "slot free", copy the slot
+#   issuer g of 2   for the chunks j = g, g + 2, ...: wait its accumulator drained (chunk j - 2) and the pieces of chunk j, in that
+#                   order; issue its MMAs, which free the buffer (and the slot) and complete the chunk
+#   drain           for every chunk: wait it complete, announce its accumulator drained
+# (where two barriers are looked at behind one another first, that is these waits passing without delay)
+def f32_product(chunks, groups, buffers, stages, slots=0, drained_first=True):
+    producer, drain, planes = [], [], []
+    converters, issuers = [[] for _ in range(groups)], ([], [])
+    for i in range(2 * chunks):
+        s, buf, use = i % stages, i // 2 % buffers, i // 2 // buffers
+        if i >= stages:
+            producer.append(("wait", "empty", s, i // stages - 1))
+        producer.append(("copy", "full", s))
+        freed = [("wait", "freed", buf, use - 1)] if use else []
+        converters[i % groups] += [("wait", "full", s, i // stages), *freed, ("arrive", "empty", s), ("arrive", "ready", buf)]
+    for j in range(chunks):
+        buf, g, use = j % buffers, j % 2, j // 2
+        drained = [("wait", "drained", g, use - 1)] if use else []
+        ready = [("wait", "ready", buf, j // buffers)]
+        frees = [("freed", buf), ("done", g)]
+        if slots:
+            planes += [("wait", "slot_free", j % slots, j // slots - 1)] if j >= slots else []
+            planes.append(("copy", "slot_full", j % slots))
+            issuers[g].append(("wait", "slot_full", j % slots, j // slots))
+            frees = [("slot_free", j % slots)] + frees
+        issuers[g].extend((drained + ready if drained_first else ready + drained) + [("issue", f"MMA{g}", frees)])
+        drain += [("wait", "done", g, use), ("arrive", "drained", g)]
+    sizes = dict(full=stages, empty=stages, ready=buffers, freed=buffers, done=2, drained=2, slot_full=max(slots, 1), slot_free=max(slots, 1))
+    return explore((producer, *converters, *issuers, drain, planes), sizes, {"ready": 2})
+
+
+@pytest.mark.parametrize("rows, chunks", [(16, 1), (16, 9), (32, 7), (64, 1), (64, 4), (64, 7), (64, 10)])
+def test_no_interleaving_of_the_float32_products_protocol_goes_wrong(rows, chunks):
+    n, form = NUMBERS["f32"], "few" if rows <= 32 else "wide"
+    planes, _, stages, _, _ = ops.gemm_f32_tc_plan(rows, 2048, 64 * chunks)
+    assert not planes and n["drained_first"] == 1
+    assert f32_product(chunks, n[form + "_groups"], n[form + "_buffers"], stages) is None
+
+
+@pytest.mark.parametrize("chunks, stages", [(1, 4), (4, 4), (3, 6)])
+def test_no_interleaving_of_the_float32_products_protocol_with_planes_goes_wrong(chunks, stages):
+    n = NUMBERS["f32"]
+    assert f32_product(chunks, n["planes_groups"], n["planes_buffers"], stages, n["plane_slots"]) is None
+    assert f32_product(chunks + 2, n["planes_groups"], n["planes_buffers"], stages, 2) is None      # (fewer slots: more reuse in fewer chunks)
+
+
+def test_the_float32_products_two_rules_are_needed():
+    """Pieces looked at before the accumulator is drained (tiles of 64 rows did, three buffers between two issuers): the parity of the phase before the
+    last passes.  Four groups of converters over eight stages instead of four: so does a buffer's, in front of the writes."""
+    n = NUMBERS["f32"]
+    assert "of ready" in f32_product(4, n["wide_groups"], n["wide_buffers"], 4, drained_first=False)
+    assert f32_product(4, n["wide_groups"], n["wide_buffers"], 4) is None
+    for rows in (33, 64):
+        assert ops.gemm_f32_tc_plan(rows, 2048, 2048)[2] == 4
