@@ -669,14 +669,14 @@ def protocol_numbers() -> dict:
     """The numbers that the barrier protocols of the tcgen05 kernels are built on, as compiled (stages, slots, barriers
     per purpose, issuers): what an exploration of the protocols has to be run with.  Works without a GPU."""
     def ask(fn, names):
-        out = (ctypes.c_int * 8)()
+        out = (ctypes.c_int * 16)()
         getattr(_lib(), fn)(out)
         return dict(zip(names, out))
     return {"prefill": ask("hymt2_attention_prefill_tc_protocol", ("kv_stages", "k_slots", "p_bars", "o_bars", "stage_holders", "s_buffers")),
             "decode": ask("hymt2_attention_decode_tc_protocol", ("stages", "accumulators")),
             "gemm": ask("hymt2_gemm_tc_protocol", ("max_stages", "accumulators", "issuers", "issuers_own_stages", "epilogue_groups")),
             "f32": ask("hymt2_gemm_f32_tc_protocol", ("few_groups", "few_buffers", "wide_groups", "wide_buffers", "planes_groups", "planes_buffers",
-                                                      "plane_slots", "drained_first"))}
+                                                      "plane_slots", "drained_first", "gated_warps", "gated_vote"))}
 
 
 def gemm_tc_rope_kv_wants_angles(tokens: int, rope_dim: int) -> bool:
