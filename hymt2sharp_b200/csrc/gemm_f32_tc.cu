@@ -750,6 +750,7 @@ HYMT2_API int hymt2_gemm_f32_tc(void* C, const void* A, const void* W, int M, in
     if (M == 0 || N == 0) return HYMT2_OK;
     HYMT2_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32_tc: bad sizes M=%d N=%d K=%d", M, N, K);
     HYMT2_REQUIRE(epilogue >= 0 && epilogue <= 2 && status, "gemm_f32_tc: epilogue %d, or no status word", epilogue);
+    HYMT2_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32_tc: a leading dimension is smaller than its row");
     HYMT2_REQUIRE((uintptr_t)W % 16 == 0 && ldw % 4 == 0, "gemm_f32_tc: rows of W must start on 16 bytes (ldw=%ld)", ldw);
     F32Plan pl;
     plan_f32(M, N, K, epilogue, rows_on_16(A, lda), &pl);

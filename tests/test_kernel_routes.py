@@ -1,4 +1,6 @@
-"""Which kernel a call takes, where a rule on its sizes decides (no GPU)."""
+"""Which kernel a call takes, where a rule on its sizes decides, and what is refused before anything is launched (no GPU)."""
+import ctypes
+
 import pytest
 
 from hymt2sharp_b200.kernels import ops
@@ -36,3 +38,15 @@ def test_few_rows_stream_their_weights_as_far_as_that_is_faster(rows, widest, wi
                                                     (4096, 16, 24, 32), (4096, 16, 136, 32), (18944, 1, 128, 64)])
 def test_rows_a_block_of_32_bit_prompt_attention(tokens, heads, d, rows):
     assert ops.attention_prompt_rows(tokens, heads, d) == rows
+
+
+@pytest.mark.parametrize("lda, ldw, ldc", [(2044, 2048, 1024), (0, 2048, 1024), (2048, 2044, 1024), (2048, 0, 1024), (2048, 2048, 1023), (2048, 2048, 0)])
+def test_float32_products_refuse_rows_that_overlap(lda, ldw, ldc):
+    """As the CUDA-core product does: such rows of C would be written by several at once."""
+    lib, at = ops._lib(), 1 << 20          # (an address that nothing gets to read)
+    for name, call in (("gemm_f32_tc", lambda: lib.hymt2_gemm_f32_tc(at, at, at, 8, 1024, 2048, lda, ldw, ldc, 0, None, 0, at, None, 0, 0.0, 1.0, None)),
+                       ("gemm", lambda: lib.hymt2_gemm_simt(ctypes.c_void_p(at), 0, ctypes.c_void_p(at), 0, ctypes.c_void_p(at), 0, 8, 1024, 2048,
+                                                            ctypes.c_long(lda), ctypes.c_long(ldw), ctypes.c_long(ldc), 0, 0, ctypes.c_float(0),
+                                                            ctypes.c_float(1), None, None))):
+        assert call() == -1
+        assert "leading dimension is smaller than its row" in lib.hymt2_last_error().decode(), name
