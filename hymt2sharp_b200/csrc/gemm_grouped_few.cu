@@ -297,7 +297,12 @@ int launch_few(const CUtensorMap& map, const FewParams& p, int clusters, size_t 
 
 }  // namespace
 
-HYMT2_API int hymt2_gemm_grouped_few_max_k() { return MAX_K; }
+// The numbers of the kernel's barrier protocol: out[0] CTAs of a cluster, [1] accumulators, [2] buffers of rows, [3] warps that load rows, [4] the most
+// stages of the ring, [5] buffers of the quarters' sums, [6] the largest K
+HYMT2_API int hymt2_gemm_grouped_few_protocol(int* out) {
+    out[0] = RANKS; out[1] = ACCS; out[2] = 2; out[3] = LOADERS / 32; out[4] = MAX_STAGES; out[5] = 2; out[6] = MAX_K;
+    return HYMT2_OK;
+}
 
 // Row tiles of 8 sorted rows; W the groups' matrices one after the other ([N, K] each, or N gate rows and N up rows), bfloat16.  K: a
 // multiple of 256 up to 4,096; A's rows on 16 bytes.

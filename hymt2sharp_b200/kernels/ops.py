@@ -676,7 +676,9 @@ def protocol_numbers() -> dict:
             "decode": ask("hymt2_attention_decode_tc_protocol", ("stages", "accumulators")),
             "gemm": ask("hymt2_gemm_tc_protocol", ("max_stages", "accumulators", "issuers", "issuers_own_stages", "epilogue_groups")),
             "f32": ask("hymt2_gemm_f32_tc_protocol", ("few_groups", "few_buffers", "wide_groups", "wide_buffers", "planes_groups", "planes_buffers",
-                                                      "plane_slots", "drained_first", "gated_warps", "gated_vote"))}
+                                                      "plane_slots", "drained_first", "gated_warps", "gated_vote")),
+            "grouped_few": ask("hymt2_gemm_grouped_few_protocol", ("ranks", "accumulators", "row_buffers", "loader_warps", "max_stages", "sum_buffers",
+                                                                   "max_inner"))}
 
 
 def gemm_tc_rope_kv_wants_angles(tokens: int, rope_dim: int) -> bool:
@@ -1728,13 +1730,14 @@ def gemm_grouped(kernel: str, out: torch.Tensor, a: torch.Tensor, w: torch.Tenso
 # times a matrix's entries): below, the start of its clusters is longer than the reading.  us, CUDA cores / tensor cores: 4.2 M entries 4.1 6.6
 # and 7.3 6.9; 8.4 M 7.3 7.3 and 6.6 9.3; 16.8 M 12.4 9.8, 12.3 9.7 and 13.6 11.2; 67 M 36 27 and 40 27; 134 M 53 33.
 FEW_MIN_ENTRIES = 12 << 20
+FEW_MAX_INNER = 4096           # (csrc/gemm_grouped_few.cu: MAX_K)
 
 
 def gemm_grouped_few_supported(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
     """Whether `pairs` (token, choice) pairs' grouped product runs on the tensor cores in tiles of 8 rows: bfloat16, rows on 16 bytes, the
     inner size a multiple of 256 up to 4,096, and enough of the matrices in use to be worth it."""
     K = a.shape[1]
-    return a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 256 == 0 and K <= 4096 and a.stride(1) == 1 and a.stride(0) % 8 == 0 \
+    return a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 256 == 0 and K <= FEW_MAX_INNER and a.stride(1) == 1 and a.stride(0) % 8 == 0 \
         and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous() and min(pairs, w.shape[0]) * w.shape[1] * K >= FEW_MIN_ENTRIES
 
 

@@ -165,7 +165,7 @@ class RoutedExperts:
             rows, gather = torch.empty((tiles * tile, self.hidden), dtype=x.dtype, device=dev), False
             ops.moe_gather(rows, x, row_token)
         # (one rule for both products: tiles of 8 rows go where the reading is worth the start)
-        few = kernel == "skinny" and self.intermediate % 256 == 0 and self.intermediate <= 4096 \
+        few = kernel == "skinny" and self.intermediate % 256 == 0 and self.intermediate <= ops.FEW_MAX_INNER \
             and ops.gemm_grouped_few_supported(x, self.up, T * self.top)
         grouped = ops.gemm_grouped_few if few else lambda *args: ops.gemm_grouped(kernel, *args)
         ops.tag = "experts_up"

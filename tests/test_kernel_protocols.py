@@ -30,7 +30,8 @@ NUMBERS = ops.protocol_numbers()
 def explore(roles, sizes, arrivals_needed=None):
     """roles: programs of ("wait" | "wait or not", barrier, index, phase), ("arrive", barrier, index),
     ("copy", barrier, index) — lands at any later time — and ("issue", queue, [(barrier, index), ...]) — completes at
-    any later time after the products issued before it on the same queue, and then arrives at its barriers.
+    any later time after the products issued before it on the same queue, and then arrives at its barriers.  ("must", barrier, index,
+    phase) is no wait: going on while that phase is not complete is what goes wrong (memory that others have yet to read is written).
     sizes: barriers of each name; arrivals_needed: arrivals that complete a phase (1 unless named).
     Returns None when no interleaving goes wrong, else a sentence about the first one found that does."""
     arrivals_needed = arrivals_needed or {}
@@ -68,6 +69,11 @@ def explore(roles, sizes, arrivals_needed=None):
                     if complete != phase + 1:
                         return f"role {r} passes its wait for phase {phase} of {bar}[{idx}] with {complete} phases complete"
                     after.append((moved, done, held, copies, issued))
+            elif op[0] == "must":
+                _, bar, idx, phase = op
+                if done[at[bar] + idx] <= phase:
+                    return f"role {r} goes on without phase {phase} of {bar}[{idx}]"
+                after.append((moved, done, held, copies, issued))
             elif op[0] == "arrive":
                 d, h = arrive(done, held, op[1], op[2])
                 after.append((moved, d, h, copies, issued))
@@ -221,6 +227,42 @@ def test_no_interleaving_of_the_persistent_products_protocol_goes_wrong(tiles, k
     assert persistent_gemm(tiles, k_blocks, stages, groups=1) is None
 
 
+# ---- the same by pairs of CTAs: the even one's issuer and barriers for what both bring, both CTAs' for what they are given back ----
+#   producer r     its rows of both operands, counted at the even CTA's stage (which the even producer arms: one arrival more)
+#   issuer (even)  as above; its completions free the stage in both CTAs and fill the accumulator's barrier in both
+#   epilogue r     drains its CTA's half and announces that at the even CTA (`acc_empty` wants both)
+def pair_gemm(tiles, k_blocks, stages, groups=None):
+    groups = groups or NUMBERS["gemm"]["epilogue_groups"]
+    producers, issuer, epilogues = ([], []), [], [[] for _ in range(2 * groups)]
+    block = 0
+    for j in range(tiles):
+        if j >= 2:
+            issuer.append(("wait", "acc_empty", j & 1, (j >> 1) - 1))
+        for _ in range(k_blocks):
+            s, use = block % stages, block // stages
+            for r, producer in enumerate(producers):
+                if use > 0:
+                    producer.append(("wait", f"empty{r}", s, use - 1))
+                producer += ([("arrive", "full", s)] if r == 0 else []) + [("copy", "full", s)]
+            issuer += [("wait", "full", s, use), ("issue", "MMA", [("empty0", s), ("empty1", s)])]
+            block += 1
+        issuer.append(("issue", "MMA", [("acc_full0", j & 1), ("acc_full1", j & 1)]))
+        for r in range(2):
+            epilogues[r * groups + j % groups] += [("wait", f"acc_full{r}", j & 1, j >> 1), ("arrive", "acc_empty", j & 1)]
+    if groups == 2:
+        last = tiles - 1
+        for r in range(2):
+            epilogues[r * groups + 1 - last % 2].append(("wait", f"acc_full{r}", last & 1, last >> 1))
+    sizes = {"full": stages, "empty0": stages, "empty1": stages, "acc_full0": 2, "acc_full1": 2, "acc_empty": 2}
+    return explore((*producers, issuer, *epilogues), sizes, {"full": 3, "acc_empty": 2})
+
+
+@pytest.mark.parametrize("tiles, k_blocks, stages", [(1, 1, 4), (3, 2, 4), (5, 3, 2), (4, 4, 3)])
+def test_no_interleaving_of_the_pairs_protocol_goes_wrong(tiles, k_blocks, stages):
+    assert pair_gemm(tiles, k_blocks, stages) is None
+    assert pair_gemm(tiles, k_blocks, stages, groups=1) is None
+
+
 # ---- the tile kernel of the matrix product with several MMA issuers (few tokens): who may read which stage's barrier ----
 #   producer   for every k block i: wait "stage i mod stages free" (block i - stages), copy the stage
 #   issuer j   takes some of the k blocks: wait the stage, issue its MMAs into an accumulator of its own (they free the stage)
@@ -309,6 +351,74 @@ def test_the_float32_products_two_rules_are_needed():
     assert f32_product(4, n["wide_groups"], n["wide_buffers"], 4) is None
     for rows in (33, 64):
         assert ops.gemm_f32_tc_plan(rows, 2048, 2048)[2] == 4
+
+
+# ---- the grouped product of few rows (hymt2sharp_b200/csrc/gemm_grouped_few.cu): a CTA by itself, then what a cluster's CTAs hand each other ----
+#   producer   for every weight block: wait "stage free", copy it
+#   loaders    for the q-th row tile of the CTA's items: wait "rows free" (tile q - 2), announce the rows (all loaders)
+#   issuer     an item of another row tile: wait its rows; for every block: wait the stage, wait "accumulator drained" (`accs` blocks
+#              earlier), issue (frees the stage, completes the accumulator); behind a row tile's last item a completion frees its rows
+#   sums       for every block: wait the accumulator, announce it drained
+def few_rows_cta(items, blocks, stages, accs, loaders):
+    producer, rows, issuer, sums = [], [], [], []
+    q, tile, j = -1, None, 0
+    for n, item in enumerate(items):
+        if item != tile:
+            tile, q = item, q + 1
+            if q >= 2:
+                rows.append(("wait", "rows_free", q & 1, (q >> 1) - 1))
+            rows.append(("arrive", "rows_full", q & 1))
+            issuer.append(("wait", "rows_full", q & 1, q >> 1))
+        for _ in range(blocks):
+            s, use = j % stages, j // stages
+            if use > 0:
+                producer.append(("wait", "empty", s, use - 1))
+            producer.append(("copy", "full", s))
+            issuer.append(("wait", "full", s, use))
+            if j >= accs:
+                issuer.append(("wait", "acc_empty", j % accs, j // accs - 1))
+            issuer.append(("issue", "MMA", [("empty", s), ("acc_full", j % accs)]))
+            sums += [("wait", "acc_full", j % accs, j // accs), ("arrive", "acc_empty", j % accs)]
+            j += 1
+        if n + 1 < len(items) and items[n + 1] != tile:
+            issuer.append(("issue", "MMA", [("rows_free", q & 1)]))
+    sizes = {"full": stages, "empty": stages, "acc_full": accs, "acc_empty": accs, "rows_full": 2, "rows_free": 2}
+    return explore((producer, *[rows] * loaders, issuer, sums), sizes, {"rows_full": loaders})
+
+
+@pytest.mark.parametrize("items, blocks, stages", [([0], 1, 2), ([0, 0, 0], 2, 2), ([0, 1, 2, 3, 4], 1, 2), ([0, 0, 1, 2, 2, 3], 2, 3), ([3, 4, 4, 4, 5, 6], 1, 8)])
+def test_no_interleaving_of_the_few_rows_protocol_within_a_cta_goes_wrong(items, blocks, stages):
+    n = NUMBERS["grouped_few"]
+    assert n["max_inner"] == ops.FEW_MAX_INNER and n["row_buffers"] == 2 and 2 <= stages <= n["max_stages"]
+    assert few_rows_cta(items, blocks, stages, n["accumulators"], n["loader_warps"]) is None
+
+
+def few_rows_cluster(items, ranks, warps, buffers):
+    """Every summing warp of every CTA, item after item: write its sums into each CTA's buffer, announce them there, wait for all of them in its own CTA,
+    read.  Writing while a warp of the CTA written to has yet to read what stood in that buffer is what must not happen."""
+    roles = []
+    for r in range(ranks):
+        for _ in range(warps):
+            role = []
+            for n in range(items):
+                b, use = n % buffers, n // buffers
+                if use > 0:
+                    role += [("must", f"read{q}", b, use - 1) for q in range(ranks)]
+                role += [("arrive", f"parts{q}", b) for q in range(ranks)]
+                role += [("wait", f"parts{r}", b, use), ("arrive", f"read{r}", b)]
+            roles.append(role)
+    sizes = {f"{kind}{q}": buffers for kind in ("parts", "read") for q in range(ranks)}
+    return explore(tuple(roles), sizes, {**{f"parts{q}": ranks * warps for q in range(ranks)}, **{f"read{q}": warps for q in range(ranks)}})
+
+
+@pytest.mark.parametrize("items, ranks, warps", [(1, 4, 1), (4, 2, 2), (5, 3, 1), (7, 2, 1)])
+def test_no_interleaving_of_the_few_rows_protocol_between_ctas_goes_wrong(items, ranks, warps):
+    assert NUMBERS["grouped_few"]["ranks"] >= ranks
+    assert few_rows_cluster(items, ranks, warps, NUMBERS["grouped_few"]["sum_buffers"]) is None
+
+
+def test_the_few_rows_sums_need_two_buffers():
+    assert "goes on without" in few_rows_cluster(3, 2, 1, 1)
 
 
 def gated_drain(tiles, gives_up, vote):
