@@ -38,11 +38,6 @@ struct FewParams {
     GluRule glu;
 };
 
-__device__ __forceinline__ uint32_t at_rank(uint32_t addr, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    return remote;
-}
 __device__ __forceinline__ void arrive_at_rank(uint32_t bar, uint32_t rank) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at_rank(bar, rank)) : "memory");
 }

@@ -208,7 +208,7 @@ __device__ __forceinline__ bool umma_block_looking_ahead(uint32_t tmem_d, uint64
     return seen != 0;
 }
 // ---- the same for a pair of CTAs (cta_group::2): the even CTA's barriers, and MMAs that both SMs work on ------------------------
-constexpr uint32_t EVEN_CTA = 0xFEFFFFFFu;      // an address of this CTA's shared memory, turned to the pair's even CTA
+// (an `even` barrier is one of the even CTA's, by its address in the cluster)
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t even_bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -216,9 +216,9 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 }
 // tma_stage_looking_ahead of one CTA of a pair: its rows of both operands, counted at the even CTA's barrier, which the even CTA arms with both
 // CTAs' bytes (`arm`).
-__device__ __forceinline__ bool tma_pair_stage_looking_ahead(uint32_t bar, uint32_t arm, uint32_t bytes, uint32_t a_dst, const CUtensorMap* map_a, int x,
-                                                             int ay, uint32_t b_dst, const CUtensorMap* map_b, int by, uint32_t next_bar,
-                                                             uint32_t next_parity) {
+__device__ __forceinline__ bool tma_pair_stage_looking_ahead(uint32_t bar, uint32_t arm, uint32_t bytes, uint32_t even_bar, uint32_t a_dst,
+                                                             const CUtensorMap* map_a, int x, int ay, uint32_t b_dst, const CUtensorMap* map_b, int by,
+                                                             uint32_t next_bar, uint32_t next_parity) {
     uint32_t seen;
     asm volatile(
         "{\n\t.reg .pred look, even;\n\t"
@@ -230,7 +230,7 @@ __device__ __forceinline__ bool tma_pair_stage_looking_ahead(uint32_t bar, uint3
         "selp.u32 %0, 1, 0, look;\n\t}"
         : "=r"(seen)
         : "r"(bar), "r"(arm), "r"(bytes), "r"(a_dst), "l"((uint64_t)map_a), "r"(x), "r"(b_dst), "l"((uint64_t)map_b), "r"(by), "r"(next_bar),
-          "r"(next_parity), "r"(bar & EVEN_CTA), "r"(ay)
+          "r"(next_parity), "r"(even_bar), "r"(ay)
         : "memory");
     return seen != 0;
 }
@@ -258,8 +258,8 @@ __device__ __forceinline__ bool umma_pair_block_looking_ahead(uint32_t tmem_d, u
         : "memory");
     return seen != 0;
 }
-__device__ __forceinline__ void mbar_arrive_even(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar & EVEN_CTA) : "memory");
+__device__ __forceinline__ void mbar_arrive_even(uint32_t even_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(even_bar) : "memory");
 }
 __device__ __forceinline__ void umma_pair_commit(uint32_t bar) {      // the barrier at this place in both CTAs
     asm volatile(
@@ -954,6 +954,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     const int stages = p.stages;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES]);
     const uint32_t acc_full0 = smem_u32(&bars[2 * MAX_STAGES]), acc_empty0 = acc_full0 + 16;
+    const uint32_t even_full0 = PAIR ? at_rank(full0, 0) : full0, even_acc_empty0 = PAIR ? at_rank(acc_empty0, 0) : acc_empty0;
     volatile int* abort_flag = &abort_s;
     const int num_k_blocks = (p.K + BLOCK_K - 1) / BLOCK_K;
     int tiles_m = (p.T + TILE_ROWS - 1) / TILE_ROWS;
@@ -1018,9 +1019,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 if (first) {
                     if constexpr (PAIR) {
                         if (rank == 0) mbar_expect_tx(bar, 2 * STAGE_BYTES);
-                        tma_load_2d_pair(b_dst, &map_b, bar & EVEN_CTA, k, b_row0);
+                        tma_load_2d_pair(b_dst, &map_b, even_full0 + 8 * s, k, b_row0);
                         pdl_wait();
-                        tma_load_2d_pair(a_dst, &map_a, bar & EVEN_CTA, k, a_row0);
+                        tma_load_2d_pair(a_dst, &map_a, even_full0 + 8 * s, k, a_row0);
                     } else {
                         mbar_expect_tx(bar, STAGE_BYTES);
                         tma_load_2d(b_dst, &map_b, bar, k, b_row0);
@@ -1033,8 +1034,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 } else {
                     bool seen;
                     if constexpr (PAIR)
-                        seen = tma_pair_stage_looking_ahead(bar, rank == 0 ? 1u : 0u, 2 * STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, b_row0,
-                                                            empty0 + 8 * s_next, (round_next & 1) ^ 1);
+                        seen = tma_pair_stage_looking_ahead(bar, rank == 0 ? 1u : 0u, 2 * STAGE_BYTES, even_full0 + 8 * s, a_dst, &map_a, k, a_row0,
+                                                            b_dst, &map_b, b_row0, empty0 + 8 * s_next, (round_next & 1) ^ 1);
                     else
                         seen = tma_stage_looking_ahead(bar, STAGE_BYTES, a_dst, &map_a, k, a_row0, b_dst, &map_b, k, b_row0,
                                                        b_dst + B_TILE_BYTES / 2, p.N + b_row0, SPLIT_B ? 1u : 0u,
@@ -1210,7 +1211,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             // this thread (a pair's: this warp) has taken its row out of the accumulator
             if constexpr (PAIR) {
                 __syncwarp();
-                if (lane == 0) mbar_arrive_even(acc_empty0 + 8 * buf);
+                if (lane == 0) mbar_arrive_even(even_acc_empty0 + 8 * buf);
             } else mbar_arrive(acc_empty0 + 8 * buf);
         }
     }
