@@ -954,7 +954,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     const int stages = p.stages;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[MAX_STAGES]);
     const uint32_t acc_full0 = smem_u32(&bars[2 * MAX_STAGES]), acc_empty0 = acc_full0 + 16;
-    const uint32_t even_full0 = PAIR ? at_rank(full0, 0) : full0, even_acc_empty0 = PAIR ? at_rank(acc_empty0, 0) : acc_empty0;
     volatile int* abort_flag = &abort_s;
     const int num_k_blocks = (p.K + BLOCK_K - 1) / BLOCK_K;
     int tiles_m = (p.T + TILE_ROWS - 1) / TILE_ROWS;
@@ -1001,6 +1000,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         // were issued (the stages of the first round are free anyway).
         uint32_t s = 0, round = 0;
         bool first = true, looked = true;
+        const uint32_t even_full0 = PAIR ? at_rank(full0, 0) : full0;
         if (!PAIR && p.tile_group) pdl_wait();   // which weights a tile meets was written by the kernel before
         for (int tile = unit; tile < num_tiles && !*abort_flag; tile += units) {
             const int a_row0 = (tile % tiles_m) * TILE_ROWS + rank * TILE_M;
@@ -1211,7 +1211,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             // this thread (a pair's: this warp) has taken its row out of the accumulator
             if constexpr (PAIR) {
                 __syncwarp();
-                if (lane == 0) mbar_arrive_even(even_acc_empty0 + 8 * buf);
+                if (lane == 0) mbar_arrive_even(at_rank(acc_empty0 + 8 * buf, 0));
             } else mbar_arrive(acc_empty0 + 8 * buf);
         }
     }
