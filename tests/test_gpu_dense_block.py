@@ -17,9 +17,9 @@ def _weights(h, nh, nkv, f, gen):
             "d": m(h, f), "n1": g(h), "n2": g(h)}
 
 
-@pytest.mark.parametrize("news, past", [([61], [0]), ([129], [0]), ([300, 7, 64], [0, 33, 100]), ([1000], [70])])
-@pytest.mark.parametrize("h, nh, nkv, f, window, rope, qk_norm", [(1024, 8, 2, 2816, 0, 128, True), (512, 4, 4, 1000, 50, 0, False), (512, 4, 1, 520, 0, 128, True)])
-def test_one_call_is_the_parts_one_by_one(news, past, h, nh, nkv, f, window, rope, qk_norm):
+def _compare(monkeypatch, news, past, h, nh, nkv, f, window, rope, qk_norm, taken):
+    """A block's step twice over (the second takes what the first has prepared), by its parts and as `dense` allows it; `taken`: whether the one
+    call is to launch it.  Launches of the two ways."""
     from hymt2sharp_b200.cache import PagedCache
     from hymt2sharp_b200.engine.engine import StepEntry, make_context
     from hymt2sharp_b200.parts import MixerSlot, PartSpec, build_part
@@ -39,7 +39,9 @@ def test_one_call_is_the_parts_one_by_one(news, past, h, nh, nkv, f, window, rop
     T = sum(news)
     start = torch.randn(T, h, generator=gen, device=DEV)
     filling = torch.randn(1, generator=gen, device=DEV)
-    results, launches = [], []
+    results, launches, calls = [], [], []
+    launch = ops.dense_block
+    monkeypatch.setattr(ops, "dense_block", lambda *args: (calls.append(1), launch(*args)))
     for whole in (False, True):
         cache = PagedCache([need], torch.bfloat16, DEV, 4096, max_slots=len(news), max_sequence_tokens=2048)
         slots = cache.alloc_slots(len(news))
@@ -63,9 +65,24 @@ def test_one_call_is_the_parts_one_by_one(news, past, h, nh, nkv, f, window, rop
                 left = (ctx.prenormed.normed.clone(), ctx.prenormed.ss.clone()) if ctx.prenormed is not None else ()
         assert ctx.prenormed is None
         launches.append(ops.launches - before)
+        assert len(calls) == (2 if whole and taken else 0)
         results.append((residual, *left, *[s.clone() for s in cache.storage]))
-    assert launches[0] == launches[1] or T <= 128
     assert len(results[0]) == len(results[1])
     for a, b in zip(*results):
         assert torch.equal(a, b)
     assert ops.device_status(torch.device(DEV))[0].item() == 0
+    return launches
+
+
+@pytest.mark.parametrize("news, past", [([61], [0]), ([129], [0]), ([300, 7, 64], [0, 33, 100]), ([1000], [70])])
+@pytest.mark.parametrize("h, nh, nkv, f, window, rope, qk_norm", [(1024, 8, 2, 2816, 0, 128, True), (512, 4, 4, 1000, 50, 0, False), (512, 4, 1, 520, 0, 128, True)])
+def test_one_call_is_the_parts_one_by_one(monkeypatch, news, past, h, nh, nkv, f, window, rope, qk_norm):
+    parts, whole = _compare(monkeypatch, news, past, h, nh, nkv, f, window, rope, qk_norm, taken=True)
+    assert parts == whole
+
+
+@pytest.mark.parametrize("news, f, rope", [([61], 1002, 128), ([300], 1002, 128), ([300], 1000, 48)])
+def test_what_the_one_call_does_not_take_goes_through_the_parts(monkeypatch, news, f, rope):
+    """An inner width that is no multiple of 8; heads rotated in part beyond 128 tokens."""
+    parts, whole = _compare(monkeypatch, news, [0], 512, 4, 2, f, 0, rope, True, taken=False)
+    assert parts == whole
