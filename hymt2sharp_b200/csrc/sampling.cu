@@ -374,12 +374,15 @@ struct FilterParams {
 // passes, a barrier of the row's blocks behind each.  120,818 logits, 8 rows: with top-p alone 57 us (one block a row: 317), with
 // min-p alone 13 (32).
 //
-// A top-k of up to FEW entries with min-p or top-p behind it needs one pass over the bins, of the threads' largest keys alone: the
-// lower edge of the bin that holds the k-th largest of them cannot lie above the k-th largest key of the row.  What reaches that
-// edge (a few more than k entries, as a rule) goes to the first block, which ranks it, keeps k, settles min-p and top-p and, asked
-// to, draws the token as the kernels above would.  With more than FEW such entries the row goes the long way.  120,818 logits, 8 rows,
-// top-k 20, top-p and penalty: 20 us with the draw; three passes over all keys took 25 us, and the draw's own pass over the row 20 more.
-constexpr int FEW = 1024, BINS = 2048;
+// A top-k of up to QUICK entries with min-p or top-p behind it needs one pass over the bins, of the threads' largest keys alone: the
+// lower edge of the bin that holds the k-th largest of them cannot lie above the k-th largest key of the row.  Where many of them crowd that
+// bin (logits far from zero: a bin is a quarter of an octave), it is cut into bins of its own.  What reaches the edge (a few more than k
+// entries, as a rule) goes to the first block, which ranks it, keeps k, settles min-p and top-p and, asked to, draws the token as the kernels
+// above would.  With more than FEW such entries, as with a larger k, the row goes the long way, and the first block gets its k entries.
+// 120,818 logits, top-k + top-p, us with the argmax and sampling kernels behind it, three passes over all keys and a draw over the row / this: 8 rows,
+// k = 20 47 / 21, k = 100 50 / 24, k = 512 62 / 36; the same around 20 instead of 0 48 / 23, 50 / 24, 62 / 36; 64 rows 112 / 53, 120 / 61, 160 / 105.
+// The ranking costs 32 cycles an entry where all warps run it, so only those with an entry do.
+constexpr int FEW = 1024, BINS = 2048, QUICK = 512, CROWD = 128;
 
 struct FilterShared {
     int hist[BINS];              // this block's counts (or masses, as floats)
@@ -395,7 +398,7 @@ struct FilterShared {
     float floats[CLUSTER];
     int total_i, bin, need, n_few;
     float total_f, above, u;
-    int owner, last;
+    int owner, last, upto;       // (upto: the first threads, of which some hold a survivor)
 };
 
 template <typename V> __device__ __forceinline__ V* bins_of(FilterShared& s) { return reinterpret_cast<V*>(s.hist); }
@@ -453,7 +456,8 @@ __device__ __forceinline__ void find_bin(FilterShared& s, int bins, int remainin
     __syncthreads();
 }
 
-// The token of a row of which `kept` of the first block's threads hold one survivor each: its value v = logit * inv_t and its index.
+// The token of a row of which `kept` of the first block's threads hold one survivor each: its value v = logit * inv_t
+// and its index.  (s.upto is 0.)
 // What sample_kernel makes of the row with everything else at -inf, bit for bit: its pieces' sums hold the same terms in the order
 // of their indices, and zeros.  False (nothing drawn): a value is not finite.
 __device__ __forceinline__ bool draw_from(FilterShared& s, const FilterParams& p, int row, int srow, bool kept, float v, int index) {
@@ -470,10 +474,12 @@ __device__ __forceinline__ bool draw_from(FilterShared& s, const FilterParams& p
         s.owner = 0x7fffffff;
         s.last = -1;
     }
+    const uint32_t mine = __ballot_sync(0xffffffffu, kept);
+    if ((tid & 31) == 0 && mine) atomicMax(&s.upto, tid + 32 - __clz(mine));
     const int n = __syncthreads_count(kept);
     int place = 0;
     if (kept)
-        for (int j = 0; j < FEW && j < s.n_few; j++) place += s.at[j] < index;
+        for (int j = 0; j < s.upto; j++) place += s.at[j] < index;
     __syncthreads();
     if (kept) {
         s.sorted[place] = pr;
@@ -487,6 +493,7 @@ __device__ __forceinline__ bool draw_from(FilterShared& s, const FilterParams& p
             float part = 0.f;
             for (int j = tid; j < n && s.order[j] / piece == mine; j++) part += s.sorted[j];
             s.parts[mine] = part;
+            s.hist[mine] = tid;      // where the piece's survivors begin
         }
     }
     __syncthreads();
@@ -499,8 +506,8 @@ __device__ __forceinline__ bool draw_from(FilterShared& s, const FilterParams& p
     if (tid == s.owner) {
         float acc = before;
         int pick = -1, last = -1;
-        for (int j = 0; j < n; j++) {
-            if (s.order[j] / piece != tid || s.sorted[j] <= 0.f) continue;
+        for (int j = s.hist[tid]; j < n && s.order[j] / piece == tid; j++) {
+            if (s.sorted[j] <= 0.f) continue;
             last = s.order[j];
             acc += s.sorted[j];
             if (acc >= r) { pick = last; break; }
@@ -518,9 +525,9 @@ __device__ __forceinline__ void settle_few(FilterShared& s, const FilterParams& 
     const int tid = threadIdx.x;
     // ranks by key, ties by index; the mass before an entry is then a scan
     const unsigned long long mine = tid < n ? s.few[tid] : 0ull;
-    int place = 0;
-    for (int j = 0; j < n; j++) place += s.few[j] > mine;
-    if (tid < n) {
+    if (tid < n) {                    // (the warps without an entry stay out of the loop, which they would slow)
+        int place = 0;
+        for (int j = 0; j < n; j++) place += s.few[j] > mine;
         const int i = (int)~(uint32_t)mine;
         if (place < k) {
             s.sorted[place] = x[i] * inv_t;
@@ -543,8 +550,9 @@ __device__ __forceinline__ void settle_few(FilterShared& s, const FilterParams& 
     }
 }
 
-template <int BLOCKS>
-__global__ void __launch_bounds__(THREADS, 1)
+// RESIDENT: the blocks that are to share an SM.  One has 64 registers a thread and more loads in flight, two have 32.
+template <int BLOCKS, int RESIDENT>
+__global__ void __launch_bounds__(THREADS, RESIDENT)
 filter_kernel(FilterParams p) {
     __shared__ FilterShared s;
     const RowBlocks<BLOCKS> blocks;
@@ -584,45 +592,65 @@ filter_kernel(FilterParams p) {
     if (!(inv_t > 0.f)) return;  // greedy: temperature 0 bypasses every other field (Sampling.cs:81-84)
     const int k = p.top_k ? p.top_k[srow] : 0;
     const float top_p = p.top_p ? p.top_p[srow] : 1.f, min_p = p.min_p ? p.min_p[srow] : 0.f;
-    if (tid == 0) s.n_few = 0;
+    if (tid == 0) s.n_few = s.upto = 0;
     blocks.sync();     // every block of the row runs: its shared memory may be written to (the returns above are the whole row's)
     const bool by_mass = top_p < 1.f || min_p > 0.f;
     const bool by_rank = k > 0 && k < vocab, few = by_rank && k <= FEW && by_mass;
 
-    if (few) {
+    if (few && k <= QUICK) {
         // a lower edge of the k-th largest key, from the threads' largest
         for (int i = tid; i < BINS; i += THREADS) s.hist[i] = 0;
+        const bool any = begin + tid < end;
         uint32_t largest = 0;
 #pragma unroll 8
         for (int i = begin + tid; i < end; i += THREADS) largest = max(largest, float_key(x[i] * inv_t));
         __syncthreads();
-        if (begin + tid < end) atomicAdd(&s.hist[largest >> 21], 1);
+        if (any) atomicAdd(&s.hist[largest >> 21], 1);
         gather_bins<int>(blocks, s, BINS);
-        if (tid == 0) s.bin = 0;                    // (fewer threads than k hold an entry: everything reaches the edge)
+        if (tid == 0) s.bin = -1;                   // (fewer threads than k hold an entry: everything reaches the edge)
         __syncthreads();
         find_bin(s, BINS, k);
-        const uint32_t edge = (uint32_t)s.bin << 21, lowest = float_key(-INFINITY);
-        int* n_few = blocks.of(&s.n_few, 0);
-        unsigned long long* list = blocks.of(s.few, 0);
-        // what lies below the edge is dropped whichever way the row goes on
+        uint32_t edge = 0;
+        int reach = 0;                              // how many of the threads' largest reach it
+        if (s.bin >= 0) {
+            const int bin = s.bin, need = s.need, crowd = s.total[bin];
+            edge = (uint32_t)bin << 21;
+            reach = k - need + crowd;
+            if (crowd > CROWD) {                    // the bin is cut into bins of its own
+                __syncthreads();
+                for (int i = tid; i < BINS; i += THREADS) s.hist[i] = 0;
+                __syncthreads();
+                if (any && largest >> 21 == (uint32_t)bin) atomicAdd(&s.hist[(largest >> 10) & (BINS - 1)], 1);
+                gather_bins<int>(blocks, s, BINS);
+                find_bin(s, BINS, need);
+                edge |= (uint32_t)s.bin << 10;
+                reach = k - s.need + s.total[s.bin];
+            }
+        }
+        if (reach <= FEW) {                         // (the same in all blocks of the row)
+            const uint32_t lowest = float_key(-INFINITY);
+            int* n_few = blocks.of(&s.n_few, 0);
+            unsigned long long* list = blocks.of(s.few, 0);
+            // what lies below the edge is dropped whichever way the row goes on
 #pragma unroll 8
-        for (int i = begin + tid; i < end; i += THREADS) {
-            const uint32_t key = float_key(x[i] * inv_t);
-            if (key < edge) x[i] = -INFINITY;
-            else if (key > lowest) {
-                const int at = atomicAdd(n_few, 1);
-                if (at < FEW) list[at] = (unsigned long long)key << 32 | (uint32_t)~i;
-            } else x[i] = -INFINITY;
+            for (int i = begin + tid; i < end; i += THREADS) {
+                const uint32_t key = float_key(x[i] * inv_t);
+                if (key < edge) x[i] = -INFINITY;
+                else if (key > lowest) {
+                    const int at = atomicAdd(n_few, 1);
+                    if (at < FEW) list[at] = (unsigned long long)key << 32 | (uint32_t)~i;
+                } else x[i] = -INFINITY;
+            }
+            blocks.sync();
+            const int n = *n_few;
+            if (n <= FEW) {
+                if (rank == 0) settle_few(s, p, row, srow, x, inv_t, n, k, top_p, min_p);
+                blocks.sync();     // (the first block stays until the others have read its count)
+                return;
+            }
+            blocks.sync();         // (everyone has read the count)
+            if (rank == 0 && tid == 0) s.n_few = 0;
         }
-        blocks.sync();
-        const int n = *n_few;
-        if (n <= FEW) {
-            if (rank == 0) settle_few(s, p, row, srow, x, inv_t, n, k, top_p, min_p);
-            blocks.sync();     // (the first block stays until the others have read its count)
-            return;
-        }
-        blocks.sync();         // (everyone has read the count)
-        if (rank == 0 && tid == 0) s.n_few = 0;
     }
 
     if (by_rank) {
@@ -864,6 +892,13 @@ HYMT2_API int hymt2_filter_blocks(int rows, int vocab) {
     return vocab >= 8192 && rows <= vocab / 400 && (rows <= 64 || rows <= vocab / 2000) ? CLUSTER : 1;
 }
 
+// Blocks of the filters that share an SM: one as long as all of them find an SM of their own, beyond that two.  A cluster lies within a processing
+// cluster of the chip, and 14 clusters of eight fit with an SM a block, not 16.  120,818 logits, top-k 20 with top-p and the draw, us with one and two:
+// 8 rows 20.8 21.0, 14 rows 23.0 23.7, 16 rows 37 24, 64 rows 107 53; top-p alone, 64 rows 320 and 229.
+HYMT2_API int hymt2_filter_resident(int rows, int vocab) {
+    return rows <= (hymt2_filter_blocks(rows, vocab) == CLUSTER ? 14 : 148) ? 1 : 2;
+}
+
 HYMT2_API int hymt2_sample(int* out, const float* logits, long row_stride, int rows, int vocab,
                            const float* inv_temperature, uint64_t* rng_states, const int* row_map, const int* drawn,
                            cudaStream_t stream) {
@@ -893,7 +928,13 @@ HYMT2_API int hymt2_filter_logits(float* logits, long row_stride, int rows, int 
     FilterParams p{logits, row_stride, vocab, inv_temperature, top_k, top_p, min_p, penalty, history,
                    history_stride, row_map, out, rng_states, drawn};
     HYMT2_REQUIRE(!drawn || (out && rng_states), "filter: a draw needs the tokens' place and the random streams");
-    if (hymt2_filter_blocks(rows, vocab) == CLUSTER) launch_clusters(filter_kernel<CLUSTER>, rows, 0, stream, p);
-    else launch_pdl(filter_kernel<1>, dim3(rows), dim3(THREADS), 0, stream, p);
+    const bool cluster = hymt2_filter_blocks(rows, vocab) == CLUSTER;
+    if (hymt2_filter_resident(rows, vocab) == 1) {
+        if (cluster) launch_clusters(filter_kernel<CLUSTER, 1>, rows, 0, stream, p);
+        else launch_pdl(filter_kernel<1, 1>, dim3(rows), dim3(THREADS), 0, stream, p);
+    } else {
+        if (cluster) launch_clusters(filter_kernel<CLUSTER, 2>, rows, 0, stream, p);
+        else launch_pdl(filter_kernel<1, 2>, dim3(rows), dim3(THREADS), 0, stream, p);
+    }
     return hymt2_check_launch("filter_logits");
 }

@@ -950,6 +950,11 @@ def filter_blocks(rows: int, vocab: int) -> int:
     return int(_lib().hymt2_filter_blocks(c_int(rows), c_int(vocab)))
 
 
+def filter_resident(rows: int, vocab: int) -> int:
+    """Blocks of the filters that share an SM.  Works without a GPU."""
+    return int(_lib().hymt2_filter_resident(c_int(rows), c_int(vocab)))
+
+
 def filter_logits(logits: torch.Tensor, inv_temperature: torch.Tensor, top_k: torch.Tensor | None,
                   top_p: torch.Tensor | None, min_p: torch.Tensor | None, penalty: torch.Tensor | None,
                   history: torch.Tensor | None, row_map: torch.Tensor | None = None, draw: tuple | None = None) -> None:

@@ -50,3 +50,27 @@ def test_a_draw_on_the_way_is_the_draw_behind(vocab, k, top_p, min_p):
         assert drawn[0] == 1 and drawn[1] == 1 and drawn[4] == 0
     else:
         assert not any(drawn)
+
+
+@pytest.mark.parametrize("rows, vocab", [(3, 9000), (20, 9000), (3, 3000), (160, 3000)])
+@pytest.mark.parametrize("k", [1, 50, 512, 513, 1024])
+@pytest.mark.parametrize("form", ["around zero", "far from zero", "on a grid", "flat", "few finite"])
+def test_a_top_k_keeps_the_k_largest_whichever_way_it_goes(rows, vocab, k, form):
+    """One block a row and eight, one block an SM and two; with the threads' largest spread over their bins, crowding one of them, and equal."""
+    ops = _ops()
+    torch.manual_seed(rows + k)
+    x = torch.randn(rows, vocab, device=DEV)
+    if form == "far from zero":
+        x = x + 40
+    elif form == "on a grid":
+        x = (x * 8).round() / 8 + 40
+    elif form == "flat":
+        x = torch.full_like(x, -3.0)
+    elif form == "few finite":
+        x[:, 700:] = -math.inf
+    f32 = lambda v: torch.full((rows,), v, device=DEV)
+    y, top_k = x.clone(), torch.full((rows,), k, dtype=torch.int32, device=DEV)
+    ops.filter_logits(y, f32(1.0), top_k, f32(1.0), f32(1e-38), None, None)      # (a min-p that drops nothing here)
+    order = torch.sort(x, dim=1, descending=True, stable=True).indices[:, :k]    # ties in index order
+    want = torch.full_like(x, -math.inf).scatter(1, order, x.gather(1, order))
+    assert torch.equal(y, want)

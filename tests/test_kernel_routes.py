@@ -14,6 +14,11 @@ def test_rows_are_filtered_and_drawn_by_one_block_where_a_cluster_would_be_slowe
     assert (ops.filter_blocks(rows, vocab), ops.sample_blocks(rows, vocab)) == (filters, draw)
 
 
+@pytest.mark.parametrize("rows, vocab, resident", [(1, 120818, 1), (14, 120818, 1), (15, 120818, 2), (64, 120818, 2), (64, 5000, 1), (148, 5000, 1), (149, 5000, 2)])
+def test_blocks_of_the_filters_share_an_sm_where_they_would_wait_for_one(rows, vocab, resident):
+    assert ops.filter_resident(rows, vocab) == resident
+
+
 @pytest.mark.parametrize("rows, columns, epilogue, narrow, kernel", [
     (129, 2048, 0, True, "64x64 short"), (300, 1000, 0, True, "64x64 short"), (600, 500, 0, True, "64x64 short"), (1, 8192, 0, True, "64x64 short"),
     (129, 4096, 2, True, "64x64"), (64, 9472, 0, True, "64x64 short"), (64, 9473, 0, True, "64x128"), (531, 6144, 2, True, "64x128"),
