@@ -1731,16 +1731,17 @@ def gemm_grouped(kernel: str, out: torch.Tensor, a: torch.Tensor, w: torch.Tenso
                "gemm_tc_grouped")
 
 
-# The grouped product of few rows goes to the tensor cores from this many weight entries on that a step may touch (pairs of token and choice
-# times a matrix's entries): below, the start of its clusters is longer than the reading.  us, CUDA cores / tensor cores: 4.2 M entries 4.1 6.6
-# and 7.3 6.9; 8.4 M 7.3 7.3 and 6.6 9.3; 16.8 M 12.4 9.8, 12.3 9.7 and 13.6 11.2; 67 M 36 27 and 40 27; 134 M 53 33.
+# The grouped product of few rows goes to the tensor cores where its largest step touches this many weight entries (pairs of token and choice
+# times a matrix's entries, every expert once at most).  A single token of small experts pays for its clusters' start, a few tokens gain.  us of
+# both products, CUDA cores and tensor cores, 1 / 4 / 16 tokens, top 2 of 32 experts (gate and up as one matrix): 1.05 M entries a matrix 8.5 11.3 /
+# 16 15 / 36 25; 2.1 M 13.8 14.2 / 27 20 / 64 41; 4.2 M 18.3 15.7 / 40 29 / 112 65; top 4 of 4.2 M 27 20 / 64 47 / 166 80.
 FEW_MIN_ENTRIES = 12 << 20
 FEW_MAX_INNER = 4096           # (csrc/gemm_grouped_few.cu: MAX_K)
 
 
 def gemm_grouped_few_supported(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
-    """Whether `pairs` (token, choice) pairs' grouped product runs on the tensor cores in tiles of 8 rows: bfloat16, rows on 16 bytes, the
-    inner size a multiple of 256 up to 4,096, and enough of the matrices in use to be worth it."""
+    """Whether the grouped product of steps of up to `pairs` (token, choice) pairs runs on the tensor cores in tiles of 8 rows: bfloat16, rows
+    on 16 bytes, the inner size a multiple of 256 up to 4,096, and enough of the matrices in use in the largest to be worth it."""
     K = a.shape[1]
     return a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 256 == 0 and K <= FEW_MAX_INNER and a.stride(1) == 1 and a.stride(0) % 8 == 0 \
         and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous() and min(pairs, w.shape[0]) * w.shape[1] * K >= FEW_MIN_ENTRIES

@@ -164,9 +164,10 @@ class RoutedExperts:
         if kernel == "tc":     # its tiles come by TMA, which reads rows side by side
             rows, gather = torch.empty((tiles * tile, self.hidden), dtype=x.dtype, device=dev), False
             ops.moe_gather(rows, x, row_token)
-        # (one rule for both products: tiles of 8 rows go where the reading is worth the start)
+        # (one rule for both products, and for every step that comes here: asked about the largest of them, so that a token's bits do not
+        # hang on how many others its step has)
         few = kernel == "skinny" and self.intermediate % 256 == 0 and self.intermediate <= ops.FEW_MAX_INNER \
-            and ops.gemm_grouped_few_supported(x, self.up, T * self.top)
+            and ops.gemm_grouped_few_supported(x, self.up, SKINNY_PAIRS_BESIDE_TC)
         grouped = ops.gemm_grouped_few if few else lambda *args: ops.gemm_grouped(kernel, *args)
         ops.tag = "experts_up"
         if self.gated and self.activation in ("silu", "clamped") and kernel != "simt":

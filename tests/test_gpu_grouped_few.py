@@ -79,3 +79,29 @@ def test_what_the_kernel_of_few_rows_does_not_take_goes_to_the_cuda_cores():
     assert not ops.gemm_grouped_few_supported(a.float(), w.float(), 64)
     assert not ops.gemm_grouped_few_supported(a[:, :500], w[:, :, :500].contiguous(), 64)
     assert not ops.gemm_grouped_few_supported(a, w, 8)                       # too little to read
+
+
+@pytest.mark.parametrize("hidden, ff, experts, top", [(2048, 1024, 8, 2), (1024, 512, 16, 2), (512, 256, 8, 2)])
+def test_a_token_of_a_mixture_does_not_depend_on_the_size_of_its_step(hidden, ff, experts, top):
+    """Steps of up to 64 (token, choice) pairs: the rule that picks their kernel hangs on the weights alone."""
+    from hymt2sharp_b200.parts import PartSpec, build_part
+    ops = _ops()
+    torch.manual_seed(hidden)
+    bf = torch.bfloat16
+    part = build_part("feed_forward", PartSpec("routed_experts", dict(hidden=hidden, experts=experts, identity=0, top=top, intermediate=ff, activation="silu",
+                                                                      router="r", gate_proj="{}.g", up_proj="{}.u", down_proj="{}.d")))
+    m = lambda r, c: (torch.randn(r, c, device=DEV) / math.sqrt(c)).to(bf)
+    weights = {"r": m(experts, hidden)}
+    for e in range(experts):
+        weights.update({f"{e}.g": m(ff, hidden), f"{e}.u": m(ff, hidden), f"{e}.d": m(hidden, ff)})
+    part.load(weights, DEV, bf)
+    x = torch.randn(32, hidden, device=DEV).to(bf)
+
+    def rows(n):
+        y, pair_row, _, _ = part._experts(x[:n].contiguous(), None)
+        return y[pair_row.long()]
+
+    whole = rows(32)
+    for n in (1, 2, 5, 6, 11, 31):
+        assert torch.equal(rows(n), whole[:n]), n
+    assert ops.device_status(torch.device(DEV))[0].item() == 0
