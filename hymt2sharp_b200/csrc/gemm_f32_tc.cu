@@ -152,13 +152,6 @@ __device__ __forceinline__ bool mbar_wait_both(uint32_t a, uint32_t parity_a, ui
         : "=r"(both) : "r"(a), "r"(parity_a), "r"(b), "r"(parity_b) : "memory");
     return both || (mbar_wait(a, parity_a, abort_flag, status, code) && mbar_wait(b, parity_b, abort_flag, status, code));
 }
-// Whether `mine` is true in all 128 threads that meet at named barrier `id`.
-__device__ __forceinline__ bool all_of_group(int id, bool mine) {
-    uint32_t all;
-    asm volatile("{\n\t.reg .pred in, out;\n\tsetp.ne.u32 in, %2, 0;\n\tbar.red.and.pred out, %1, 128, in;\n\tselp.u32 %0, 1, 0, out;\n\t}"
-                 : "=r"(all) : "r"(id), "r"((uint32_t)mine) : "memory");
-    return all != 0;
-}
 template <int REGS> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 template <int REGS> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
 // Registers of a thread by what its warp does: with tiles of 64 tokens the drain holds 64 sums a thread.  A block is launched with 768 threads
@@ -421,12 +414,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         pdl_wait();       // C may still be in use by the kernel in front
         uint32_t i = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < tiles && ok; tile += stride) {
+        constexpr bool MEETS = PLANES && EPI == EPI_SWIGLU;
+        for (int tile = first_tile; tile < tiles; tile += stride) {
             float acc[OWN], total[PLANES ? OWN : 1];
 #pragma unroll
             for (int j = 0; j < OWN; j++) acc[j] = 0.f;
             int in_part = 0, part = 0;
-            for (int c = 0; c < chunks; c++, i++) {
+            for (int c = 0; c < chunks && (ok || !MEETS); c++, i++) {
                 const int g = i & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(done0 + 8 * g, (i >> 1) & 1, abort_flag, p.status, 137));
                 if (!ok) break;
@@ -461,12 +455,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     in_part = 0;
                 }
             }
-            // A gated tile's group of four warps meets at a named barrier, which has no limit: whether it goes on is the whole group's decision, so
-            // that none stands there for a warp whose own wait gave up.  (Such a warp comes here too.)
-            if constexpr (PLANES && EPI == EPI_SWIGLU) ok = all_of_group(1 + share, ok);
-            if (!ok) break;
+            // (a gated tile's group of four warps meets at a named barrier, which has no limit: a warp whose own wait gave up goes there all the
+            // same, for this tile and all that follow, and stores nothing)
+            if (!ok && !MEETS) break;
             if constexpr (PLANES) {
-                const int m0 = tile_t(tile) + col0, cols = min(own, p.M - m0);
+                const int m0 = tile_t(tile) + col0, cols = MEETS && !ok ? 0 : min(own, p.M - m0);
                 if (part > 0) {
 #pragma unroll
                     for (int j = 0; j < OWN; j++) acc[j] = total[j] + acc[j];
@@ -724,7 +717,7 @@ inline bool rows_on_16(const void* A, long lda) { return (uintptr_t)A % 16 == 0 
 
 // The numbers of the kernel's barrier protocol: out[0] groups of converters and [1] buffers of pieces with up to 32 tokens, [2], [3] with tiles of 64,
 // [4], [5] with planes, [6] slots of planes, [7] 1: an issuer waits for its accumulator before it looks at the pieces,
-// [8] warps of a group of the gated drain, [9] 1: they vote on going on before they meet
+// [8] warps of a group of the gated drain, [9] 1: one whose wait gave up meets the others all the same
 HYMT2_API int hymt2_gemm_f32_tc_protocol(int* out) {
     out[0] = converters(false, 32); out[1] = buffers(false, 32); out[2] = converters(false, 64); out[3] = buffers(false, 64);
     out[4] = converters(true, PLANES_BN); out[5] = buffers(true, PLANES_BN); out[6] = PLANE_SLOTS; out[7] = 1;

@@ -676,7 +676,7 @@ def protocol_numbers() -> dict:
             "decode": ask("hymt2_attention_decode_tc_protocol", ("stages", "accumulators")),
             "gemm": ask("hymt2_gemm_tc_protocol", ("max_stages", "accumulators", "issuers", "issuers_own_stages", "epilogue_groups")),
             "f32": ask("hymt2_gemm_f32_tc_protocol", ("few_groups", "few_buffers", "wide_groups", "wide_buffers", "planes_groups", "planes_buffers",
-                                                      "plane_slots", "drained_first", "gated_warps", "gated_vote")),
+                                                      "plane_slots", "drained_first", "gated_warps", "gated_walks_on")),
             "grouped_few": ask("hymt2_gemm_grouped_few_protocol", ("ranks", "accumulators", "row_buffers", "loader_warps", "max_stages", "sum_buffers",
                                                                    "max_inner"))}
 

@@ -421,31 +421,20 @@ def test_the_few_rows_sums_need_two_buffers():
     assert "goes on without" in few_rows_cluster(3, 2, 1, 1)
 
 
-def gated_drain(tiles, gives_up, vote):
+def gated_drain(tiles, gives_up, walks_on):
     """The warps of a gated drain group, which meet twice a tile at a barrier that has no limit.  gives_up[w]: the tile in which warp w's bounded wait
-    gives up (None: never).  With `vote` all meet once more in front, and go on only if none has given up."""
-    roles, first = [], min((t for t in gives_up if t is not None), default=tiles)
+    gives up (None: never); with `walks_on` it meets the others in that tile and all that follow."""
+    roles = []
     for mine in gives_up:
-        role, phase = [], 0
-        for t in range(tiles):
-            out = mine is not None and t >= mine
-            if out and not vote:
-                break
-            for _ in range(3 if vote else 2):
-                role += [("arrive", "meet", 0), ("wait", "meet", 0, phase)]
-                phase += 1
-                if vote and t >= first:      # the vote's answer: they leave together
-                    break
-            if vote and t >= first:
-                break
-        roles.append(role)
+        meets = 2 * (tiles if mine is None or walks_on else mine)
+        roles.append([op for phase in range(meets) for op in (("arrive", "meet", 0), ("wait", "meet", 0, phase))])
     return explore(tuple(roles), {"meet": 1}, {"meet": len(gives_up)})
 
 
 @pytest.mark.parametrize("gives_up", [(None, None, None, None), (0, None, None, None), (None, 2, None, None), (1, 1, None, 2), (2, 2, 2, 2), (0, 1, 2, None)])
-def test_a_warp_that_gives_up_takes_its_gated_drain_group_along(gives_up):
+def test_a_warp_that_gives_up_still_meets_its_gated_drain_group(gives_up):
     n = NUMBERS["f32"]
-    assert n["gated_vote"] == 1 and n["gated_warps"] == len(gives_up)
-    assert gated_drain(3, gives_up, vote=True) is None
-    if len(set(gives_up)) > 1:      # without the vote, as it was: the others stand at the barrier for ever
-        assert "nothing can move" in gated_drain(3, gives_up, vote=False)
+    assert n["gated_walks_on"] == 1 and n["gated_warps"] == len(gives_up)
+    assert gated_drain(3, gives_up, walks_on=True) is None
+    if len(set(gives_up)) > 1:      # leaving, as it did: the others stand at the barrier for ever
+        assert "nothing can move" in gated_drain(3, gives_up, walks_on=False)
