@@ -152,6 +152,11 @@ __device__ __forceinline__ bool mbar_wait_both(uint32_t a, uint32_t parity_a, ui
         : "=r"(both) : "r"(a), "r"(parity_a), "r"(b), "r"(parity_b) : "memory");
     return both || (mbar_wait(a, parity_a, abort_flag, status, code) && mbar_wait(b, parity_b, abort_flag, status, code));
 }
+// The rest of a group's meetings, for a warp that has nothing more to bring.  (A call: inline it moved the drain's registers about, gate and up of 531
+// rows 154 -> 158 us.)
+__device__ __noinline__ void keep_meeting(int id, int times) {
+    for (int i = 0; i < times; i++) asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory");
+}
 template <int REGS> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 template <int REGS> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
 // Registers of a thread by what its warp does: with tiles of 64 tokens the drain holds 64 sums a thread.  A block is launched with 768 threads
@@ -414,13 +419,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         pdl_wait();       // C may still be in use by the kernel in front
         uint32_t i = 0;
         bool ok = true;
-        constexpr bool MEETS = PLANES && EPI == EPI_SWIGLU;
-        for (int tile = first_tile; tile < tiles; tile += stride) {
+        for (int tile = first_tile; tile < tiles && ok; tile += stride) {
             float acc[OWN], total[PLANES ? OWN : 1];
 #pragma unroll
             for (int j = 0; j < OWN; j++) acc[j] = 0.f;
             int in_part = 0, part = 0;
-            for (int c = 0; c < chunks && (ok || !MEETS); c++, i++) {
+            for (int c = 0; c < chunks; c++, i++) {
                 const int g = i & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(done0 + 8 * g, (i >> 1) & 1, abort_flag, p.status, 137));
                 if (!ok) break;
@@ -455,11 +459,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     in_part = 0;
                 }
             }
-            // (a gated tile's group of four warps meets at a named barrier, which has no limit: a warp whose own wait gave up goes there all the
-            // same, for this tile and all that follow, and stores nothing)
-            if (!ok && !MEETS) break;
+            if (!ok) {
+                // (a gated tile's group meets at a named barrier, which has no limit: a warp whose own wait gave up goes there all the same, for this tile
+                // and all that follow; what the others then store is no product, as the status says)
+                if constexpr (PLANES && EPI == EPI_SWIGLU) keep_meeting(1 + share, 2 * ((tiles - 1 - tile) / stride + 1) * (own / MEET));
+                break;
+            }
             if constexpr (PLANES) {
-                const int m0 = tile_t(tile) + col0, cols = MEETS && !ok ? 0 : min(own, p.M - m0);
+                const int m0 = tile_t(tile) + col0, cols = min(own, p.M - m0);
                 if (part > 0) {
 #pragma unroll
                     for (int j = 0; j < OWN; j++) acc[j] = total[j] + acc[j];
