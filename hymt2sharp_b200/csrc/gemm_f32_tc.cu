@@ -83,9 +83,26 @@ __device__ __forceinline__ void cut(float x0, float x1, uint32_t& hi, uint32_t& 
 }
 
 __device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+// The plain chain of K FMAs of a row of A and one of W (whose rows start on 16 bytes).  NaN stays what it is, whatever follows, and the chain ends
+// there: what a step gone wrong leaves is whole rows of it, and each cost N chains to their ends.  2,048 x 14,336, ms, chains to their ends and now:
+// 531 rows of NaN 62 and 0.24 (finite 0.23), one among 8 rows 2.96 and 0.05 (0.045).  A lone infinity in every row still takes 18 (62), in which no
+// wait of the other warps comes near its limit.
 __device__ __noinline__ float fma_chain(const float* a, const float* w, int K) {
     float acc = 0.f;
-    for (int k = 0; k < K; k++) acc = fmaf(a[k], w[k], acc);
+    int k = 0;
+#pragma unroll 1
+    for (; k + 16 <= K && acc == acc; k += 16) {
+        float x[16];
+        float4 y[4];
+#pragma unroll
+        for (int j = 0; j < 16; j++) x[j] = a[k + j];
+#pragma unroll
+        for (int j = 0; j < 4; j++) y[j] = *reinterpret_cast<const float4*>(w + k + 4 * j);
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc = fmaf(x[4 * j + 3], y[j].w, fmaf(x[4 * j + 2], y[j].z, fmaf(x[4 * j + 1], y[j].y, fmaf(x[4 * j], y[j].x, acc))));
+    }
+#pragma unroll 1
+    for (; k < K && acc == acc; k++) acc = fmaf(a[k], w[k], acc);
     return acc;
 }
 

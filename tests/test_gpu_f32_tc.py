@@ -97,3 +97,42 @@ def test_entries_at_the_ends_of_the_range(M):
         if epilogue == ops.EPILOGUE_STORE:          # (the chain's own error is K * 2^-24 * sum |a| |w|)
             assert ((got.double() - want.double()).abs() <= bound + 1e-44)[ok].all()
     assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M, epilogue", [(8, 0), (64, 0), (150, 1), (531, 2)])
+def test_rows_of_nan_cost_no_more_than_some_finite_ones(M, epilogue):
+    """Rows of NaN are what a step gone wrong leaves; their outputs are computed again as chains of FMAs, which end at the first NaN.  (To their ends they
+    took 50 to 450 times as long as finite rows.)  A lone infinity has its chain to the end, and no wait gives up meanwhile."""
+    ops = _ops()
+    torch.manual_seed(M)
+    N, K = 1024, 14336
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    w = torch.randn(2 * N if epilogue == ops.EPILOGUE_SWIGLU else N, K, device=DEV) / math.sqrt(K)
+    out, took = torch.zeros(M, N, device=DEV), []
+
+    def best(a):
+        times = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            out.zero_()
+            begin.record()
+            ops.gemm_f32_tc(out, a, w, epilogue, status)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    finite = torch.randn(M, K, device=DEV)
+    took.append(best(finite))
+    took.append(best(torch.full_like(finite, math.nan)))
+    assert out.isnan().all()
+    one = finite.clone()
+    one[M // 2] = math.nan
+    took.append(best(one))
+    assert out[M // 2].isnan().all() and out.isnan().sum() == N
+    assert max(took[1:]) <= 5 * took[0], took
+    one[M // 2] = finite[M // 2]
+    one[M // 2, K // 2] = math.inf
+    ops.gemm_f32_tc(out, one, w, epilogue, status)
+    assert not out[torch.arange(M, device=DEV) != M // 2].isinf().any() and not out[M // 2].isfinite().all()
+    assert status.tolist() == [0, 0, 0, 0]
