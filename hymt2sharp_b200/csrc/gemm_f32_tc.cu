@@ -1,13 +1,15 @@
 // float32 matrix product on the 5th-generation tensor cores of sm_100a:
-//   C = epilogue(A[M,K] · W[N,K]^T), float32 in, float32 out, no less exact than a chain of float32 FMAs.
+//   C = epilogue(A[M,K] · W[N,K]^T), float32 in, float32 out; sums of many terms no less exact than a chain of float32 FMAs.
 //
-// A float32 number is the sum of three bfloat16 numbers without loss: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (8 + 8 + 8
-// bits, and bfloat16 has float32's exponents).  A product of two numbers is then nine products of pieces, of which six count: the
-// three that are dropped (mid·lo, lo·mid, lo·lo) are at most 2^-26 of the whole.  Products of pieces are exact; what is left are
+// A float32 number from 2^-110 on is the sum of three bfloat16 numbers without loss: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (8 + 8 +
+// 8 bits, and bfloat16 has float32's exponents).  Below, the third piece falls under bfloat16's smallest number, and an entry loses up to 2^-134.
+// A product of two numbers is then nine products of pieces, of which six count: the three that are dropped (mid·lo, lo·mid, lo·lo) are some
+// 2^-24 of the whole at most (|mid| <= 2^-8, |lo| <= 2^-17 of an entry near 1).  Products of pieces are exact; what is left are
 // the additions.  The tensor core cuts its sums off where an FMA rounds them, so no long sum is left to it: CHUNK entries of K are
 // added up in tensor memory, the small products first and the four large ones last (so only four cut-offs of the chunk's own size
 // happen), and the chunks are added by float32 additions in registers.  Relative distance to 64-bit sums, normal entries: K = 512 9e-8,
-// 2,048 1.0e-7, 6,144 9e-8; a chain of K FMAs 4e-7, 8e-7, 1.0e-6.
+// 2,048 1.0e-7, 6,144 9e-8; a chain of K FMAs 4e-7, 8e-7, 1.0e-6.  It is the long sums that gain: rows of 2,048 of which 64 entries are not 0 come to
+// 8.3e-8 (1.4e-7), of 8 to 6.8e-8 (5.4e-8), of a single one to 4.6e-8, where one rounding makes 2.5e-8 (at most 2.3 and 1 times 2^-24).
 //
 // Every output is the same sum in the same order whatever M is and whichever of the two kernels below runs: chunks in ascending order
 // within a part of K, the parts (1 to 8, a rule on N and K alone) in ascending order.
@@ -151,7 +153,7 @@ __host__ __device__ constexpr int token_bytes(bool planes, int bn) { return plan
 
 // Warp 0 brings W's stages (and with few rows the tokens'), warp 3 the planes, in a ring of their own: a stage of W is free again when it
 // is cut, planes when they are multiplied.  Groups of four warps cut W's (and, with few rows, the tokens') entries of stage after stage into
-// pieces (a stage takes a group 2,400 cycles, most of them latency: looks at barriers, shared memory, conversions, tensor memory), warps 1
+// pieces (a stage takes a group 1,500 to 1,800 cycles, most of them latency: looks at barriers, shared memory, conversions, tensor memory), warps 1
 // and 2 issue the MMAs of the even and the odd chunks (an accumulator each), the rest drains accumulators and
 // writes C.  A look at a barrier takes hundreds of cycles, and an accumulator's way around (MMAs, drain, MMAs) holds three of them: chunks of
 // 32 took 1,650 cycles whatever the MMAs in them, so a chunk is two stages.
@@ -667,8 +669,8 @@ void plan_f32(int M, int N, int K, int epi, bool aligned, F32Plan* out) {
     pl.parts = (chunks + pl.chunks_per_part - 1) / pl.chunks_per_part;
     // Few rows: tiles of 16 to 64 tokens, a CTA a part.  Up to 64 rows always; beyond, where their waves cost less than the planes' (cycles, as
     // measured: a chunk 5,600 with 64 tokens in one kernel, 1,900 and 8.5 a column with planes; a wave's start and fold 5,000; the kernel that
-    // cuts the rows 9,500).  us, few rows / planes: 128 rows, 3,072 wide over 2,048 40 / 45, 6,144 gated 109 / 85; 531 rows, 1,536 over 1,024
-    // 60 / 28.
+    // cuts the rows 9,500).  us, few rows / planes: 128 rows, 2,048 wide over 2,048 27 / 32, over 6,144 51 / 87; 200 rows, 1,024 over 1,024 19.4 / 19.0;
+    // 160 rows, 1,536 over 1,024 21 / 19.  Of 33 to 64 rows 2,048 wide over 2,048 takes 18 / 32, but 6,144 gated 51 to 53 / 39.
     const int few_bn = M <= 16 ? 16 : M <= 32 ? 32 : 64, few_tiles = (M + few_bn - 1) / few_bn;
     const long few_ctas = (long)pl.tiles_n * few_tiles * pl.parts;
     const double few_cost = (double)((few_ctas + SMS - 1) / SMS) * (pl.chunks_per_part * 5600.0 + 5000.0);

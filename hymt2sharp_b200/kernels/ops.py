@@ -370,8 +370,9 @@ def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int
 
 
 # float32 products from these sizes of the weight on go to the tensor cores, whatever the number of rows, so that a row's sums do not depend
-# on it.  us on CUDA cores and there, 1 row / 8 / 32 / 531: 512 x 512 3.4 5.4 / 3.9 5.3 / 7.0 6.4 / 23 14; 1,536 x 512 gated 4.9 5.9 / 5.7 6.2 /
-# 9.5 7.4 / 33 19; 1,024 x 1,024 5.7 6.0 / 7.0 6.2 / 14 7.6 / 48 26; 2,048 x 2,048 10.3 10.2 / 13.0 10.4 / 24 13 / 127 45.
+# on it.  us on CUDA cores and there, 1 row / 8 / 32 / 531: 512 x 512 3.1 4.2 / 3.7 4.4 / 6.7 5.4 / 23 13; 1,536 x 512 gated 4.6 5.4 / 5.5 5.6 /
+# 9.3 6.8 / 47 18; 1,024 x 1,024 5.3 4.6 / 6.5 4.9 / 12 5.9 / 45 20; 2,048 x 2,048 9.9 8.2 / 12.3 8.4 / 23 10.4 / 123 36.  The shortest inner size pays at
+# up to 16 rows for what it gains beyond: 2,048 x 512, 1 row 3.2 4.9, 16 rows 5.0 5.3, 64 rows 11.3 7.1, 700 rows 46 15.
 F32_TC_MIN_SIDE, F32_TC_MIN_ENTRIES = 512, 1 << 20
 _f32_plans: dict = {}
 
@@ -405,8 +406,9 @@ def gemm_f32_tc_supported(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, e
 def gemm_f32_tc(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int, status: torch.Tensor, glu: GluRule | None = None,
                 glu_bias: torch.Tensor | None = None) -> None:
     """out[M, N] = epilogue(a[M, K] @ w[N, K]^T), float32, on the tcgen05 tensor cores: every operand as three bfloat16 pieces whose
-    products are exact, the sums in float32.  Not further from the exact product than a chain of float32 FMAs, and the same bit
-    for bit for a row whatever other rows there are.  With EPILOGUE_SWIGLU w has 2N rows."""
+    products are exact, the sums in float32.  Long sums are nearer to the exact ones than a chain of float32 FMAs (a row with few entries that are not
+    0 is off by some 2^-22 of its terms, an entry below 2^-110 by 2^-134), and a row is the same bit for bit whatever other rows there are.  With
+    EPILOGUE_SWIGLU w has 2N rows."""
     M, N = out.shape
     K = a.shape[1]
     rows_w = 2 * N if epilogue == EPILOGUE_SWIGLU else N
@@ -440,7 +442,9 @@ def device_status(device) -> torch.Tensor:
     """The int32[4] status word of a device: kernels set [0] when a device-side check fails or a
     bounded wait gives up (1: token id outside the table; 2: a sequence longer than the split attention was given
     room for; 3: a position outside the table of positions; 101-106: a wait of the tensor-core GEMM (106: for the partial sums of a tile's other CTAs); 108-119: of the prompt attention; 120-129: of the decode
-    attention)."""
+    attention; 131-139: of the float32 products on tensor cores (131 copies of the weights, 132 pieces and accumulators, 135 stages and buffers to cut into,
+    137 sums, 138 and 139 the tokens' pieces); 141-147: of the experts' product of few rows (141 copies, 142 and 145 rows, 143 and 146 accumulators, 144 stages, 147 the
+    quarters' sums))."""
     hit = _status_of.get(device)
     if hit is not None:
         return hit

@@ -77,7 +77,8 @@ def test_a_row_does_not_depend_on_the_others_and_is_nearer_than_a_chain(N, K, ep
 
 @pytest.mark.parametrize("M", [8, 150])
 def test_entries_at_the_ends_of_the_range(M):
-    """Infinities, NaN and entries whose first piece rounds to infinity give what the chain of FMAs gives; tiny ones lose nothing."""
+    """Infinities, NaN and entries whose first piece rounds to infinity give what the chain of FMAs gives, beside rows and columns of small ones
+    (how exact those are is asked below)."""
     ops = _ops()
     torch.manual_seed(M)
     status = torch.zeros(4, dtype=torch.int32, device=DEV)
@@ -135,4 +136,44 @@ def test_rows_of_nan_cost_no_more_than_some_finite_ones(M, epilogue):
     one[M // 2, K // 2] = math.inf
     ops.gemm_f32_tc(out, one, w, epilogue, status)
     assert not out[torch.arange(M, device=DEV) != M // 2].isinf().any() and not out[M // 2].isfinite().all()
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M", [8, 40, 300])
+def test_small_and_large_entries_lose_nothing_down_to_2_to_the_minus_110(M):
+    """A power of two on either side comes out as that power of two, bit for bit, as long as no entry falls below 2^-110 (2^-70 here, and none of these
+    normal entries is below 2^-40).  Below, the third piece is lost: an entry is off by half of bfloat16's smallest number, 2^-134, at most."""
+    ops = _ops()
+    torch.manual_seed(M)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    N, K = 640, 2048
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV) / math.sqrt(K)
+    a, w = (torch.where(t.abs() < 2.0 ** -40, 2.0 ** -40, t) for t in (a, w))
+    product = lambda x, y: (out := torch.empty(M, N, device=DEV), ops.gemm_f32_tc(out, x, y, ops.EPILOGUE_STORE, status))[0]
+    base = product(a, w)
+    for e in (60, -60, -70):
+        assert torch.equal(product(a * 2.0 ** e, w), base * 2.0 ** e) and torch.equal(product(a, w * 2.0 ** e), base * 2.0 ** e), e
+    for e, f in ((-116, 0), (-116, 20), (-125, 30), (-130, 40)):       # (the last rows are no normal numbers themselves; the products are)
+        x, y = a * 2.0 ** e, w * 2.0 ** f
+        ref, sums = x.double() @ y.double().T, x.double().abs() @ y.double().abs().T
+        bound = (1 + 16 + K // 64 + 8) * 2.0 ** -24 * sums + 2.0 ** -134 * y.double().abs().sum(1)
+        assert ((product(x, y).double() - ref).abs() <= bound).all(), (e, f)
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M", [8, 32, 48, 300])
+@pytest.mark.parametrize("entries", [1, 2, 8])
+def test_rows_with_few_entries(M, entries):
+    """Where a chain of FMAs rounds once a term, this is off by the dropped pieces (2^-24 of a term) and a cut-off at 2^-22 and a rounding a term; the
+    small products' cut-offs are some 2^-24 together."""
+    ops = _ops()
+    torch.manual_seed(M + entries)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    N, K = 1024, 2048
+    a, w, out = torch.zeros(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.empty(M, N, device=DEV)
+    for m in range(M):
+        a[m, torch.randperm(K, device=DEV)[:entries]] = torch.randn(entries, device=DEV)
+    ops.gemm_f32_tc(out, a, w, ops.EPILOGUE_STORE, status)
+    ref, sums = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert ((out.double() - ref).abs() <= (2 + 5 * entries) * 2.0 ** -24 * sums).all()
     assert status.tolist() == [0, 0, 0, 0]
